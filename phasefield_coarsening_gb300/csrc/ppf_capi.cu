@@ -6,6 +6,8 @@
 // fused step recomputes them per plane in shared memory) and the
 // increments detaS/detaL/dc are never stored either (only their squared
 // sums, phasefield.c:228-238, are kept for the convergence test).
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -263,15 +265,70 @@ extern "C" int ppf_set_stream(ppf_ctx *c, void *stream) {
     return PPF_OK;
 }
 
-int do_pack(ppf_ctx *c) {
+static int pack_from(ppf_ctx *c, const double *const src[3]) {
     c->cur_eta = 0;
     c->cur_c = 0;
-    if (c->prec == PPF_F32) CU(launch_pack<float>(c->g, c->staging, ff(c, 0, 0), c->stream));
-    else CU(launch_pack<double>(c->g, c->staging, fd(c, 0, 0), c->stream));
+    if (c->prec == PPF_F32) CU(launch_pack<float>(c->g, src, ff(c, 0, 0), c->stream));
+    else CU(launch_pack<double>(c->g, src, fd(c, 0, 0), c->stream));
     CU(cudaMemsetAsync(c->dres, 0, 3 * sizeof(double), c->stream));
     c->uploaded = 1;
     c->steps = 0;
     return PPF_OK;
+}
+
+int do_pack(ppf_ctx *c) {
+    const size_t n = (size_t)c->nz * c->ny * c->nx;
+    const double *const src[3] = {c->staging, c->staging + n, c->staging + 2 * n};
+    return pack_from(c, src);
+}
+
+static int unpack_to(ppf_ctx *c, double *const dst[3]) {
+    if (!c->uploaded) return seterr(PPF_ESTATE, "no state uploaded");
+    if (c->prec == PPF_F32) CU(launch_unpack<float>(c->g, cst(ff(c, c->cur_eta, c->cur_c)), dst, c->stream));
+    else CU(launch_unpack<double>(c->g, cst(fd(c, c->cur_eta, c->cur_c)), dst, c->stream));
+    return PPF_OK;
+}
+
+int do_unpack(ppf_ctx *c) {
+    const size_t n = (size_t)c->nz * c->ny * c->nx;
+    double *const dst[3] = {c->staging, c->staging + n, c->staging + 2 * n};
+    return unpack_to(c, dst);
+}
+
+// Whether the pack and unpack kernels may use the caller's three device
+// arrays themselves: memory of this device, 8-byte aligned, each inside one
+// allocation, not overlapping.  Anything else goes through the staging
+// array by cudaMemcpyAsync, which takes or refuses it as it always did.
+static bool direct_io(ppf_ctx *c, const double *const p[3]) {
+    const size_t bytes = (size_t)c->nz * c->ny * c->nx * sizeof(double);
+    static const PFN_cuPointerGetAttributes_v7000 query = [] {
+        cudaDriverEntryPointQueryResult q;
+        void *f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (PFN_cuPointerGetAttributes_v7000)f;
+    }();
+    if (!query) return false;
+    for (int k = 0; k < 3; ++k) {
+        unsigned type = 0, managed = 0;
+        int dev = -1;
+        CUdeviceptr base = 0;
+        size_t size = 0;
+        CUpointer_attribute at[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                     CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE,
+                                     CU_POINTER_ATTRIBUTE_IS_MANAGED};
+        void *out[5] = {&type, &dev, &base, &size, &managed};
+        const uintptr_t a = (uintptr_t)p[k];
+        if ((a & 7) || query(5, at, out, (CUdeviceptr)a) != CUDA_SUCCESS) return false;
+        if (type != CU_MEMORYTYPE_DEVICE || managed || dev != c->dev) return false;
+        if (a < base || a - base > size || size - (a - base) < bytes) return false;
+        for (int j = 0; j < k; ++j) {
+            const uintptr_t b = (uintptr_t)p[j];
+            if (a < b + bytes && b < a + bytes) return false;
+        }
+    }
+    return true;
 }
 
 extern "C" int ppf_upload(ppf_ctx *c, const double *etaS, const double *etaL, const double *cc) {
@@ -289,21 +346,17 @@ extern "C" int ppf_upload(ppf_ctx *c, const double *etaS, const double *etaL, co
 extern "C" int ppf_upload_device(ppf_ctx *c, const double *etaS, const double *etaL, const double *cc) {
     if (!c || !etaS || !etaL || !cc) return seterr(PPF_EINVAL, "null argument");
     const size_t n = (size_t)c->nz * c->ny * c->nx;
-    CU(cudaMemcpyAsync(c->staging, etaS, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->staging + n, etaL, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->staging + 2 * n, cc, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    int rc = do_pack(c);
+    const double *const src[3] = {etaS, etaL, cc};
+    int rc;
+    if (direct_io(c, src)) {
+        rc = pack_from(c, src);
+    } else {
+        for (int k = 0; k < 3; ++k)
+            CU(cudaMemcpyAsync(c->staging + k * n, src[k], n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+        rc = do_pack(c);
+    }
     if (rc) return rc;
     CU(cudaStreamSynchronize(c->stream));
-    return PPF_OK;
-}
-
-int do_unpack(ppf_ctx *c) {
-    if (!c->uploaded) return seterr(PPF_ESTATE, "no state uploaded");
-    if (c->prec == PPF_F32)
-        CU(launch_unpack<float>(c->g, cst(ff(c, c->cur_eta, c->cur_c)), c->staging, c->stream));
-    else
-        CU(launch_unpack<double>(c->g, cst(fd(c, c->cur_eta, c->cur_c)), c->staging, c->stream));
     return PPF_OK;
 }
 
@@ -315,18 +368,23 @@ extern "C" int ppf_download(ppf_ctx *c, double *etaS, double *etaL, double *cc) 
     CU(cudaMemcpyAsync(etaS, c->staging, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CU(cudaMemcpyAsync(etaL, c->staging + n, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CU(cudaMemcpyAsync(cc, c->staging + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
     return check_device_error(c);
 }
 
 extern "C" int ppf_download_device(ppf_ctx *c, double *etaS, double *etaL, double *cc) {
     if (!c || !etaS || !etaL || !cc) return seterr(PPF_EINVAL, "null argument");
-    int rc = do_unpack(c);
-    if (rc) return rc;
+    if (!c->uploaded) return seterr(PPF_ESTATE, "no state uploaded");
     const size_t n = (size_t)c->nz * c->ny * c->nx;
-    CU(cudaMemcpyAsync(etaS, c->staging, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CU(cudaMemcpyAsync(etaL, c->staging + n, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    CU(cudaMemcpyAsync(cc, c->staging + 2 * n, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    double *const dst[3] = {etaS, etaL, cc};
+    if (direct_io(c, dst)) {
+        int rc = unpack_to(c, dst);
+        if (rc) return rc;
+    } else {
+        int rc = do_unpack(c);
+        if (rc) return rc;
+        for (int k = 0; k < 3; ++k)
+            CU(cudaMemcpyAsync(dst[k], c->staging + k * n, n * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
+    }
     CU(cudaStreamSynchronize(c->stream));
     return PPF_OK;
 }
@@ -390,18 +448,16 @@ extern "C" int ppf_reduce(ppf_ctx *c, ppf_stats *out) {
     if (!c || !out) return seterr(PPF_EINVAL, "null argument");
     if (!c->uploaded) return seterr(PPF_ESTATE, "no state uploaded");
     const int64_t cells = (int64_t)c->nz * c->ny * c->nx;
-    int nb = c->ny * c->nz;                     // one block per x row at most
-    if (nb > 8 * c->num_sms) nb = 8 * c->num_sms;
+    const int nb = c->prec == PPF_F32 ? observe_blocks<float>(c->g, c->num_sms) : observe_blocks<double>(c->g, c->num_sms);
     int rc = ensure_partials(c, 5 * nb);
     if (rc) return rc;
     if (c->prec == PPF_F32)
-        CU(launch_observe<float>(c->g, c->cd, cst(ff(c, c->cur_eta, c->cur_c)), c->partials, nb, c->stream));
+        CU(launch_observe<float>(c->g, c->cd, cst(ff(c, c->cur_eta, c->cur_c)), c->partials, c->num_sms, c->stream));
     else
-        CU(launch_observe<double>(c->g, c->cd, cst(fd(c, c->cur_eta, c->cur_c)), c->partials, nb, c->stream));
+        CU(launch_observe<double>(c->g, c->cd, cst(fd(c, c->cur_eta, c->cur_c)), c->partials, c->num_sms, c->stream));
     CU(launch_final_sum(c->partials, nb, 5, 5, c->dres + 3, c->stream));
     double h[8];
     CU(cudaMemcpyAsync(h, c->dres, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
     rc = check_device_error(c);
     if (rc) return rc;
     out->sum_dc2 = h[0];
@@ -419,7 +475,6 @@ extern "C" int ppf_reduce(ppf_ctx *c, ppf_stats *out) {
 
 extern "C" int ppf_sync(ppf_ctx *c) {
     if (!c) return seterr(PPF_EINVAL, "null context");
-    CU(cudaStreamSynchronize(c->stream));
     return check_device_error(c);
 }
 

@@ -73,7 +73,7 @@ struct ppf_ensemble {
     DomainDesc *dtable;          // device
     double **ddres;              // device: each domain's dres pointer
     IoDesc *dio;                 // device: each domain's batched-I/O descriptor (domain order)
-    int64_t max_cells;           // cells of the largest domain
+    int64_t max_rows;           // x rows of the domain with most of them
     double *partials;            // 3 doubles per work item
     int partials_cap;
     int items[3];                // work items of the edge-tile [0], whole-tile [1] and every-tile [2] launches
@@ -260,8 +260,8 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
             for (int b = 0; b < 2; ++b)
                 for (int f = 0; f < 3; ++f) t.fld[b][f] = x->fld[b][f];
             t.dres = x->dres;
-            const int64_t cells = (int64_t)x->nz * x->ny * x->nx;
-            if (cells > e->max_cells) e->max_cells = cells;
+            const int64_t rows = (int64_t)x->nz * x->ny;
+            if (rows > e->max_rows) e->max_rows = rows;
         }
         ce = cudaMemcpy(e->dio, io.data(), io.size() * sizeof(IoDesc), cudaMemcpyHostToDevice);
     }
@@ -326,8 +326,8 @@ extern "C" int ppf_ensemble_upload_all(ppf_ensemble *e, const double *const *eta
         ECU(cudaMemcpyAsync(x->staging + n, etaL[d], n * sizeof(double), cudaMemcpyHostToDevice, e->stream));
         ECU(cudaMemcpyAsync(x->staging + 2 * n, c[d], n * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     }
-    if (e->prec == PPF_F32) ECU(launch_pack_multi<float>(e->dio, e->n, e->max_cells, e->stream));
-    else ECU(launch_pack_multi<double>(e->dio, e->n, e->max_cells, e->stream));
+    if (e->prec == PPF_F32) ECU(launch_pack_multi<float>(e->dio, e->n, e->max_rows, e->stream));
+    else ECU(launch_pack_multi<double>(e->dio, e->n, e->max_rows, e->stream));
     for (ppf_ctx *x : e->dom) {
         x->cur_eta = x->cur_c = 0;
         x->uploaded = 1;
@@ -357,8 +357,8 @@ extern "C" int ppf_ensemble_download_all(ppf_ensemble *e, double *const *etaS, d
     }
     // one conversion launch for all domains, then every domain's copies, then
     // one synchronisation
-    if (e->prec == PPF_F32) ECU(launch_unpack_multi<float>(e->dio, e->n, e->max_cells, e->parity, e->stream));
-    else ECU(launch_unpack_multi<double>(e->dio, e->n, e->max_cells, e->parity, e->stream));
+    if (e->prec == PPF_F32) ECU(launch_unpack_multi<float>(e->dio, e->n, e->max_rows, e->parity, e->stream));
+    else ECU(launch_unpack_multi<double>(e->dio, e->n, e->max_rows, e->parity, e->stream));
     for (int d = 0; d < e->n; ++d) {
         ppf_ctx *x = e->dom[(size_t)d];
         const size_t n = (size_t)x->nz * x->ny * x->nx;

@@ -65,12 +65,13 @@ struct Fields {
     T *eS, *eL, *c;
 };
 
-// Pack/unpack between compact double arrays [z][y][x] and the padded
-// layout; pack also writes the face ghosts (the BC fill of :207-211).
+// Pack/unpack between three compact double arrays [z][y][x] (8-byte aligned
+// device memory, not overlapping) and the padded layout; pack also writes
+// the face ghosts (the BC fill of :207-211).
 template <typename T>
-cudaError_t launch_pack(const Geom &g, const double *src3, Fields<T> dst, cudaStream_t s);
+cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, cudaStream_t s);
 template <typename T>
-cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *dst3, cudaStream_t s);
+cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[3], cudaStream_t s);
 
 // One domain of a batched pack / unpack (device table): its geometry, its
 // compact float64 staging array (3 fields), its two state buffers and its
@@ -84,23 +85,26 @@ struct IoDesc {
 
 // Pack every domain's staging into its buffer 0 (clearing its increment
 // sums), or unpack every domain's buffer `buf` into its staging: one launch
-// for `n` domains (grid y = domain), the largest holding max_cells cells.
+// for `n` domains (grid y = domain), the largest holding max_rows x rows.
 template <typename T>
-cudaError_t launch_pack_multi(const IoDesc *table, int n, int64_t max_cells, cudaStream_t s);
+cudaError_t launch_pack_multi(const IoDesc *table, int n, int64_t max_rows, cudaStream_t s);
 template <typename T>
-cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_cells, int buf, cudaStream_t s);
+cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_rows, int buf, cudaStream_t s);
 
-// Observables of a state: per-CTA partial sums of
-// {mass, solid, solid_cells, free energy, nonfinite} into partials[5*b+i].
+// Observables of a state: per-block partial sums of
+// {mass, solid, solid_cells, free energy, nonfinite} into partials[5*b+i]
+// for b < observe_blocks.
+template <typename T>
+int observe_blocks(const Geom &g, int num_sms);
 template <typename T>
 cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, double *partials,
-                           int nblocks, cudaStream_t s);
+                           int num_sms, cudaStream_t s);
 
 // Record `msg` as the calling thread's ppf_last_error() text; returns code.
 int set_last_error(int code, const char *msg);
 
 // Deterministic final sum: out[i] = sum_b partials[stride*b + i] for
-// i < nvals (fixed order, one CTA).
+// i < nvals (fixed order, one CTA per value).
 cudaError_t launch_final_sum(const double *partials, int nblocks, int stride, int nvals, double *out,
                              cudaStream_t s);
 

@@ -1,7 +1,7 @@
 // ppf_state.cu -- state movement and reductions around the fused step:
 // pack/unpack between the caller's compact [z][y][x] double arrays and the
 // padded ghosted device layout (the BC fill of phasefield.c:207-211 is done
-// on pack), the observables reduction (FP64 accumulation) and the
+// on pack), the observables reduction and the
 // deterministic final sum of per-CTA partials.
 #include <cuda_runtime.h>
 
@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "ppf_internal.h"
+#include "ppf_pair.h"
 
 namespace ppf {
 
@@ -76,214 +77,483 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double *partial
     }
 }
 
-// ---------------------------------------------------------------- pack ----
+// ------------------------------------------------------- pack / unpack ----
+//
+// Bound by HBM: 24 bytes of float64 per cell on the caller's side and 12 or
+// 24 in the state.  One warp per x row, so that a row's y, z and ghost rows
+// are worked out once and a lane only adds x (no 64-bit divisions per cell).
+// The caller's three arrays are read and written in place when they are
+// device memory of this device; host arrays pass through the staging array.
+// 256^3 FP32, state to device arrays: 101 us, 6.0 TB/s; through the staging
+// array with one thread per cell it was 106 us and 126 us of copies.
+
+constexpr int kRowWarps = 8;   // rows per block and pass
 
 template <typename T>
-__global__ void pack_kernel(Geom g, const double *__restrict__ src, Fields<T> dst) {
-    const int64_t n = (int64_t)g.nx * g.ny * g.nz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % g.nx);
-        const int y = (int)((i / g.nx) % g.ny);
-        const int z = (int)(i / ((int64_t)g.nx * g.ny));
-        store_with_ghosts(g, dst, x, y, z, (T)src[i], (T)src[n + i], (T)src[2 * n + i], false);
+__device__ __forceinline__ void pack_rows(const Geom &g, const double *__restrict__ s0, const double *__restrict__ s1,
+                                          const double *__restrict__ s2, const Fields<T> &dst) {
+    const int lane = threadIdx.x & 31;
+    const int nrows = g.ny * g.nz;
+    for (int r = blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < nrows; r += gridDim.x * kRowWarps) {
+        const int z = r / g.ny, y = r - z * g.ny;
+        const int64_t i0 = (int64_t)r * g.nx;
+        const bool inner = y > 0 && y < g.ny - 1 && z > 0 && z < g.nz - 1;   // feeds x ghosts only
+        const int64_t a0 = g.at(0, y, z);
+#pragma unroll 4
+        for (int x = lane; x < g.nx; x += 32) {
+            const T s = (T)s0[i0 + x], l = (T)s1[i0 + x], c = (T)s2[i0 + x];
+            if (inner && x > 0 && x < g.nx - 1) {
+                dst.eS[a0 + x] = s;
+                dst.eL[a0 + x] = l;
+                dst.c[a0 + x] = c;
+            } else {
+                store_with_ghosts(g, dst, x, y, z, s, l, c, false);
+            }
+        }
+    }
+}
+
+// A float as a double.  The conversion instruction runs at the FP64 rate,
+// 1/64 of the FP32 rate here, and bounded the FP32 unpack (three per cell);
+// for normal numbers and zeros the double's bits are the float's, shifted,
+// with the exponent rebased.
+__device__ __forceinline__ double widen(float v) {
+    const unsigned b = __float_as_uint(v), m = b & 0x7fffffffu;
+    if (m - 0x00800000u < 0x7f000000u || m == 0u) {
+        const unsigned hi = (m >> 3) + (m ? 0x38000000u : 0u);
+        return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
+    }
+    // denormals, infinities, NaN (volatile: not evaluated ahead of the test)
+    double d;
+    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(d) : "f"(v));
+    return d;
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
+template <typename T>
+__device__ __forceinline__ void unpack_rows(const Geom &g, const T *__restrict__ eS, const T *__restrict__ eL,
+                                            const T *__restrict__ c, double *__restrict__ d0, double *__restrict__ d1,
+                                            double *__restrict__ d2) {
+    const int lane = threadIdx.x & 31;
+    const int nrows = g.ny * g.nz;
+    // rows that start on 16 bytes everywhere: two cells per lane and access
+    const bool two = (g.nx & 1) == 0 && (((uintptr_t)d0 | (uintptr_t)d1 | (uintptr_t)d2) & 15) == 0;
+    for (int r = blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < nrows; r += gridDim.x * kRowWarps) {
+        const int z = r / g.ny, y = r - z * g.ny;
+        const int64_t i0 = (int64_t)r * g.nx, a0 = g.at(0, y, z);
+        if (two) {
+#pragma unroll 4
+            for (int x = 2 * lane; x < g.nx; x += 64) {
+                const V2<T> s = ld2(eS + a0 + x), l = ld2(eL + a0 + x), q = ld2(c + a0 + x);
+                st2(d0 + i0 + x, V2<double>(widen(s.x()), widen(s.y())));
+                st2(d1 + i0 + x, V2<double>(widen(l.x()), widen(l.y())));
+                st2(d2 + i0 + x, V2<double>(widen(q.x()), widen(q.y())));
+            }
+        } else {
+#pragma unroll 4
+            for (int x = lane; x < g.nx; x += 32) {
+                d0[i0 + x] = widen(eS[a0 + x]);
+                d1[i0 + x] = widen(eL[a0 + x]);
+                d2[i0 + x] = widen(c[a0 + x]);
+            }
+        }
     }
 }
 
 template <typename T>
-__global__ void unpack_kernel(Geom g, Fields<const T> src, double *__restrict__ dst) {
-    const int64_t n = (int64_t)g.nx * g.ny * g.nz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % g.nx);
-        const int y = (int)((i / g.nx) % g.ny);
-        const int z = (int)(i / ((int64_t)g.nx * g.ny));
-        const int64_t j = g.at(x, y, z);
-        dst[i] = (double)src.eS[j];
-        dst[n + i] = (double)src.eL[j];
-        dst[2 * n + i] = (double)src.c[j];
-    }
-}
-
-static int grid_for(int64_t n, int nt) {
-    int64_t b = (n + nt - 1) / nt;
-    return (int)(b < 152 * 16 ? (b < 1 ? 1 : b) : 152 * 16);
+__global__ void __launch_bounds__(32 * kRowWarps) pack_kernel(Geom g, const double *s0, const double *s1,
+                                                              const double *s2, Fields<T> dst) {
+    pack_rows<T>(g, s0, s1, s2, dst);
 }
 
 template <typename T>
-__global__ void pack_multi_kernel(const IoDesc *__restrict__ table) {
+__global__ void __launch_bounds__(32 * kRowWarps) unpack_kernel(Geom g, Fields<const T> src, double *d0, double *d1,
+                                                                double *d2) {
+    unpack_rows<T>(g, src.eS, src.eL, src.c, d0, d1, d2);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(32 * kRowWarps) pack_multi_kernel(const IoDesc *__restrict__ table) {
     const IoDesc &d = table[blockIdx.y];
     const Geom g = d.g;
     const Fields<T> dst = {(T *)d.fld[0][0], (T *)d.fld[0][1], (T *)d.fld[0][2]};
-    const double *src = d.staging;
     if (blockIdx.x == 0 && threadIdx.x < 3) d.dres[threadIdx.x] = 0.0;
     const int64_t n = (int64_t)g.nx * g.ny * g.nz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % g.nx);
-        const int y = (int)((i / g.nx) % g.ny);
-        const int z = (int)(i / ((int64_t)g.nx * g.ny));
-        store_with_ghosts(g, dst, x, y, z, (T)src[i], (T)src[n + i], (T)src[2 * n + i], false);
-    }
+    pack_rows<T>(g, d.staging, d.staging + n, d.staging + 2 * n, dst);
 }
 
 template <typename T>
-__global__ void unpack_multi_kernel(const IoDesc *__restrict__ table, int buf) {
+__global__ void __launch_bounds__(32 * kRowWarps) unpack_multi_kernel(const IoDesc *__restrict__ table, int buf) {
     const IoDesc &d = table[blockIdx.y];
     const Geom g = d.g;
-    const T *sS = (const T *)d.fld[buf][0], *sL = (const T *)d.fld[buf][1], *sC = (const T *)d.fld[buf][2];
-    double *dst = d.staging;
     const int64_t n = (int64_t)g.nx * g.ny * g.nz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int x = (int)(i % g.nx);
-        const int y = (int)((i / g.nx) % g.ny);
-        const int z = (int)(i / ((int64_t)g.nx * g.ny));
-        const int64_t j = g.at(x, y, z);
-        dst[i] = (double)sS[j];
-        dst[n + i] = (double)sL[j];
-        dst[2 * n + i] = (double)sC[j];
-    }
+    unpack_rows<T>(g, (const T *)d.fld[buf][0], (const T *)d.fld[buf][1], (const T *)d.fld[buf][2], d.staging,
+                   d.staging + n, d.staging + 2 * n);
+}
+
+static int row_grid(int64_t nrows) {
+    const int64_t b = (nrows + kRowWarps - 1) / kRowWarps;
+    return (int)(b < 152 * 8 ? b : 152 * 8);
 }
 
 template <typename T>
-cudaError_t launch_pack_multi(const IoDesc *table, int n, int64_t max_cells, cudaStream_t s) {
-    pack_multi_kernel<T><<<dim3((unsigned)grid_for(max_cells, 256), (unsigned)n), 256, 0, s>>>(table);
+cudaError_t launch_pack_multi(const IoDesc *table, int n, int64_t max_rows, cudaStream_t s) {
+    pack_multi_kernel<T><<<dim3((unsigned)row_grid(max_rows), (unsigned)n), 32 * kRowWarps, 0, s>>>(table);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_cells, int buf, cudaStream_t s) {
-    unpack_multi_kernel<T><<<dim3((unsigned)grid_for(max_cells, 256), (unsigned)n), 256, 0, s>>>(table, buf);
+cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_rows, int buf, cudaStream_t s) {
+    unpack_multi_kernel<T><<<dim3((unsigned)row_grid(max_rows), (unsigned)n), 32 * kRowWarps, 0, s>>>(table, buf);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_pack(const Geom &g, const double *src3, Fields<T> dst, cudaStream_t s) {
-    pack_kernel<T><<<grid_for((int64_t)g.nx * g.ny * g.nz, 256), 256, 0, s>>>(g, src3, dst);
+cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, cudaStream_t s) {
+    pack_kernel<T><<<row_grid((int64_t)g.ny * g.nz), 32 * kRowWarps, 0, s>>>(g, src[0], src[1], src[2], dst);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *dst3, cudaStream_t s) {
-    unpack_kernel<T><<<grid_for((int64_t)g.nx * g.ny * g.nz, 256), 256, 0, s>>>(g, src, dst3);
+cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[3], cudaStream_t s) {
+    unpack_kernel<T><<<row_grid((int64_t)g.ny * g.nz), 32 * kRowWarps, 0, s>>>(g, src, dst[0], dst[1], dst[2]);
     return cudaGetLastError();
 }
 
 // ----------------------------------------------------------- observables --
-// Energy density in the step's precision, accumulated in double.  Free
-// energy density (no counterpart in the reference; its variational
+// Free energy density (no counterpart in the reference; its variational
 // derivative is the bracket of phasefield.c:360-373):
-//   m f0(etaS, etaL) + kappa/2 |grad eta|^2 (forward differences) + hS fS + (1-hS) fL
+//   m f0(etaS, etaL) + kappa/2 |grad eta|^2 (forward differences) + hS fS + (1-hS) fL.
+// By the KKS identity AS (cS-cS0) = AL (cL-cL0) = mu the chemical part is
+//   AS AL / (2 (AS + (AL-AS) hS)) w^2 + CL + hS (CS-CL),  w = c - cL0 + (cL0-cS0) hS,
+// so that only w^2 is summed per cell and the constants CS, CL (orders of
+// magnitude above the rest) enter once per block, through the cell count and
+// the sum of hS.
+//
+// Each thread owns 16 bytes of cells in x and marches up z, so that a
+// plane's upper neighbours are the next plane's own cells; an FP32 thread
+// evaluates its four cells as two packed pairs.  FP32 state: the solid
+// fraction and the energy terms are compensated float sums per thread
+// (about 48 bits), the solute mass a float sum in three parts (about 72
+// bits: more than an FP64 running sum keeps), FP64 beyond the thread.  FP64
+// accumulation per cell is what bounded the FP32 form (one conversion and
+// one addition per cell, each 1/64 of the FP32 rate); the FP64 state's form
+// is bound by the FP64 pipe, so it is written for few FP64 operations
+// (about 32 per cell).  256^3 FP32: 54 us (186 us with one cell per thread
+// and FP64 sums of the solute mass); 64^3: 7 us (33 us).
 
-// A float sum carried with its rounding error (Knuth's TwoSum): about 48
-// bits, enough for per-thread partial sums of FP32 cell terms; FP32 adds are
-// far cheaper than FP64 ones on this GPU.
-struct FSum {
-    float hi, lo;
-};
-__device__ __forceinline__ void fsum_add(FSum &a, float x) {
-    const float s = a.hi + x;
-    const float bp = s - a.hi;
-    const float err = (a.hi - (s - bp)) + (x - bp);
-    a.hi = s;
-    a.lo += err;
+// sums of pairs of floats carried with their rounding errors (Knuth's TwoSum)
+__device__ __forceinline__ V2<float> two_sum(V2<float> a, V2<float> x, V2<float> &err) {
+    const V2<float> s = a + x;
+    const V2<float> bp = s - a;
+    err = (a - (s - bp)) + (x - bp);
+    return s;
+}
+
+__device__ __forceinline__ float two_sum1(float a, float x, float &err) {
+    const float s = a + x;
+    const float bp = s - a;
+    err = (a - (s - bp)) + (x - bp);
+    return s;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) observe_kernel(Geom g, CoefD kd, Fields<const T> f, double *partials) {
-    const T AS = (T)kd.AS, AL = (T)kd.AL, dA = (T)kd.dA, cS0 = (T)kd.cS0, cL0 = (T)kd.cL0;
-    const T CS = (T)kd.CS, CL = (T)kd.CL, tmp2 = (T)kd.tmp2, m = (T)kd.m, gam = (T)kd.gamma;
-    const T kg = (T)kd.kappa_h2_half;
-    constexpr bool F32 = std::is_same<T, float>::value;
-    double acc[5] = {0, 0, 0, 0, 0};
-    // FP32 state: the solid fraction and the free energy are summed per
-    // thread as compensated float sums (the solute mass stays an FP64 sum of
-    // the stored values, exact to rounding); FP64 state: FP64 throughout
-    FSum hsum = {0.f, 0.f}, fsum = {0.f, 0.f};
-    int nsolid = 0, nbad = 0;
-    // one block per x row (grid-stride over rows): no per-cell index division
-    const int nrows = g.ny * g.nz;
-    for (int rr = blockIdx.x; rr < nrows; rr += gridDim.x) {
-        const int64_t j0 = g.at(0, rr % g.ny, rr / g.ny);
-        for (int x = threadIdx.x; x < g.nx; x += blockDim.x) {
-            const int64_t j = j0 + x;
-            const T eS = f.eS[j], eL = f.eL[j], c = f.c[j];
-            if (!isfinite(eS) || !isfinite(eL) || !isfinite(c)) {
-                ++nbad;
-                continue;
+struct Sum;   // a pair of running sums, about 48 bits or better
+template <>
+struct Sum<float> {
+    V2<float> hi = splat(0.f), lo = splat(0.f);
+    __device__ __forceinline__ void add(V2<float> x) {
+        V2<float> e;
+        hi = two_sum(hi, x, e);
+        lo = lo + e;
+    }
+    __device__ __forceinline__ double get() const {
+        float e;
+        const float h = two_sum1(hi.x(), hi.y(), e);
+        return (double)h + (double)(lo.x() + lo.y() + e);
+    }
+};
+template <>
+struct Sum<double> {
+    V2<double> s = splat(0.0);
+    __device__ __forceinline__ void add(V2<double> x) { s = s + x; }
+    __device__ __forceinline__ double get() const { return s.x() + s.y(); }
+};
+
+template <typename T>
+struct Mass : Sum<double> {};   // FP64: the plain sum
+template <>
+struct Mass<float> {            // FP32: three parts
+    V2<float> hi = splat(0.f), mid = splat(0.f), lo = splat(0.f);
+    __device__ __forceinline__ void add(V2<float> x) {
+        V2<float> e, f;
+        hi = two_sum(hi, x, e);
+        mid = two_sum(mid, e, f);
+        lo = lo + f;
+    }
+    __device__ __forceinline__ double get() const {
+        float e, f, q;
+        const float h = two_sum1(hi.x(), hi.y(), e);
+        const float m = two_sum1(two_sum1(mid.x(), mid.y(), f), e, q);
+        return (double)h + ((double)m + (double)(lo.x() + lo.y() + f + q));
+    }
+};
+
+// 1/x of a pair: the hardware's estimate (about 1 ulp) and a Newton step
+__device__ __forceinline__ V2<float> recip(V2<float> x) {
+    float a, b;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(x.x()));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(x.y()));
+    const V2<float> y(a, b), e = fma2(splat(0.f) - x, y, splat(1.f));
+    return fma2(y, e, y);
+}
+// 1/x by one third-order Newton step y (1 + e + e^2), e = 1 - x y, on the
+// hardware's estimate (e below 2^-20, so the remainder e^3 is far below an
+// ulp): three FP64 operations.  Operands near the ends of the range take
+// the exact division.
+__device__ __forceinline__ double recip(double x) {
+    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+    if (ex - 64u > 1920u) return 1.0 / x;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ V2<double> recip(V2<double> x) { return V2<double>(recip(x.x()), recip(x.y())); }
+
+// finite, and above one half, without FP64 instructions
+__device__ __forceinline__ bool finite_(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite_(double v) {
+    return ((unsigned)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u;
+}
+__device__ __forceinline__ bool above_half(float v) { return v > 0.5f; }
+__device__ __forceinline__ bool above_half(double v) { return __double_as_longlong(v) > 0x3fe0000000000000ll; }
+
+template <typename T>
+struct ObsCoef {
+    T cL0, dc0, AS, dA, m, kg, g;
+    int eq;                       // AS == AL: w^2 is summed without its denominator
+    double hA, CL, dC, vol;       // hA = AS AL / 2 (AS / 2 when eq)
+};
+
+template <typename T>
+struct ObsAcc {
+    Mass<T> mass;
+    Sum<T> h, w, f;      // solid fraction, chemical energy, m f0 + gradient energy
+    int n = 0, solid = 0, bad = 0;
+
+    // a pair of finite cells (own values and the +x, +y, +z neighbours), of
+    // which only the first counts when `one` is set
+    __device__ __forceinline__ void pair(const ObsCoef<T> &k, V2<T> eS, V2<T> eL, V2<T> c, V2<T> sx, V2<T> lx,
+                                         V2<T> sy, V2<T> ly, V2<T> sz, V2<T> lz, bool one = false) {
+        const V2<T> S2 = eS * eS, L2 = eL * eL, s2 = fma2(eL, eL, S2);
+        const V2<T> hh = S2 * recip(s2);
+        const V2<T> ww = fma2(hh, splat(k.dc0), c - splat(k.cL0));
+        V2<T> ch = ww * ww;
+        if (!k.eq) {
+            const V2<T> den = fma2(hh, splat(k.dA), splat(k.AS));
+            ch = ch * recip(den);
+        }
+        // f0 = S2 (S2/4 - 1/2 + gamma L2) + L2 (L2/4 - 1/2) + 1/4
+        const V2<T> q = splat(T(0.25)), hf = splat(T(-0.5));
+        const V2<T> f0 = fma2(S2, fma2(S2, q, fma2(splat(k.g), L2, hf)), fma2(L2, fma2(L2, q, hf), q));
+        V2<T> d = sx - eS;
+        V2<T> gr = d * d;
+        d = lx - eL;
+        gr = fma2(d, d, gr);
+        d = sy - eS;
+        gr = fma2(d, d, gr);
+        d = ly - eL;
+        gr = fma2(d, d, gr);
+        d = sz - eS;
+        gr = fma2(d, d, gr);
+        d = lz - eL;
+        gr = fma2(d, d, gr);
+        const V2<T> ff = fma2(splat(k.kg), gr, splat(k.m) * f0);
+        auto in = [&](V2<T> v) { return one ? V2<T>(v.x(), T(0)) : v; };
+        mass.add(in(c));
+        h.add(in(hh));
+        w.add(in(ch));
+        f.add(in(ff));
+    }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256, 3) observe_kernel(Geom g, ObsCoef<T> k, Fields<const T> fl, int nq, int zc,
+                                                      double *partials) {
+    constexpr int Q = 16 / (int)sizeof(T), NP = Q / 2;   // cells and pairs per thread
+    ObsAcc<T> acc;
+    const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int y = (int)(t / nq), x0 = (int)(t - (int64_t)y * nq) * Q;
+    if (y < g.ny) {
+        const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
+        const bool whole = x0 + Q <= g.nx;
+        int64_t j = g.at(x0, y, z0);        // rows start on a sector: 16-byte aligned
+        T s[Q], l[Q];
+        auto load = [](const T *p, T (&v)[Q]) {
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+                const V2<T> w = ld2(p + 2 * i);
+                v[2 * i] = w.x();
+                v[2 * i + 1] = w.y();
             }
-            // +x/+y/+z neighbours read through the ghost layer (periodic wrap or no-flux copy)
-            const T sx = f.eS[j + 1], sy = f.eS[j + g.P], sz = f.eS[j + g.PS];
-            const T lx = f.eL[j + 1], ly = f.eL[j + g.P], lz = f.eL[j + g.PS];
-            const T s2 = eS * eS + eL * eL;
-            const T h = eS * eS / s2;
-            const T f0 = eS * eS * eS * eS / T(4) - eS * eS / T(2) + eL * eL * eL * eL / T(4) - eL * eL / T(2) +
-                         gam * eS * eS * eL * eL + T(0.25);
-            const T gr = (sx - eS) * (sx - eS) + (lx - eL) * (lx - eL) + (sy - eS) * (sy - eS) +
-                         (ly - eL) * (ly - eL) + (sz - eS) * (sz - eS) + (lz - eL) * (lz - eL);
-            const T rA = T(1) / (AS + dA * h);
-            const T cSp = rA * (AL * c + (T(1) - h) * tmp2);
-            const T cLp = rA * (AS * c - h * tmp2);
-            const T fS = T(0.5) * AS * (cSp - cS0) * (cSp - cS0) + CS;
-            const T fL = T(0.5) * AL * (cLp - cL0) * (cLp - cL0) + CL;
-            acc[0] += (double)c;
-            nsolid += eS > T(0.5) ? 1 : 0;
-            if constexpr (F32) {
-                fsum_add(hsum, h);
-                // the terms differ by orders of magnitude (the parabola offsets
-                // CS, CL against gradient and well terms): each added on its own
-                fsum_add(fsum, m * f0);
-                fsum_add(fsum, kg * gr);
-                fsum_add(fsum, h * fS);
-                fsum_add(fsum, (T(1) - h) * fL);
+        };
+        load(fl.eS + j, s);
+        load(fl.eL + j, l);
+        for (int z = z0; z < z1; ++z, j += g.PS) {
+            T c[Q], sy[Q], ly[Q], sz[Q], lz[Q];
+            load(fl.c + j, c);
+            load(fl.eS + j + g.P, sy);
+            load(fl.eL + j + g.P, ly);
+            load(fl.eS + j + g.PS, sz);
+            load(fl.eL + j + g.PS, lz);
+            // the cell after the last one (a ghost at the domain's end)
+            const T sx = whole ? fl.eS[j + Q] : T(0), lx = whole ? fl.eL[j + Q] : T(0);
+            bool fine = whole;
+#pragma unroll
+            for (int i = 0; i < Q; ++i) fine = fine && finite_(s[i]) && finite_(l[i]) && finite_(c[i]);
+            if (fine) {
+                acc.n += Q;
+#pragma unroll
+                for (int i = 0; i < Q; ++i) acc.solid += above_half(s[i]) ? 1 : 0;
+#pragma unroll
+                for (int i = 0; i < NP; ++i) {
+                    const int a = 2 * i, b = a + 1;
+                    const bool e = b == Q - 1;
+                    acc.pair(k, V2<T>(s[a], s[b]), V2<T>(l[a], l[b]), V2<T>(c[a], c[b]),
+                             V2<T>(s[b], e ? sx : s[(b + 1) % Q]), V2<T>(l[b], e ? lx : l[(b + 1) % Q]),
+                             V2<T>(sy[a], sy[b]), V2<T>(ly[a], ly[b]), V2<T>(sz[a], sz[b]), V2<T>(lz[a], lz[b]));
+                }
             } else {
-                acc[1] += (double)h;
-                acc[3] += ((double)(m * f0) + (double)(kg * gr)) + ((double)(h * fS) + (double)((T(1) - h) * fL));
+                // a partial group at the row's end, or non-finite cells (counted
+                // and left out): cell by cell, twice the same cell in a pair
+                for (int i = 0; i < Q && x0 + i < g.nx; ++i) {
+                    const int64_t a = j + i;
+                    const T S = fl.eS[a], L = fl.eL[a], C = fl.c[a];
+                    if (!finite_(S) || !finite_(L) || !finite_(C)) {
+                        ++acc.bad;
+                        continue;
+                    }
+                    ++acc.n;
+                    acc.solid += above_half(S) ? 1 : 0;
+                    acc.pair(k, splat(S), splat(L), splat(C), splat(fl.eS[a + 1]), splat(fl.eL[a + 1]),
+                             splat(fl.eS[a + g.P]), splat(fl.eL[a + g.P]), splat(fl.eS[a + g.PS]),
+                             splat(fl.eL[a + g.PS]), true);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                s[i] = sz[i];
+                l[i] = lz[i];
             }
         }
     }
-    if constexpr (F32) {
-        acc[1] = (double)hsum.hi + (double)hsum.lo;
-        acc[3] = (double)fsum.hi + (double)fsum.lo;
+    // Four sums over the warp: each exchange halves the sums a lane carries
+    // (six FP64 additions a thread instead of twenty; with a few dozen cells a
+    // thread the reduction itself would otherwise fill the FP64 pipe), and
+    // lanes 0, 8, 16, 24 end with mass, h, w and f.
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double v[4] = {acc.mass.get(), acc.h.get(), acc.w.get(), acc.f.get()};
+    const bool up = lane & 16, up2 = lane & 8;
+    double a0 = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
+    const double a1 = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
+    a0 = (up2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up2 ? a0 : a1, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+    __shared__ double red[8][4];
+    __shared__ int cnt[8][3];
+    if ((lane & 7) == 0) red[warp][lane >> 3] = a0;
+    const int n = __reduce_add_sync(0xffffffffu, acc.n), ns = __reduce_add_sync(0xffffffffu, acc.solid),
+              nb = __reduce_add_sync(0xffffffffu, acc.bad);
+    if (lane == 0) {
+        cnt[warp][0] = n;
+        cnt[warp][1] = ns;
+        cnt[warp][2] = nb;
     }
-    acc[2] = (double)nsolid;
-    acc[4] = (double)nbad;
-    acc[3] *= kd.vol;
-    block_sum_store<256, 5>(acc, partials, blockIdx.x);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t[4] = {0, 0, 0, 0};
+        int64_t u[3] = {0, 0, 0};
+        for (int q = 0; q < 8; ++q) {
+            for (int i = 0; i < 4; ++i) t[i] += red[q][i];
+            for (int i = 0; i < 3; ++i) u[i] += cnt[q][i];
+        }
+        double *o = partials + 5 * ((int64_t)blockIdx.x + (int64_t)gridDim.x * blockIdx.y);
+        o[0] = t[0];
+        o[1] = t[1];
+        o[2] = (double)u[1];
+        o[3] = k.vol * (t[3] + k.hA * t[2] + (double)u[0] * k.CL + k.dC * t[1]);
+        o[4] = (double)u[2];
+    }
+}
+
+// Blocks of the observables reduction: 256 groups of 16 bytes of cells, in
+// z chunks that give about three blocks per SM, what the registers let
+// reside at once (each chunk reads one plane more than it owns).
+static void observe_shape(const Geom &g, int group, int num_sms, int *nq, int *bx, int *zc, int *bz) {
+    *nq = (g.nx + group - 1) / group;
+    *bx = (int)(((int64_t)*nq * g.ny + 255) / 256);
+    int chunks = 3 * num_sms / *bx;
+    chunks = chunks < 1 ? 1 : chunks > g.nz ? g.nz : chunks;
+    *zc = (g.nz + chunks - 1) / chunks;
+    *bz = (g.nz + *zc - 1) / *zc;
 }
 
 template <typename T>
-cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, double *partials, int nblocks,
+int observe_blocks(const Geom &g, int num_sms) {
+    int nq, bx, zc, bz;
+    observe_shape(g, 16 / (int)sizeof(T), num_sms, &nq, &bx, &zc, &bz);
+    return bx * bz;
+}
+
+template <typename T>
+cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, double *partials, int num_sms,
                            cudaStream_t s) {
-    observe_kernel<T><<<nblocks, 256, 0, s>>>(g, k, f, partials);
+    int nq, bx, zc, bz;
+    observe_shape(g, 16 / (int)sizeof(T), num_sms, &nq, &bx, &zc, &bz);
+    ObsCoef<T> o;
+    o.cL0 = (T)k.cL0;
+    o.dc0 = (T)(k.cL0 - k.cS0);
+    o.AS = (T)k.AS;
+    o.dA = (T)k.dA;
+    o.m = (T)k.m;
+    o.kg = (T)k.kappa_h2_half;
+    o.g = (T)k.gamma;
+    o.eq = k.AS == k.AL;
+    o.hA = 0.5 * k.AS * (o.eq ? 1.0 : k.AL);
+    o.CL = k.CL;
+    o.dC = k.CS - k.CL;
+    o.vol = k.vol;
+    observe_kernel<T><<<dim3((unsigned)bx, (unsigned)bz), 256, 0, s>>>(g, o, f, nq, zc, partials);
     return cudaGetLastError();
 }
 
-__global__ void final_sum_kernel(const double *__restrict__ partials, int nblocks, int stride, int nvals,
-                                 double *out) {
-    __shared__ double red[256];
-    for (int v = 0; v < nvals; ++v) {
-        double s = 0;
-        for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partials[(int64_t)stride * b + v];
-        red[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = 128; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) out[v] = red[0];
-        __syncthreads();
-    }
+// one block per value: four independent chains of loads per thread, then a
+// fixed tree (the order depends only on the number of partial sums)
+__global__ void __launch_bounds__(256) final_sum_kernel(const double *__restrict__ partials, int nblocks, int stride,
+                                                        double *out) {
+    const double *p = partials + blockIdx.x;
+    double a[4] = {0, 0, 0, 0};
+    int b = threadIdx.x;
+    for (; b + 768 < nblocks; b += 1024)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] += p[(int64_t)stride * (b + 256 * q)];
+    for (; b < nblocks; b += 256) a[0] += p[(int64_t)stride * b];
+    double s[1] = {(a[0] + a[1]) + (a[2] + a[3])};
+    block_sum_store<256, 1>(s, out, blockIdx.x);
 }
 
 cudaError_t launch_final_sum(const double *partials, int nblocks, int stride, int nvals, double *out,
                              cudaStream_t s) {
-    final_sum_kernel<<<1, 256, 0, s>>>(partials, nblocks, stride, nvals, out);
+    final_sum_kernel<<<nvals, 256, 0, s>>>(partials, nblocks, stride, out);
     return cudaGetLastError();
 }
 
 // explicit instantiations
-template cudaError_t launch_pack<float>(const Geom &, const double *, Fields<float>, cudaStream_t);
-template cudaError_t launch_pack<double>(const Geom &, const double *, Fields<double>, cudaStream_t);
-template cudaError_t launch_unpack<float>(const Geom &, Fields<const float>, double *, cudaStream_t);
-template cudaError_t launch_unpack<double>(const Geom &, Fields<const double>, double *, cudaStream_t);
+template cudaError_t launch_pack<float>(const Geom &, const double *const[3], Fields<float>, cudaStream_t);
+template cudaError_t launch_pack<double>(const Geom &, const double *const[3], Fields<double>, cudaStream_t);
+template cudaError_t launch_unpack<float>(const Geom &, Fields<const float>, double *const[3], cudaStream_t);
+template cudaError_t launch_unpack<double>(const Geom &, Fields<const double>, double *const[3], cudaStream_t);
 template cudaError_t launch_pack_multi<float>(const IoDesc *, int, int64_t, cudaStream_t);
 template cudaError_t launch_pack_multi<double>(const IoDesc *, int, int64_t, cudaStream_t);
 template cudaError_t launch_unpack_multi<float>(const IoDesc *, int, int64_t, int, cudaStream_t);
@@ -292,5 +562,8 @@ template cudaError_t launch_observe<float>(const Geom &, const CoefD &, Fields<c
                                            cudaStream_t);
 template cudaError_t launch_observe<double>(const Geom &, const CoefD &, Fields<const double>, double *, int,
                                             cudaStream_t);
+
+template int observe_blocks<float>(const Geom &, int);
+template int observe_blocks<double>(const Geom &, int);
 
 }  // namespace ppf

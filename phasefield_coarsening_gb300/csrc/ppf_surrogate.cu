@@ -703,7 +703,9 @@ extern "C" int ppf_surrogate_predict(ppf_surrogate *s, ppf_ctx *c, double *out3)
     a.s1 = {o, o + T, o + 2 * T};
     a.mass_part = s->mpart;
     if ((rc = run_conv(s, c, s->ci[5], 16, EPI_STATE, a))) return rc;
-    SCU(launch_unpack<float>(c->g, Fields<const float>{o, o + T, o + 2 * T}, s->stage, c->stream));
+    const size_t cells = (size_t)c->nz * c->ny * c->nx;
+    double *const st3[3] = {s->stage, s->stage + cells, s->stage + 2 * cells};
+    SCU(launch_unpack<float>(c->g, Fields<const float>{o, o + T, o + 2 * T}, st3, c->stream));
     SCU(cudaMemcpyAsync(out3, s->stage, (size_t)3 * c->nz * c->ny * c->nx * sizeof(double), cudaMemcpyDeviceToHost,
                         c->stream));
     SCU(cudaStreamSynchronize(c->stream));
