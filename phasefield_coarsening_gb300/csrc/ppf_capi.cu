@@ -20,6 +20,7 @@
 #include "ppf.h"
 #include "ppf_internal.h"
 #include "ppf_particles.h"
+#include "ppf_step_fx.h"
 #include "ppf_step_tma.h"
 
 using namespace ppf;
@@ -177,6 +178,11 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
     c->kf = make_coef<float>(prm, der);
     c->kd = make_coef<double>(prm, der);
     c->eqA = prm.AS == prm.AL;
+    if (precision == PPF_F64) {
+        const Coef<double> &k = c->kd;
+        c->fx_ok = c->g.total <= ((int64_t)1 << 32) &&
+                   fx::make_fxcoef(prm.AS, prm.AL, k.cL0, k.dc0, k.Mt0, k.Mt1, k.dC, k.q1, k.dm2, k.mt, k.tg, k.kt, &c->kx);
+    }
     c->cd.AS = prm.AS; c->cd.AL = prm.AL; c->cd.dA = prm.AL - prm.AS;
     c->cd.cS0 = prm.cS0; c->cd.cL0 = prm.cL0; c->cd.CS = prm.CS; c->cd.CL = prm.CL;
     c->cd.tmp2 = prm.AS * prm.cS0 - prm.AL * prm.cL0;
@@ -197,6 +203,7 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
     c->stream = c->own;
     c->derr = (int *)(c->dres + 32);
     c->dsched = c->derr + 4;
+    c->dbox = own_box(c);
     c->wait_limit_ns = 1000000000ULL;
     for (int b = 0; b < 2; ++b)
         for (int f = 0; f < 3; ++f) c->fld[b][f] = (char *)c->state + (size_t)(3 * b + f) * fbytes;
@@ -218,7 +225,7 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
     c->tune.split = kStepSplit;
     c->tune.grid = precision == PPF_F32 ? tma_grid<float>(c->g, c->num_sms, &c->tune.zc)
                                         : tma_grid<double>(c->g, c->num_sms, &c->tune.zc);
-    if (c->tune.grid < 1) {
+    if (c->tune.grid < 1 || (c->fx_ok && fx_occupancy(false) < 1)) {
         ppf_destroy(c);
         return seterr(PPF_ECUDA, "kernel attribute setup failed");
     }
@@ -268,8 +275,11 @@ extern "C" int ppf_set_stream(ppf_ctx *c, void *stream) {
 static int pack_from(ppf_ctx *c, const double *const src[3]) {
     c->cur_eta = 0;
     c->cur_c = 0;
-    if (c->prec == PPF_F32) CU(launch_pack<float>(c->g, src, ff(c, 0, 0), c->stream));
-    else CU(launch_pack<double>(c->g, src, fd(c, 0, 0), c->stream));
+    // (slabs of one domain share the first one's words, cleared with its upload)
+    if (c->fx_ok && !c->shared_box) CU(cudaMemsetAsync(c->dbox, 0, 2 * sizeof(int), c->stream));
+    const BoxCheck box = {c->fx_ok ? c->dbox : nullptr, c->kx.cmax};
+    if (c->prec == PPF_F32) CU(launch_pack<float>(c->g, src, ff(c, 0, 0), box, c->stream));
+    else CU(launch_pack<double>(c->g, src, fd(c, 0, 0), box, c->stream));
     CU(cudaMemsetAsync(c->dres, 0, 3 * sizeof(double), c->stream));
     c->uploaded = 1;
     c->steps = 0;
@@ -331,6 +341,24 @@ static bool direct_io(ppf_ctx *c, const double *const p[3]) {
     return true;
 }
 
+// Waits for the stream, and learns whether the uploaded state lies outside
+// the fixed-point step's box (its steps are then launched in float64).
+static int read_box(ppf_ctx *c) {
+    int h = 0;
+    if (c->fx_ok) CU(cudaMemcpyAsync(&h, c->dbox, sizeof h, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaStreamSynchronize(c->stream));
+    c->left_box = h != 0;
+    return PPF_OK;
+}
+
+int recheck_box(ppf_ctx *c) {
+    if (c->fx_ok) {
+        CU(cudaMemsetAsync(c->dbox, 0, 2 * sizeof(int), c->stream));
+        CU(launch_box_check(c->g, cst(fd(c, 0, 0)), BoxCheck{c->dbox, c->kx.cmax}, c->stream));
+    }
+    return read_box(c);
+}
+
 extern "C" int ppf_upload(ppf_ctx *c, const double *etaS, const double *etaL, const double *cc) {
     if (!c || !etaS || !etaL || !cc) return seterr(PPF_EINVAL, "null argument");
     const size_t n = (size_t)c->nz * c->ny * c->nx;
@@ -339,8 +367,7 @@ extern "C" int ppf_upload(ppf_ctx *c, const double *etaS, const double *etaL, co
     CU(cudaMemcpyAsync(c->staging + 2 * n, cc, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     int rc = do_pack(c);
     if (rc) return rc;
-    CU(cudaStreamSynchronize(c->stream));
-    return PPF_OK;
+    return read_box(c);
 }
 
 extern "C" int ppf_upload_device(ppf_ctx *c, const double *etaS, const double *etaL, const double *cc) {
@@ -356,8 +383,7 @@ extern "C" int ppf_upload_device(ppf_ctx *c, const double *etaS, const double *e
         rc = do_pack(c);
     }
     if (rc) return rc;
-    CU(cudaStreamSynchronize(c->stream));
-    return PPF_OK;
+    return read_box(c);
 }
 
 extern "C" int ppf_download(ppf_ctx *c, double *etaS, double *etaL, double *cc) {
@@ -392,10 +418,11 @@ extern "C" int ppf_download_device(ppf_ctx *c, double *etaS, double *etaL, doubl
 // Reads and clears the device error word; PPF_ETIMEOUT when a kernel's
 // bounded wait ran out since the last check.
 int check_device_error(ppf_ctx *c) {
-    int h = 0;
-    CU(cudaMemcpyAsync(&h, c->derr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    int w[10] = {0};   // the error word, ..., the context's own box words
+    CU(cudaMemcpyAsync(w, c->derr, sizeof w, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    if (h) {
+    if (c->fx_ok && c->dbox == own_box(c) && w[8 + c->cur_c]) c->left_box = 1;
+    if (w[0]) {
         // the error word, and the scheduler pairs that an abandoned step may leave set
         CU(cudaMemsetAsync(c->derr, 0, 8 * sizeof(int), c->stream));
         CU(cudaStreamSynchronize(c->stream));
@@ -428,8 +455,12 @@ static int run_steps(ppf_ctx *c, int64_t nsteps, bool c_only) {
                                        c->derr, c->wait_limit_ns, inject, c->dsched, c->stream);
         } else {
             const CUtensorMap m[3] = {c->maps[0][ie][0], c->maps[0][ie][1], c->maps[0][ic][2]};
-            e = launch_step_tma<double>(c->g, c->kd, m, fd(c, oe, oc), c_only, c->eqA, part, c->tune,
-                                        c->derr, c->wait_limit_ns, inject, c->dsched, c->stream);
+            if (fx_step(c))
+                e = launch_step_fx(c->g, c->kd, c->kx, m, cst(fd(c, ie, ic)), fd(c, oe, oc), c_only, part, c->tune,
+                                   c->derr, c->wait_limit_ns, inject, c->dsched, c->dbox, ic, c->stream);
+            else
+                e = launch_step_tma<double>(c->g, c->kd, m, fd(c, oe, oc), c_only, c->eqA, part, c->tune,
+                                            c->derr, c->wait_limit_ns, inject, c->dsched, c->stream);
         }
         if (e != cudaSuccess) return seterr(PPF_ECUDA, "step launch failed: %s", cudaGetErrorString(e));
         c->cur_eta = oe;
@@ -452,9 +483,10 @@ extern "C" int ppf_reduce(ppf_ctx *c, ppf_stats *out) {
     int rc = ensure_partials(c, 5 * nb);
     if (rc) return rc;
     if (c->prec == PPF_F32)
-        CU(launch_observe<float>(c->g, c->cd, cst(ff(c, c->cur_eta, c->cur_c)), c->partials, c->num_sms, c->stream));
+        CU(launch_observe<float>(c->g, c->cd, nullptr, cst(ff(c, c->cur_eta, c->cur_c)), c->partials, c->num_sms, c->stream));
     else
-        CU(launch_observe<double>(c->g, c->cd, cst(fd(c, c->cur_eta, c->cur_c)), c->partials, c->num_sms, c->stream));
+        CU(launch_observe<double>(c->g, c->cd, c->fx_ok ? &c->kx : nullptr, cst(fd(c, c->cur_eta, c->cur_c)), c->partials,
+                                  c->num_sms, c->stream));
     CU(launch_final_sum(c->partials, nb, 5, 5, c->dres + 3, c->stream));
     double h[8];
     CU(cudaMemcpyAsync(h, c->dres, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));

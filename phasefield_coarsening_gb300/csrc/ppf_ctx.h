@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "ppf.h"
+#include "ppf_fx.h"
 #include "ppf_internal.h"
 #include "ppf_step_tma.h"
 
@@ -41,11 +42,22 @@ struct ppf_ctx {
     ppf::Coef<float> kf;
     ppf::Coef<double> kd;
     int eqA;              // AS == AL: the mu reciprocal is a constant
+    ppf::fx::FxCoef kx;   // FP64: coefficients of the fixed-point step
+    int fx_ok;            // FP64: the parameters and the grid fit the fixed-point step
+    int left_box;         // the host knows that the state has left the fixed-point step's box
+    int shared_box;       // dbox belongs to another slab of the same domain
+    int *dbox;            // box words of the two buffers (launch_step_fx): the context's own, behind the
+                          // scheduler words, or shared with the slabs of one domain / in the ensemble's array
     ppf::CoefD cd;
 };
 
 // helpers of ppf_capi.cu (return PPF_* codes, set ppf_last_error)
 int ensure_partials(ppf_ctx *c, int ndoubles);
-int do_pack(ppf_ctx *c);        // staging -> state buffer 0 (+ ghosts)
+int do_pack(ppf_ctx *c);        // staging -> state buffer 0 (+ ghosts, box word)
 int do_unpack(ppf_ctx *c);      // current state -> staging
 int check_device_error(ppf_ctx *c);
+// FP64: sets the box words for the state in buffer 0 and learns of them; waits for the stream
+int recheck_box(ppf_ctx *c);
+inline int *own_box(ppf_ctx *c) { return c->derr + 8; }
+// whether the next FP64 step runs in fixed-point arithmetic
+inline bool fx_step(const ppf_ctx *c) { return c->fx_ok && !c->left_box; }

@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "ppf_ctx.h"
+#include "ppf_step_fx.h"
 
 using namespace ppf;
 
@@ -74,6 +75,7 @@ struct ppf_ensemble {
     double **ddres;              // device: each domain's dres pointer
     IoDesc *dio;                 // device: each domain's batched-I/O descriptor (domain order)
     int64_t max_rows;           // x rows of the domain with most of them
+    int *boxes;                  // device: the domains' box words (FP64, launch_step_fx), two each in domain order
     double *partials;            // 3 doubles per work item
     int partials_cap;
     int items[3];                // work items of the edge-tile [0], whole-tile [1] and every-tile [2] launches
@@ -87,7 +89,7 @@ struct ppf_ensemble {
     int64_t steps;
     cudaStream_t stream;
     cudaGraphExec_t graph;       // kGraphSteps plain steps, starting and ending at parity 0
-    int graph_ok;
+    int graph_ok, graph_fx;      // graph_fx: of fixed-point steps
     int num_sms;
 };
 
@@ -109,6 +111,7 @@ static int build_table(ppf_ensemble *e) {
                 t.fld[b][f] = c->fld[b][f];
             }
         t.g = c->g;
+        t.box = c->dbox;
         t.ntx = (c->nx + tx - 1) / tx;
         t.nty = (c->ny + ty - 1) / ty;
         t.nfx = c->nx / tx;
@@ -144,12 +147,24 @@ static int build_table(ppf_ensemble *e) {
     return PPF_OK;
 }
 
+// whether the next step runs in fixed-point arithmetic (the kernel computes
+// domains that leave the box later in float64)
+static bool fx_ensemble(const ppf_ensemble *e) {
+    for (const ppf_ctx *c : e->dom)
+        if (!fx_step(c)) return false;
+    return true;
+}
+
 static int launch_one(ppf_ensemble *e, bool stats) {
     const int inj = 0;
     (void)inj;
     ppf_ctx *c0 = e->dom[0];
     cudaError_t r;
-    if (e->prec == PPF_F32)
+    if (fx_ensemble(e))
+        r = launch_step_fx_multi(e->dtable, e->n, e->items, c0->kd, c0->kx, e->parity, stats ? e->partials : nullptr,
+                                 e->grid, e->pdl != 0, e->split != 0, c0->derr, c0->wait_limit_ns,
+                                 e->sched ? c0->dsched : nullptr, e->stream);
+    else if (e->prec == PPF_F32)
         r = launch_step_multi<float>(e->dtable, e->n, e->items, c0->kf, false, e->eqA, e->parity,
                                      stats ? e->partials : nullptr, e->grid, e->roll, e->pdl != 0, e->split != 0,
                                      e->tile, c0->derr, c0->wait_limit_ns, e->sched ? c0->dsched : nullptr, e->stream);
@@ -163,7 +178,10 @@ static int launch_one(ppf_ensemble *e, bool stats) {
 }
 
 static int ensure_graph(ppf_ensemble *e) {
-    if (e->graph_ok) return PPF_OK;
+    if (e->graph_ok && e->graph_fx == (int)fx_ensemble(e)) return PPF_OK;
+    if (e->graph_ok) cudaGraphExecDestroy(e->graph);
+    e->graph_ok = 0;
+    e->graph_fx = fx_ensemble(e);
     cudaGraph_t g;
     const int p0 = e->parity;
     e->parity = 0;
@@ -189,6 +207,7 @@ extern "C" int ppf_ensemble_destroy(ppf_ensemble *e) {
     if (e->dtable) cudaFree(e->dtable);
     if (e->ddres) cudaFree(e->ddres);
     if (e->dio) cudaFree(e->dio);
+    if (e->boxes) cudaFree(e->boxes);
     if (e->partials) cudaFree(e->partials);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
@@ -233,6 +252,9 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
     if (ce == cudaSuccess) ce = cudaMalloc(&e->dtable, (size_t)n * sizeof(DomainDesc));
     if (ce == cudaSuccess) ce = cudaMalloc(&e->ddres, (size_t)n * sizeof(double *));
     if (ce == cudaSuccess) ce = cudaMalloc(&e->dio, (size_t)n * sizeof(IoDesc));
+    if (ce == cudaSuccess) ce = cudaMalloc(&e->boxes, (size_t)n * 2 * sizeof(int));
+    if (ce == cudaSuccess) ce = cudaMemset(e->boxes, 0, (size_t)n * 2 * sizeof(int));
+    if (ce == cudaSuccess && c0->fx_ok && fx_occupancy(true) < 1) ce = cudaErrorInvalidConfiguration;
     if (ce != cudaSuccess) {
         ppf_ensemble_destroy(e);
         return err_(PPF_ECUDA, "ensemble setup: %s", cudaGetErrorString(ce));
@@ -247,7 +269,10 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
     });
     std::vector<double *> h((size_t)n);
     for (int k = 0; k < n; ++k) h[(size_t)k] = e->dom[(size_t)e->order[(size_t)k]]->dres;
-    for (int d = 0; d < n; ++d) e->dom[(size_t)d]->stream = e->stream;   // one stream orders every domain's work
+    for (int d = 0; d < n; ++d) {
+        e->dom[(size_t)d]->stream = e->stream;   // one stream orders every domain's work
+        e->dom[(size_t)d]->dbox = e->boxes + 2 * d;
+    }
     ce = cudaMemcpy(e->ddres, h.data(), (size_t)n * sizeof(double *), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) {
         std::vector<IoDesc> io((size_t)n);
@@ -260,6 +285,7 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
             for (int b = 0; b < 2; ++b)
                 for (int f = 0; f < 3; ++f) t.fld[b][f] = x->fld[b][f];
             t.dres = x->dres;
+            t.box = {x->fx_ok ? x->dbox : nullptr, x->kx.cmax};
             const int64_t rows = (int64_t)x->nz * x->ny;
             if (rows > e->max_rows) e->max_rows = rows;
         }
@@ -326,6 +352,7 @@ extern "C" int ppf_ensemble_upload_all(ppf_ensemble *e, const double *const *eta
         ECU(cudaMemcpyAsync(x->staging + n, etaL[d], n * sizeof(double), cudaMemcpyHostToDevice, e->stream));
         ECU(cudaMemcpyAsync(x->staging + 2 * n, c[d], n * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     }
+    ECU(cudaMemsetAsync(e->boxes, 0, (size_t)e->n * 2 * sizeof(int), e->stream));
     if (e->prec == PPF_F32) ECU(launch_pack_multi<float>(e->dio, e->n, e->max_rows, e->stream));
     else ECU(launch_pack_multi<double>(e->dio, e->n, e->max_rows, e->stream));
     for (ppf_ctx *x : e->dom) {
@@ -334,7 +361,10 @@ extern "C" int ppf_ensemble_upload_all(ppf_ensemble *e, const double *const *eta
         x->steps = 0;
     }
     e->parity = 0;
+    std::vector<int> box((size_t)e->n * 2);
+    ECU(cudaMemcpyAsync(box.data(), e->boxes, box.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     ECU(cudaStreamSynchronize(e->stream));
+    for (int d = 0; d < e->n; ++d) e->dom[(size_t)d]->left_box = box[2 * (size_t)d] != 0;
     return PPF_OK;
 }
 

@@ -1,0 +1,257 @@
+// ppf_fx.h -- the cell arithmetic of the float64 step in 64-bit fixed point.
+//
+// The float64 step is bound by this GPU's FP64 pipe (1/64 of the FP32 and
+// integer rates: about 75 FP64 operations per cell-step, 85 % of the pipe
+// busy).  Every quantity of the step but the state itself is bounded once
+// the state lies in a box (|eta| < 1.75, eta_S^2 + eta_L^2 >= 1/4, |c| below
+// twice a power of two above the parabola minima), so it is held here as a
+// 64-bit integer with a fixed binary scale ("x@s" is x 2^s).  The absolute
+// resolution of the products, 2^-56 to 2^-59, is finer than the rounding of
+// the same values in float64 (2^-53 to 2^-54 near 1), and the increments are
+// added to the float64 state with one rounding (a fused multiply-add), so
+// the result is no less accurate than float64 arithmetic throughout;
+// integer sums are exact, and a face's flux is the same number with the
+// opposite sign seen from its other side.  A product is three 32 x 32 ->
+// 64-bit multiply-adds.
+//
+// Functions are host-callable, so that their accuracy can be measured
+// against extended precision without a GPU.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+namespace ppf {
+namespace fx {
+
+#ifdef __CUDACC__
+#define PPF_FX __host__ __device__ __forceinline__
+#else
+#define PPF_FX inline
+#endif
+
+typedef long long i64;
+
+// the box
+constexpr double kEtaMax = 1.75;     // |eta| below
+constexpr double kS2Min = 0.25;      // eta_S^2 + eta_L^2 at least
+
+// Coefficients (see Coef in ppf_internal.h), as integers at the scales that
+// the products below need, and the scales of the results.
+struct FxCoef {
+    i64 cL0;       // @59, in units of 2^ec
+    i64 dc0;       // @62
+    i64 m0, m1;    // A M' = m0 + m1 h: m0@64, m1@65
+    i64 k0, k1;    // drive k = k0 + k1 w, in units of 2^eu: k0@60, k1@65
+    i64 mt, mtg;   // mt and mt (2 gamma - 1) @68, units of 2^eu
+    i64 nkt;       // @66, units of 2^eu
+    i64 g;         // gamma @61
+    double su, sc; // 2^(eu-59), 2^(ec-59): increments of eta and c
+    int ec, eu;
+    unsigned cmax; // high word of the box bound of |c|, 2^(ec+1)
+};
+
+PPF_FX int hi32(i64 v) { return (int)(v >> 32); }
+PPF_FX unsigned lo32(i64 v) { return (unsigned)v; }
+PPF_FX i64 wide(int a, int b) { return (i64)a * (i64)b; }
+
+// a b / 2^64, rounded to nearest (up to the neglected low x low part, a
+// quarter of the last unit): the words of an operand are rebalanced so that
+// the low one is signed.  |a|, |b| <= 2^62.
+PPF_FX i64 mulq(i64 a, i64 b) {
+    const int al = (int)lo32(a), bl = (int)lo32(b);
+    const int ah = hi32(a) + (int)(lo32(a) >> 31), bh = hi32(b) + (int)(lo32(b) >> 31);
+    const i64 cross = wide(ah, bl) + (wide(al, bh) + 0x80000000ll);
+    return wide(ah, bh) + (i64)hi32(cross);
+}
+
+// The same with X more bits of the product, a b / 2^(64-X): the cross
+// products' low bits are kept and the low x low part is added to them.
+template <int X>
+PPF_FX i64 mulx(i64 a, i64 b) {
+    const int al = (int)lo32(a), bl = (int)lo32(b);
+    const int ah = hi32(a) + (int)(lo32(a) >> 31), bh = hi32(b) + (int)(lo32(b) >> 31);
+    const i64 low = (i64)hi32(wide(al, bl)) + (1ll << (31 - X));
+    const i64 cross = wide(ah, bl) + (wide(al, bh) + low);
+    return (i64)((unsigned long long)wide(ah, bh) << X) + (cross >> (32 - X));
+}
+
+// v 2^(1085 - bias), |v| < 2^(bias - 1022); truncated towards zero.  Exact for values
+// whose last bit is a unit or more.
+PPF_FX i64 to_fx(int hi, unsigned lo, int bias) {
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const unsigned long long m = ((unsigned long long)((mh << 10) | (lo >> 22)) << 32) | (lo << 10);
+    const int sh = bias - e;
+    const i64 a = (i64)(m >> (sh > 63 ? 63 : sh));
+    const i64 s = hi >> 31;
+    return (a ^ s) - s;
+}
+PPF_FX i64 to_fx(double v, int bias) {
+#ifdef __CUDA_ARCH__
+    return to_fx(__double2hiint(v), (unsigned)__double2loint(v), bias);
+#else
+    uint64_t b;
+    std::memcpy(&b, &v, 8);
+    return to_fx((int)(uint32_t)(b >> 32), (unsigned)b, bias);
+#endif
+}
+constexpr int kEtaBias = 1085 - 61;            // eta@61
+PPF_FX int c_bias(int ec) { return 1085 - 59 + ec; }   // c@59 in units of 2^ec
+
+// 1/s2 @60 for s2@60 in [1/4, 6.2): a 20-bit estimate R0 from the float
+// reciprocal of the leading bits, then R0 (1 + e + e^2) with
+// e = 1 - s2 R0 exact (the third-order Newton step; the remainder e^3 is
+// below 2^-60).
+PPF_FX i64 recip(i64 s2) {
+    const float f = (float)hi32(s2);           // s2@28
+#ifdef __CUDA_ARCH__
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+    const unsigned r0 = __float2uint_rn(y * 1125899906842624.0f);   // 2^50: R0@22
+#else
+    const unsigned r0 = (unsigned)lrintf(1.0f / f * 1125899906842624.0f);
+#endif
+    // e@82 = 2^82 - s2 R0, modulo 2^64
+    const i64 e = -(i64)((unsigned long long)s2 * (unsigned long long)r0);
+    const int eh = hi32(e);                    // @50
+    const i64 t = e + (wide(eh, eh) >> 18);    // e + e^2 @82
+    // R0 t @104 -> @72 -> @60
+    const i64 v = wide((int)r0, hi32(t)) + (i64)(unsigned)(((unsigned long long)r0 * lo32(t)) >> 32);
+    return ((i64)r0 << 38) + ((v + (1ll << 11)) >> 12);
+}
+
+// what a cell's neighbours need
+struct Nb {
+    i64 S, L;      // eta @57
+    i64 W, M;      // w @59 in units of 2^ec, A M' @64
+};
+// what the cell itself needs besides
+struct Own {
+    i64 h;         // @61
+    i64 G;         // drive k / (etaS^2 + etaL^2) @59, units of 2^eu
+};
+
+template <bool C_ONLY>
+PPF_FX void pass_a(const FxCoef &k, double eS, double eL, double c, int cbias, Nb &n, Own &o) {
+    const i64 S = to_fx(eS, kEtaBias), L = to_fx(eL, kEtaBias);
+    const i64 S2 = mulx<2>(S, S), L2 = mulx<2>(L, L);        // @60
+    const i64 R = recip(S2 + L2);                            // @60
+    const i64 h = mulx<5>(S2, R);                            // @61
+    const i64 C = to_fx(c, cbias);                           // @59
+    n.W = C - k.cL0 + mulq(k.dc0, h);
+    n.M = k.m0 + (mulq(k.m1, h) << 2);
+    if (!C_ONLY) {
+        n.S = S >> 4;
+        n.L = L >> 4;
+        o.h = h;
+        o.G = mulx<3>(k.k0 + mulq(k.k1, n.W), R);            // @59
+    }
+}
+
+// (M' + M)(mu' - mu) of one face, @59
+PPF_FX i64 face(i64 Mn, i64 M, i64 Wn, i64 W) { return mulq(Mn + M, Wn - W); }
+
+// the increments of etaS and etaL @59 (units of 2^eu): phasefield.c:360-373,
+// from the cell's own values S, L @57 and the sums S6, L6 of its six
+// neighbours' @57
+PPF_FX void eta_inc(const FxCoef &k, const Own &o, i64 S, i64 L, i64 S6, i64 L6, i64 &dS, i64 &dL) {
+    const i64 lS = S6 - 6 * S, lL = L6 - 6 * L;
+    S <<= 4;                                                                                         // @61
+    L <<= 4;
+    // mt eta (eta^2 - 1 + 2 gamma other^2), as eta (mt (etaS^2 + etaL^2 - 1) + mt (2 gamma - 1) other^2)
+    const i64 S2 = mulq(S, S), L2 = mulq(L, L);                                                      // @58
+    const i64 u = mulq(k.mt, S2 + L2 - (1ll << 58));                                                 // @62
+    const i64 wS = mulq(S, u + mulq(k.mtg, L2)), wL = mulq(L, u + mulq(k.mtg, S2));                  // @59
+    const i64 aS = mulq(S, (1ll << 61) - o.h), aL = mulq(L, o.h);                                    // @58
+    dS = wS + mulq(k.nkt, lS) + mulx<6>(aS, o.G);
+    dL = wL + mulq(k.nkt, lL) - mulx<6>(aL, o.G);
+}
+
+// A cell's terms of the observables: c @59 and w^2 @59 (in units of 2^ec and
+// 2^(2 ec)), hS @61 and the well energy f0 @53 (its constant 1/4 included).
+PPF_FX void observe(const FxCoef &k, double eS, double eL, double c, int cbias, i64 &C, i64 &h, i64 &w2, i64 &f0) {
+    const i64 S = to_fx(eS, kEtaBias), L = to_fx(eL, kEtaBias);
+    const i64 S2 = mulx<2>(S, S), L2 = mulx<2>(L, L);                                                // @60
+    C = to_fx(c, cbias);
+    h = mulx<5>(S2, recip(S2 + L2));
+    const i64 W = C - k.cL0 + mulq(k.dc0, h);
+    w2 = mulx<5>(W, W);
+    // S2 (S2/4 - 1/2 + gamma L2) + L2 (L2/4 - 1/2) + 1/4, the factors @57
+    const i64 xS = (S2 >> 5) - (1ll << 56) + mulq(k.g, L2), xL = (L2 >> 5) - (1ll << 56);
+    f0 = mulq(S2, xS) + mulq(L2, xL) + (1ll << 51);
+}
+
+// Whether a state cell lies in the box, from the high words alone (a margin
+// of 2^-20 relative towards "no"); NaN and infinities do not.
+PPF_FX int hi_fx26(unsigned hi) {              // v @26, truncated, for the high word of 0 <= v < 2
+    const int e = (int)(hi >> 20), sh = 1023 - e;
+    const unsigned m = ((hi & 0xfffffu) | 0x100000u) << 6;
+    return (int)(m >> (sh > 31 ? 31 : sh));
+}
+PPF_FX bool in_box_eta(unsigned hS, unsigned hL) {
+    const unsigned m = hS > hL ? hS : hL;
+    if (m >= 0x3ffc0000u) return false;        // 1.75
+    if (m >= 0x3fe00000u) return true;         // one of them at least 1/2
+    const int s = hi_fx26(hS), l = hi_fx26(hL);
+    return (i64)s * s + (i64)l * l >= (1ll << 50) + (1ll << 32);   // 1/4 @52
+}
+PPF_FX bool in_box_c(unsigned hC, unsigned cmax) { return (hC & 0x7fffffffu) < cmax; }
+
+// The coefficients for a parameter set; false when they do not fit (AS !=
+// AL, a time step above the solute equation's explicit limit, phase-field
+// rates so large that their increments would lose resolution): then the
+// step stays in float64 arithmetic.  `A` .. `kt` as in Coef<double>.
+inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0, double Mt1, double dC, double q1,
+                        double dm2, double mt, double tg, double kt, FxCoef *out) {
+    if (AS != AL) return false;
+    const double all[] = {AS, cL0, dc0, Mt0, Mt1, dC, q1, dm2, mt, tg, kt};
+    for (double v : all)
+        if (!std::isfinite(v)) return false;
+    FxCoef f;
+    const double cmag = std::fmax(std::fabs(cL0), std::fmax(std::fabs(cL0 - dc0), std::fabs(dc0)));
+    int ec = 0;
+    if (cmag > 0) {
+        std::frexp(cmag, &ec);                 // cmag < 2^ec
+    }
+    if (ec < -500 || ec > 500) return false;
+    // (products of coefficients in extended precision: rounded once, here)
+    typedef long double ld;
+    const ld m0 = (ld)AS * Mt0, m1 = (ld)AS * Mt1;
+    if (!(m0 >= 0 && m0 <= 1.0 / 12 && m0 + m1 >= 0 && m0 + m1 <= 1.0 / 12)) return false;
+    if (!(std::fabs(tg) < 4)) return false;
+    // drive of tmp1 dmu: dm2 (dC - q1 mu) = k0 + k1 w, w in units of 2^ec
+    const ld k0 = (ld)dm2 * dC, k1 = -(ld)dm2 * q1 * AS * std::ldexp(1.0, ec);
+    const double a0 = std::fabs((double)k0), a1 = std::fabs((double)k1);
+    const double need = std::fmax(std::fmax(8.0 * a1, 2.0 * (a0 + 3.5 * a1)),
+                                  std::fmax(1024.0 * std::fabs(mt), 32.0 * std::fabs(kt)));
+    int eu = -40;
+    if (need > 0) {
+        int e;
+        std::frexp(need, &e);                  // need < 2^e
+        if (e > eu) eu = e;
+    }
+    if (eu > 0) return false;                  // increments coarser than 2^-59
+    auto q = [](ld v, int s) { return (i64)std::llrint(std::ldexp(v, s)); };
+    f.cL0 = q(cL0, 59 - ec);
+    f.dc0 = q(dc0, 62 - ec);
+    f.m0 = q(m0, 64);
+    f.m1 = q(m1, 65);
+    f.k0 = q(k0, 60 - eu);
+    f.k1 = q(k1, 65 - eu);
+    f.mt = q(mt, 68 - eu);
+    f.mtg = q((ld)mt * ((ld)tg - 1), 68 - eu);
+    f.nkt = q(-kt, 66 - eu);
+    f.g = q(0.5 * tg, 61);
+    f.su = std::ldexp(1.0, eu - 59);
+    f.sc = std::ldexp(1.0, ec - 59);
+    f.ec = ec;
+    f.eu = eu;
+    f.cmax = (unsigned)(1023 + ec + 1) << 20;
+    *out = f;
+    return true;
+}
+
+}  // namespace fx
+}  // namespace ppf

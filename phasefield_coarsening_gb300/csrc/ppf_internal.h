@@ -68,10 +68,19 @@ struct Fields {
 // Pack/unpack between three compact double arrays [z][y][x] (8-byte aligned
 // device memory, not overlapping) and the padded layout; pack also writes
 // the face ghosts (the BC fill of :207-211).
+// With `box.word` set (FP64), *box.word becomes 1 when a cell lies outside
+// the fixed-point step's box (ppf_fx.h; cmax as in FxCoef).
+struct BoxCheck {
+    int *word;
+    unsigned cmax;
+};
 template <typename T>
-cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, cudaStream_t s);
+cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, BoxCheck box, cudaStream_t s);
 template <typename T>
 cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[3], cudaStream_t s);
+
+// The box check alone, on a state.
+cudaError_t launch_box_check(const Geom &g, Fields<const double> f, BoxCheck box, cudaStream_t s);
 
 // One domain of a batched pack / unpack (device table): its geometry, its
 // compact float64 staging array (3 fields), its two state buffers and its
@@ -81,10 +90,11 @@ struct IoDesc {
     double *staging;
     void *fld[2][3];
     double *dres;
+    BoxCheck box;   // word: that of buffer 0
 };
 
 // Pack every domain's staging into its buffer 0 (clearing its increment
-// sums), or unpack every domain's buffer `buf` into its staging: one launch
+// sums; the caller clears the box words), or unpack every domain's buffer `buf` into its staging: one launch
 // for `n` domains (grid y = domain), the largest holding max_rows x rows.
 template <typename T>
 cudaError_t launch_pack_multi(const IoDesc *table, int n, int64_t max_rows, cudaStream_t s);
@@ -96,8 +106,12 @@ cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_rows, in
 // for b < observe_blocks.
 template <typename T>
 int observe_blocks(const Geom &g, int num_sms);
+// `kx` (FP64, may be null): the fixed-point step's coefficients.
+namespace fx {
+struct FxCoef;
+}
 template <typename T>
-cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, double *partials,
+cudaError_t launch_observe(const Geom &g, const CoefD &k, const fx::FxCoef *kx, Fields<const T> f, double *partials,
                            int num_sms, cudaStream_t s);
 
 // Record `msg` as the calling thread's ppf_last_error() text; returns code.

@@ -114,6 +114,10 @@ extern "C" int ppf_slabs_create(int nz, int ny, int nx, int nslabs, const ppf_pa
         if (rc == PPF_OK) {
             s->ctx.push_back(c);
             rc = ppf_set_stream(c, s->stream);
+            // a slab's ghost planes come from its neighbours: the slabs leave
+            // the fixed-point step's box together
+            c->dbox = own_box(s->ctx[0]);
+            c->shared_box = c != s->ctx[0];
         }
     }
     if (rc) {
@@ -158,7 +162,10 @@ extern "C" int ppf_slabs_upload(ppf_slabs *s, const double *etaS, const double *
     }
     int rc = exchange(s);
     if (rc) return rc;
+    int h = 0;
+    SCU(cudaMemcpyAsync(&h, s->ctx[0]->dbox, sizeof h, cudaMemcpyDeviceToHost, s->stream));
     SCU(cudaStreamSynchronize(s->stream));
+    for (ppf_ctx *c : s->ctx) c->left_box = h != 0;
     return PPF_OK;
 }
 

@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "ppf_fx.h"
 #include "ppf_internal.h"
 #include "ppf_pair.h"
 
@@ -89,9 +90,15 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double *partial
 
 constexpr int kRowWarps = 8;   // rows per block and pass
 
+__device__ __forceinline__ bool out_of_box(double s, double l, double c, unsigned cmax) {
+    return !fx::in_box_eta((unsigned)__double2hiint(s) & 0x7fffffffu, (unsigned)__double2hiint(l) & 0x7fffffffu) ||
+           !fx::in_box_c((unsigned)__double2hiint(c), cmax);
+}
+
 template <typename T>
 __device__ __forceinline__ void pack_rows(const Geom &g, const double *__restrict__ s0, const double *__restrict__ s1,
-                                          const double *__restrict__ s2, const Fields<T> &dst) {
+                                          const double *__restrict__ s2, const Fields<T> &dst, BoxCheck box) {
+    bool bad = false;
     const int lane = threadIdx.x & 31;
     const int nrows = g.ny * g.nz;
     for (int r = blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < nrows; r += gridDim.x * kRowWarps) {
@@ -102,6 +109,8 @@ __device__ __forceinline__ void pack_rows(const Geom &g, const double *__restric
 #pragma unroll 4
         for (int x = lane; x < g.nx; x += 32) {
             const T s = (T)s0[i0 + x], l = (T)s1[i0 + x], c = (T)s2[i0 + x];
+            if (std::is_same<T, double>::value && box.word)
+                bad = bad || out_of_box(s, l, c, box.cmax);
             if (inner && x > 0 && x < g.nx - 1) {
                 dst.eS[a0 + x] = s;
                 dst.eL[a0 + x] = l;
@@ -111,6 +120,7 @@ __device__ __forceinline__ void pack_rows(const Geom &g, const double *__restric
             }
         }
     }
+    if (bad) *box.word = 1;
 }
 
 // A float as a double.  The conversion instruction runs at the FP64 rate,
@@ -162,8 +172,8 @@ __device__ __forceinline__ void unpack_rows(const Geom &g, const T *__restrict__
 
 template <typename T>
 __global__ void __launch_bounds__(32 * kRowWarps) pack_kernel(Geom g, const double *s0, const double *s1,
-                                                              const double *s2, Fields<T> dst) {
-    pack_rows<T>(g, s0, s1, s2, dst);
+                                                              const double *s2, Fields<T> dst, BoxCheck box) {
+    pack_rows<T>(g, s0, s1, s2, dst, box);
 }
 
 template <typename T>
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) pack_multi_kernel(const IoDesc
     const Fields<T> dst = {(T *)d.fld[0][0], (T *)d.fld[0][1], (T *)d.fld[0][2]};
     if (blockIdx.x == 0 && threadIdx.x < 3) d.dres[threadIdx.x] = 0.0;
     const int64_t n = (int64_t)g.nx * g.ny * g.nz;
-    pack_rows<T>(g, d.staging, d.staging + n, d.staging + 2 * n, dst);
+    pack_rows<T>(g, d.staging, d.staging + n, d.staging + 2 * n, dst, d.box);
 }
 
 template <typename T>
@@ -209,8 +219,24 @@ cudaError_t launch_unpack_multi(const IoDesc *table, int n, int64_t max_rows, in
 }
 
 template <typename T>
-cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, cudaStream_t s) {
-    pack_kernel<T><<<row_grid((int64_t)g.ny * g.nz), 32 * kRowWarps, 0, s>>>(g, src[0], src[1], src[2], dst);
+cudaError_t launch_pack(const Geom &g, const double *const src[3], Fields<T> dst, BoxCheck box, cudaStream_t s) {
+    pack_kernel<T><<<row_grid((int64_t)g.ny * g.nz), 32 * kRowWarps, 0, s>>>(g, src[0], src[1], src[2], dst, box);
+    return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(32 * kRowWarps) box_check_kernel(Geom g, Fields<const double> f, BoxCheck box) {
+    const int lane = threadIdx.x & 31, nrows = g.ny * g.nz;
+    bool bad = false;
+    for (int r = blockIdx.x * kRowWarps + (threadIdx.x >> 5); r < nrows; r += gridDim.x * kRowWarps) {
+        const int z = r / g.ny, y = r - z * g.ny;
+        const int64_t a = g.at(0, y, z);
+        for (int x = lane; x < g.nx; x += 32) bad = bad || out_of_box(f.eS[a + x], f.eL[a + x], f.c[a + x], box.cmax);
+    }
+    if (bad) *box.word = 1;
+}
+
+cudaError_t launch_box_check(const Geom &g, Fields<const double> f, BoxCheck box, cudaStream_t s) {
+    box_check_kernel<<<row_grid((int64_t)g.ny * g.nz), 32 * kRowWarps, 0, s>>>(g, f, box);
     return cudaGetLastError();
 }
 
@@ -238,8 +264,8 @@ cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[
 // bits: more than an FP64 running sum keeps), FP64 beyond the thread.  FP64
 // accumulation per cell is what bounded the FP32 form (one conversion and
 // one addition per cell, each 1/64 of the FP32 rate); the FP64 state's form
-// is bound by the FP64 pipe, so it is written for few FP64 operations
-// (about 32 per cell).  256^3 FP32: 54 us (186 us with one cell per thread
+// in FP64 arithmetic is bound by the FP64 pipe, so it has few operations
+// (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 54 us (186 us with one cell per thread
 // and FP64 sums of the solute mass); 64^3: 7 us (33 us).
 
 // sums of pairs of floats carried with their rounding errors (Knuth's TwoSum)
@@ -378,11 +404,58 @@ struct ObsAcc {
     }
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256, 3) observe_kernel(Geom g, ObsCoef<T> k, Fields<const T> fl, int nq, int zc,
-                                                      double *partials) {
+// Sums of fixed-point numbers: exact (low words and high words apart).
+struct FxSum {
+    unsigned long long lo = 0;
+    long long hi = 0;
+    __device__ __forceinline__ void add(fx::i64 v) {
+        lo += (unsigned)v;
+        hi += v >> 32;
+    }
+    __device__ __forceinline__ double get(double scale) const {
+        return scale * ((double)hi * 4294967296.0 + (double)lo);
+    }
+};
+
+// Cells of an FP64 state in fixed-point arithmetic (ppf_fx.h), but for the
+// gradient's differences and squares: those twelve are what is left of about
+// 32 operations a cell for the FP64 pipe, which runs beside the integer
+// pipes.
+struct ObsFx {
+    FxSum mass, h, w, f0;
+    double gr = 0;
+    __device__ __forceinline__ void cell(const fx::FxCoef &k, int cbias, double eS, double eL, double c, double sx,
+                                         double lx, double sy, double ly, double sz, double lz) {
+        fx::i64 C, hh, w2, f;
+        fx::observe(k, eS, eL, c, cbias, C, hh, w2, f);
+        mass.add(C);
+        h.add(hh);
+        w.add(w2);
+        f0.add(f);
+        double d = sx - eS;
+        gr = fma(d, d, gr);
+        d = lx - eL;
+        gr = fma(d, d, gr);
+        d = sy - eS;
+        gr = fma(d, d, gr);
+        d = ly - eL;
+        gr = fma(d, d, gr);
+        d = sz - eS;
+        gr = fma(d, d, gr);
+        d = lz - eL;
+        gr = fma(d, d, gr);
+    }
+};
+
+// FX: an FP64 state whose parameters fit the fixed-point step; cells outside
+// its box take the FP64 path.
+template <typename T, bool FX>
+__global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoef<T> k, Fields<const T> fl, int nq, int zc,
+                                                      double *partials, fx::FxCoef kx) {
     constexpr int Q = 16 / (int)sizeof(T), NP = Q / 2;   // cells and pairs per thread
     ObsAcc<T> acc;
+    ObsFx ax;
+    const int cbias = FX ? fx::c_bias(kx.ec) : 0;
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int y = (int)(t / nq), x0 = (int)(t - (int64_t)y * nq) * Q;
     if (y < g.ny) {
@@ -412,10 +485,20 @@ __global__ void __launch_bounds__(256, 3) observe_kernel(Geom g, ObsCoef<T> k, F
             bool fine = whole;
 #pragma unroll
             for (int i = 0; i < Q; ++i) fine = fine && finite_(s[i]) && finite_(l[i]) && finite_(c[i]);
+            if constexpr (FX) {
+#pragma unroll
+                for (int i = 0; i < Q; ++i) fine = fine && !out_of_box(s[i], l[i], c[i], kx.cmax);
+            }
             if (fine) {
                 acc.n += Q;
 #pragma unroll
                 for (int i = 0; i < Q; ++i) acc.solid += above_half(s[i]) ? 1 : 0;
+                if constexpr (FX) {
+#pragma unroll
+                    for (int i = 0; i < Q; ++i)
+                        ax.cell(kx, cbias, s[i], l[i], c[i], i == Q - 1 ? sx : s[(i + 1) % Q],
+                                i == Q - 1 ? lx : l[(i + 1) % Q], sy[i], ly[i], sz[i], lz[i]);
+                } else
 #pragma unroll
                 for (int i = 0; i < NP; ++i) {
                     const int a = 2 * i, b = a + 1;
@@ -453,7 +536,13 @@ __global__ void __launch_bounds__(256, 3) observe_kernel(Geom g, ObsCoef<T> k, F
     // thread the reduction itself would otherwise fill the FP64 pipe), and
     // lanes 0, 8, 16, 24 end with mass, h, w and f.
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double v[4] = {acc.mass.get(), acc.h.get(), acc.w.get(), acc.f.get()};
+    double v[4] = {acc.mass.get(), acc.h.get(), acc.w.get(), acc.f.get()};
+    if constexpr (FX) {
+        v[0] += ax.mass.get(kx.sc);
+        v[1] += ax.h.get(4.3368086899420177e-19);                                  // 2^-61
+        v[2] += ax.w.get(kx.sc) * (kx.sc * 5.7646075230342349e+17);                // 2^(2 ec - 59)
+        v[3] += fma(k.kg, ax.gr, k.m * ax.f0.get(1.1102230246251565e-16));         // 2^-53
+    }
     const bool up = lane & 16, up2 = lane & 8;
     double a0 = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);
     const double a1 = (up ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, up ? v[1] : v[3], 16);
@@ -507,8 +596,8 @@ int observe_blocks(const Geom &g, int num_sms) {
 }
 
 template <typename T>
-cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, double *partials, int num_sms,
-                           cudaStream_t s) {
+cudaError_t launch_observe(const Geom &g, const CoefD &k, const fx::FxCoef *kx, Fields<const T> f, double *partials,
+                           int num_sms, cudaStream_t s) {
     int nq, bx, zc, bz;
     observe_shape(g, 16 / (int)sizeof(T), num_sms, &nq, &bx, &zc, &bz);
     ObsCoef<T> o;
@@ -524,7 +613,14 @@ cudaError_t launch_observe(const Geom &g, const CoefD &k, Fields<const T> f, dou
     o.CL = k.CL;
     o.dC = k.CS - k.CL;
     o.vol = k.vol;
-    observe_kernel<T><<<dim3((unsigned)bx, (unsigned)bz), 256, 0, s>>>(g, o, f, nq, zc, partials);
+    const dim3 grid((unsigned)bx, (unsigned)bz);
+    if constexpr (std::is_same<T, double>::value) {
+        if (kx) {
+            observe_kernel<T, true><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, *kx);
+            return cudaGetLastError();
+        }
+    }
+    observe_kernel<T, false><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, fx::FxCoef());
     return cudaGetLastError();
 }
 
@@ -550,17 +646,17 @@ cudaError_t launch_final_sum(const double *partials, int nblocks, int stride, in
 }
 
 // explicit instantiations
-template cudaError_t launch_pack<float>(const Geom &, const double *const[3], Fields<float>, cudaStream_t);
-template cudaError_t launch_pack<double>(const Geom &, const double *const[3], Fields<double>, cudaStream_t);
+template cudaError_t launch_pack<float>(const Geom &, const double *const[3], Fields<float>, BoxCheck, cudaStream_t);
+template cudaError_t launch_pack<double>(const Geom &, const double *const[3], Fields<double>, BoxCheck, cudaStream_t);
 template cudaError_t launch_unpack<float>(const Geom &, Fields<const float>, double *const[3], cudaStream_t);
 template cudaError_t launch_unpack<double>(const Geom &, Fields<const double>, double *const[3], cudaStream_t);
 template cudaError_t launch_pack_multi<float>(const IoDesc *, int, int64_t, cudaStream_t);
 template cudaError_t launch_pack_multi<double>(const IoDesc *, int, int64_t, cudaStream_t);
 template cudaError_t launch_unpack_multi<float>(const IoDesc *, int, int64_t, int, cudaStream_t);
 template cudaError_t launch_unpack_multi<double>(const IoDesc *, int, int64_t, int, cudaStream_t);
-template cudaError_t launch_observe<float>(const Geom &, const CoefD &, Fields<const float>, double *, int,
+template cudaError_t launch_observe<float>(const Geom &, const CoefD &, const fx::FxCoef *, Fields<const float>, double *, int,
                                            cudaStream_t);
-template cudaError_t launch_observe<double>(const Geom &, const CoefD &, Fields<const double>, double *, int,
+template cudaError_t launch_observe<double>(const Geom &, const CoefD &, const fx::FxCoef *, Fields<const double>, double *, int,
                                             cudaStream_t);
 
 template int observe_blocks<float>(const Geom &, int);

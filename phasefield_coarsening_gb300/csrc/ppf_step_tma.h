@@ -17,6 +17,7 @@ struct alignas(128) DomainDesc {
     int ntx, nty;             // tiles in x and y
     int nfx, nfy;             // whole tiles (inside the domain) in x and y
     int zc, nc;               // z planes per work item, items per tile column
+    int *box;                 // FP64: the two box words of the domain (launch_step_fx)
     int item0[3], nitems[3];  // first work item and count of this domain in the ensemble's launch
                               // over edge tiles [0], over whole tiles [1], over every tile [2]
 };

@@ -768,6 +768,5 @@ extern "C" int ppf_copy_state(ppf_ctx *dst, ppf_ctx *src) {
     dst->cur_eta = dst->cur_c = 0;
     dst->uploaded = 1;
     dst->steps = src->steps;
-    SCU(cudaStreamSynchronize(dst->stream));
-    return PPF_OK;
+    return recheck_box(dst);   // (the contexts' parameters, and so their boxes, may differ)
 }
