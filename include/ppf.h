@@ -176,7 +176,7 @@ typedef struct ppf_particle_stats {
 
 /* `volumes` (may be NULL) receives up to `capacity` particle volumes in
  * cells, in no particular order; *nvolumes (may be NULL) the particle count.
- * Device scratch of 8 bytes per cell is allocated on the first call. */
+ * Device scratch of about 8 bytes per cell is allocated on the first call. */
 int ppf_particles(ppf_ctx *ctx, double threshold, ppf_particle_stats *out, int64_t *volumes, int64_t capacity,
                   int64_t *nvolumes);
 

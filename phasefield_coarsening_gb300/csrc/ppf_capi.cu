@@ -725,7 +725,8 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     if (volumes && capacity < 0) return seterr(PPF_EINVAL, "negative capacity");
     const int64_t cells = (int64_t)c->nz * c->ny * c->nx;
     if (cells >= ((int64_t)1 << 31)) return seterr(PPF_EINVAL, "particle labels hold at most 2^31-1 cells");
-    if (!c->plab) CU(cudaMalloc(&c->plab, (size_t)cells * sizeof(int)));
+    // labels, and behind them the bit of every cell
+    if (!c->plab) CU(cudaMalloc(&c->plab, ((size_t)cells + (size_t)particle_words(c->g)) * sizeof(int)));
     if (!c->pvol) CU(cudaMalloc(&c->pvol, (size_t)cells * sizeof(int)));
     int64_t cap = volumes ? capacity : 0;
     if (cap > 0 && cap > c->plist_cap) {
@@ -743,17 +744,16 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     double *dout = c->dres + 8;
     if (c->prec == PPF_F32)
         CU(launch_particles<float>(c->g, (const float *)c->fld[c->cur_eta][0], threshold, c->plab, c->pvol,
-                                   c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist, c->derr,
+                                   (unsigned *)c->plab + cells, c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist, c->derr,
                                    c->stream));
     else
         CU(launch_particles<double>(c->g, (const double *)c->fld[c->cur_eta][0], threshold, c->plab, c->pvol,
-                                    c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist,
+                                    (unsigned *)c->plab + cells, c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist,
                                     c->derr, c->stream));
     double h[5];
     unsigned long long hn = 0;
     CU(cudaMemcpyAsync(h, dout, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (cap > 0) CU(cudaMemcpyAsync(&hn, nlist, sizeof hn, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
     rc = check_device_error(c);
     if (rc) return rc;
     const double dx = c->p.dx;

@@ -83,3 +83,58 @@ def test_fp32_mean_radius_within_half_percent_of_fp64():
     # at 256^3); the FP64 path conserves to round-off
     assert abs(r["mass_drift_fp32"]) <= 5e-8
     assert abs(r["mass_drift_fp64"]) <= 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 31), (1, 3, 32), (3, 2, 33), (4, 5, 64), (5, 7, 65), (9, 8, 1), (6, 33, 100), (20, 24, 289)])
+@pytest.mark.parametrize("bc", [0, 1])
+@pytest.mark.parametrize("fill", [0.0, 0.15, 0.31, 0.6, 1.0])
+def test_gpu_particles_of_random_cells(shape, bc, fill):
+    """Independent random cells: many short runs, single cells, one component
+    that fills the box; rows that are one word, several, and ragged.  Exact."""
+    r = np.random.default_rng(int(100 * fill) + sum(shape) + bc)
+    e = np.where(r.random(shape) < fill, 0.9, 0.1)
+    with ppf.Simulation(shape, bc=bc, precision="f32") as s:
+        s.upload(e, 1.0 - e, np.full(shape, 0.7))
+        g = s.particles(volumes=True)
+        few = s.particles()
+    o = oracle.particles(e, bc=bc)
+    assert g["count"] == few["count"] == o["count"]
+    assert np.array_equal(g["volumes"], o["volumes"])
+    assert g["solid_volume"] == o["solid_volume"] and g["interface_area"] == o["interface_area"]
+    assert g["largest_volume"] == o["largest_volume"]
+    assert abs(g["mean_radius"] - o["mean_radius"]) <= 1e-12 * o["mean_radius"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bc", [0, 1])
+def test_gpu_particles_of_a_spiral(bc):
+    """One chain through the whole box (its ends far apart in the labelling), and
+    its complement."""
+    n = 41
+    e = np.zeros((3, n, n))
+    lo, hi = 0, n - 1
+    y, x = 0, 0
+    dy, dx = 0, 1
+    seen = np.zeros((n, n), bool)
+    seen[0, 0] = True
+    while True:                          # a spiral with one-cell gaps
+        y2, x2 = y + dy, x + dx
+        y3, x3 = y2 + dy, x2 + dx
+        blocked = not (0 <= y2 < n and 0 <= x2 < n) or (0 <= y3 < n and 0 <= x3 < n and seen[y3, x3])
+        if blocked:
+            dy, dx = dx, -dy
+            y2, x2 = y + dy, x + dx
+            y3, x3 = y2 + dy, x2 + dx
+            if not (0 <= y2 < n and 0 <= x2 < n) or seen[y2, x2] or (0 <= y3 < n and 0 <= x3 < n and seen[y3, x3]):
+                break
+        y, x = y2, x2
+        seen[y, x] = True
+    e[1][seen] = 1.0
+    for f in (e, 1.0 - e):
+        with ppf.Simulation(f.shape, bc=bc) as s:
+            s.upload(f, 1.0 - f, np.full(f.shape, 0.7))
+            g = s.particles(volumes=True)
+        o = oracle.particles(f, bc=bc)
+        assert g["count"] == o["count"] and np.array_equal(g["volumes"], o["volumes"])
+        assert g["interface_area"] == o["interface_area"]
