@@ -185,25 +185,25 @@ int ppf_particles(ppf_ctx *ctx, double threshold, ppf_particle_stats *out, int64
  * phasefield.c:58-62, :340-350). */
 typedef struct ppf_tune {
     int zc;              /* z planes per work item of the persistent grid */
-    int roll;            /* 1: one plane body (the default), 3: unrolled three times */
+    int roll;            /* 1: one plane body, 3 (the default): unrolled three times (FP32, whole tiles) */
     int grid;            /* CTAs (derived from zc; ignored by ppf_set_tune) */
     int pdl;             /* 1 (the default): consecutive steps overlap by programmatic dependent
                             launch (the next step's CTAs are placed while this one's last CTAs
                             finish; every memory access still waits for the previous step);
                             0: plain launches.  With it, a step whose domain does not fill whole
                             tiles runs its edge tiles in the tail of its whole-tile launch. */
-    int sched;           /* 1 (the default): CTAs take work items from a global counter, so that
-                            faster CTAs take more; 0: items dealt round-robin.  Both give the
-                            same bits. */
+    int sched;           /* 1 (the default where CTAs take several items): CTAs take work items from
+                            a global counter, so that faster CTAs take more; 0: items dealt
+                            round-robin.  Both give the same bits. */
     int zc2;             /* > 0 and < zc: the top `tail` planes are cut into work items of zc2
                             planes instead of zc (short items end the step, so that its CTAs end
                             closer together); 0: every item zc planes */
     int tail;
-    int split;           /* 1 (the default): a domain whose x or y edge is not a multiple of the
+    int split;           /* 1 (the default of large FP64 domains and ensembles): a domain whose x or y edge is not a multiple of the
                             tile runs its whole tiles and its edge tiles as two launches, the
                             second in the first one's tail (with pdl); 0: one launch over every
                             tile.  Both give the same bits. */
-    int tile;            /* tile shape of a work item's brick: 0 (the default) 64 x 16 cells in x, y;
+    int tile;            /* tile shape of a work item's brick: 0 64 x 16 cells in x, y (FP64: 32 x 16);
                             1 (FP32 only) 32 x 32.  All give the same bits. */
     double us_per_step;  /* measured time of the winner (ppf_autotune only) */
 } ppf_tune;

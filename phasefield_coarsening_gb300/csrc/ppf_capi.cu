@@ -27,22 +27,6 @@ using namespace ppf;
 
 static thread_local char g_err[512];
 
-// Consecutive steps overlap by programmatic dependent launch unless the
-// autotuner finds the plain launch faster: the next step's CTAs are placed
-// while this one's last CTAs drain (worth ~12 % per step at 128^3, nothing
-// at 256^3, where the step is long against the launch gap).
-static constexpr int kStepPdl = 1;
-
-// CTAs take the step's work items from a global counter (in the same
-// chunk-major order as the round-robin deal), so that CTAs that run faster
-// take more items and the launch's CTAs end closer together.
-static constexpr int kStepSched = 1;
-
-// A domain whose x or y edge is not a multiple of the tile runs its whole
-// tiles and its edge tiles as two launches, the second in the first one's
-// tail, unless the autotuner finds one launch over every tile faster.
-static constexpr int kStepSplit = 1;
-
 static int seterr(int code, const char *fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
@@ -219,13 +203,9 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
                     return seterr(PPF_ECUDA, "TMA descriptor setup failed (%d)", mr);
                 }
             }
-    c->tune.roll = 1;
-    c->tune.pdl = kStepPdl;
-    c->tune.sched = kStepSched;
-    c->tune.split = kStepSplit;
-    c->tune.grid = precision == PPF_F32 ? tma_grid<float>(c->g, c->num_sms, &c->tune.zc)
-                                        : tma_grid<double>(c->g, c->num_sms, &c->tune.zc);
-    if (c->tune.grid < 1 || (c->fx_ok && fx_occupancy(false) < 1)) {
+    if (!(precision == PPF_F32 ? default_tune<float>(c->g, c->num_sms, &c->tune)
+                               : default_tune<double>(c->g, c->num_sms, &c->tune)) ||
+        (c->fx_ok && fx_occupancy(false) < 1)) {
         ppf_destroy(c);
         return seterr(PPF_ECUDA, "kernel attribute setup failed");
     }

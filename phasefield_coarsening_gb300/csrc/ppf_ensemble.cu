@@ -95,6 +95,31 @@ struct ppf_ensemble {
 
 static constexpr int kGraphSteps = 16;
 
+// The default z chunk and deal.  The shortest chunk that gives every CTA at
+// most one work item, dealt without the counter, while it is short enough
+// that the last CTAs do not march alone (4 domains of 48-128 cells FP32: 37.1
+// -> 24.5 us per step, FP64 228 -> 174 us); else chunks of 32 planes (FP32) or
+// 16 (FP64, whose items are longer: 16 domains 668 -> 584 us) from the
+// counter.
+static void default_chunk(ppf_ensemble *e) {
+    int tx = 0, ty = 0;
+    if (e->prec == PPF_F32) step_tile<float>(&tx, &ty, 0);
+    else step_tile<double>(&tx, &ty, 0);
+    const int64_t many = (int64_t)1 << 40;
+    const int64_t slots = e->prec == PPF_F32 ? tma_grid_items<float>(many, e->num_sms, 0)
+                                             : tma_grid_items<double>(many, e->num_sms, 0);
+    const int longest = e->prec == PPF_F32 ? 32 : 24;
+    e->sched = 0;
+    for (e->zc = 1; e->zc <= longest; ++e->zc) {
+        int64_t items = 0;
+        for (const ppf_ctx *c : e->dom)
+            items += (int64_t)((c->nx + tx - 1) / tx) * ((c->ny + ty - 1) / ty) * ((c->nz + e->zc - 1) / e->zc);
+        if (items <= slots) return;
+    }
+    e->zc = e->prec == PPF_F32 ? 32 : 16;
+    e->sched = 1;
+}
+
 static int build_table(ppf_ensemble *e) {
     int tx = 0, ty = 0;
     if (e->prec == PPF_F32) step_tile<float>(&tx, &ty, e->tile);
@@ -229,11 +254,9 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
     e->n = n;
     e->prec = precision;
     e->bc = bc;
-    e->zc = 32;
-    e->roll = 1;
-    e->sched = 1;
+    e->roll = 3;
     e->pdl = 1;
-    e->split = 0;
+    e->split = precision == PPF_F64;
     e->tile = 0;
     int rc = PPF_OK;
     for (int d = 0; d < n && rc == PPF_OK; ++d) {
@@ -247,6 +270,7 @@ extern "C" int ppf_ensemble_create(int n, const int *dims, const ppf_params *p, 
     }
     ppf_ctx *c0 = e->dom[0];
     e->num_sms = c0->num_sms;
+    default_chunk(e);
     e->eqA = c0->eqA;
     cudaError_t ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaMalloc(&e->dtable, (size_t)n * sizeof(DomainDesc));

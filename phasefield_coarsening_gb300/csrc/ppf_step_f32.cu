@@ -8,7 +8,7 @@ namespace ppf {
 template void step_tile<float>(int *, int *, int);
 template int step_tile_shapes<float>();
 template int make_field_map<float>(const Geom &, const float *, CUtensorMap *, int);
-template int tma_grid<float>(const Geom &, int, int *);
+template bool default_tune<float>(const Geom &, int, StepTune *);
 template int tma_grid_for<float>(const Geom &, int, const StepTune &);
 template int64_t tma_items<float>(const Geom &, const StepTune &);
 template cudaError_t launch_step_tma<float>(const Geom &, const Coef<float> &, const CUtensorMap *, Fields<float>, bool,

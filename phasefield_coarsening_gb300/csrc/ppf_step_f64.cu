@@ -8,7 +8,7 @@ namespace ppf {
 template void step_tile<double>(int *, int *, int);
 template int step_tile_shapes<double>();
 template int make_field_map<double>(const Geom &, const double *, CUtensorMap *, int);
-template int tma_grid<double>(const Geom &, int, int *);
+template bool default_tune<double>(const Geom &, int, StepTune *);
 template int tma_grid_for<double>(const Geom &, int, const StepTune &);
 template int64_t tma_items<double>(const Geom &, const StepTune &);
 template cudaError_t launch_step_tma<double>(const Geom &, const Coef<double> &, const CUtensorMap *, Fields<double>, bool,

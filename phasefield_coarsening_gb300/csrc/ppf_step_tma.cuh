@@ -897,21 +897,36 @@ void step_tile(int *tx, int *ty, int tile) {
 template <typename T>
 int step_tile_shapes() { return kTileShapes<T>; }
 
-// Launch shape (the model behind the default z chunk).  Work items are
-// (z chunk, tile) pairs dealt round-robin to a persistent grid of `slots`
-// CTAs (occupancy x SMs).  The chunk length
-// zc is chosen to minimise the busiest CTA's load count -- its planes plus
-// two halo planes per item -- so that the resident CTAs end together;
-// *zc_out receives it (for the first tile shape).
 template <typename T>
-int tma_grid(const Geom &g, int num_sms, int *zc_out) {
+int tma_grid_for(const Geom &g, int num_sms, const StepTune &t);
+
+// The default launch choice.  Work items are (z chunk, tile) pairs for a
+// persistent grid of `slots` CTAs (occupancy x SMs).
+//
+// A model gives the chunk length zc that minimises the busiest CTA's load
+// count -- its planes plus two halo planes per item -- when the items are
+// dealt round-robin.  Where that deals every CTA at most one item, it stands,
+// and the items are dealt (the counter would only cost its round trip:
+// 64^3 FP32 6.6 -> 5.5 us, 128^3 14.9 -> 13.9 us, 192^3 40.5 -> 37.8 us).
+// Where CTAs take several items, the counter's deal is better, and with at
+// least two chunks a slot so are chunks that pay few halo planes (long ones
+// when the slots hold many planes) with about one wave of short ones at the
+// top of z (two for FP64), so that the CTAs end together (FP32 256^3 87.8 ->
+// 78.5 us, 250^3 90.3 -> 85 us, 512^3 582 -> 540 us; FP64 256^3 663 -> 640
+// us).  One launch over every tile (edge tiles are not worth their own: FP32
+// 75 x 90 x 101 9.7 -> 9.2 us, 250^3 93.5 -> 85.3 us; FP64 54.6 -> 51.2 us)
+// but for FP64 domains of several items a CTA (200^3 401 -> 380 us).  32 x 32
+// tiles where they fit an x edge that 64 x 16 ones do not (96^3 10.3 -> 9.7).
+template <typename T>
+bool default_tune(const Geom &g, int num_sms, StepTune *t) {
     using G = TmaGeo<T, 0>;
     const int occ = step_occupancy<T, false>(0);
-    if (occ < 1) return -1;
+    if (occ < 1) return false;
+    constexpr bool F32 = std::is_same<T, float>::value;
     const int64_t ntiles = (int64_t)((g.nx + G::TX - 1) / G::TX) * ((g.ny + G::TY - 1) / G::TY);
     const int64_t slots = (int64_t)occ * num_sms;
     double best_cost = -1;
-    int64_t best_zc = g.nz, best_grid = 1;
+    int64_t best_zc = g.nz;
     for (int zc = 1; zc <= g.nz; ++zc) {
         const int64_t nc = (g.nz + zc - 1) / zc;
         if (nc > 1 && (nc - 1) * zc >= g.nz) continue;
@@ -934,10 +949,29 @@ int tma_grid(const Geom &g, int num_sms, int *zc_out) {
         // the resident CTAs share the SMs: a wave with fewer CTAs than slots
         // runs each faster, roughly as slots/grid while memory is the limit
         const double cost = (double)worst * (grid < slots ? (double)slots / (double)grid : 1.0);
-        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_zc = zc; best_grid = grid; }
+        if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_zc = zc; }
     }
-    *zc_out = (int)best_zc;
-    return (int)best_grid;
+    t->zc = (int)best_zc;
+    t->zc2 = t->tail = 0;
+    t->roll = 3;
+    t->pdl = 1;
+    t->split = t->tile = 0;
+    t->sched = ntiles * ((g.nz + best_zc - 1) / best_zc) > slots;
+    if (t->sched) {
+        const bool many = ntiles * g.nz >= 100 * slots;      // planes per slot
+        const int zc = F32 ? (many ? 36 : 24) : (many ? 38 : 16), zc2 = F32 ? (many ? 9 : 12) : zc / 2;
+        if (2 * zc <= g.nz && ntiles * g.nz >= 2 * zc * slots) {
+            const int64_t tail = ((F32 ? 1 : 2) * slots + ntiles - 1) / ntiles * zc2;
+            t->split = F32 ? 0 : 1;
+            t->zc = zc;
+            t->zc2 = zc2;
+            t->tail = (int)(tail < g.nz / 2 ? tail : g.nz / 2);
+        }
+    } else if (F32 && g.nx % 64 != 0 && g.nx % 32 == 0 && g.ny % 32 == 0) {
+        t->tile = 1;
+    }
+    t->grid = tma_grid_for<T>(g, num_sms, *t);
+    return t->grid >= 1;
 }
 
 // The z split of a launch choice: chunks of zc, the top `tail` planes

@@ -40,10 +40,9 @@ struct StepTune {
 template <typename T>
 int make_field_map(const Geom &g, const T *base, CUtensorMap *map, int tile);
 
-// Persistent grid size (occupancy x SMs, capped by the work) and the z
-// chunk length of a work item, for the first tile shape; < 0 on error.
+// The default launch choice of a domain; false on error.
 template <typename T>
-int tma_grid(const Geom &g, int num_sms, int *zc);
+bool default_tune(const Geom &g, int num_sms, StepTune *t);
 
 // Grid for a launch choice (occupancy x SMs, capped by its work items).
 template <typename T>
