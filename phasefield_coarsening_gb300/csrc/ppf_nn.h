@@ -24,12 +24,13 @@ namespace nn {
 
 constexpr int kTileX = 128;                 // voxels of one tile (the MMA's M)
 constexpr int kSegRows = kTileX + 2;        // a tile plus one voxel on each side in x
-constexpr int kSegPlane = kSegRows * 16;    // bytes of one 8-channel plane of a segment
+constexpr int kSegBytes = kSegRows * 16;    // bytes of one 8-channel plane of a segment
+constexpr int kSegPlane = 2176;             // its stride in shared memory, a multiple of 128 bytes
 
 struct NNGeom {
     int nx, ny, nz, bc;
-    int X;           // nx + 2
-    int64_t YX;      // (ny + 2)(nx + 2)
+    int X;           // nx + 2, rounded up to 128 bytes of voxels
+    int64_t YX;      // (ny + 2) X
     int64_t Pst;     // voxels per channel plane
     __host__ __device__ __forceinline__ int64_t p(int x, int y, int z) const {
         return (int64_t)(z + 1) * YX + (int64_t)(y + 1) * X + (x + 1);
@@ -39,8 +40,8 @@ struct NNGeom {
 inline NNGeom make_nngeom(int nz, int ny, int nx, int bc) {
     NNGeom g;
     g.nx = nx; g.ny = ny; g.nz = nz; g.bc = bc;
-    g.X = nx + 2;
-    g.YX = (int64_t)(ny + 2) * (nx + 2);
+    g.X = (nx + 2 + 7) / 8 * 8;
+    g.YX = (int64_t)(ny + 2) * g.X;
     g.Pst = ((int64_t)(nz + 2) * g.YX + 7) / 8 * 8;
     return g;
 }

@@ -3,25 +3,27 @@
 // FP32 accumulation in TMEM).
 //
 // conv_kernel<CI, CO, EPI>: out[v] = sum over the 27 taps of W_tap * in[v + tap].
-//   One tile = 128 consecutive voxels of one x row (M = 128), N = CO,
-//   K = 27 taps x CI.  A work item is a column of tiles marching in y
-//   (rows y0..y1-1 of one z plane and x segment).  Each row of the march
-//   needs the three input rows (y-1, y, y+1) at z-1, z, z+1; an input
-//   "segment" is 130 voxels (the tile plus one each side) of one input row,
-//   moved into shared memory by 1-D bulk copies, one per 8-channel plane.
-//   A ring of RING row slots (3 segments each) holds rows y-1..y+1 while
-//   the next rows load, so every input row is fetched once per work item.
-//   The A operand of tap (dz, dy, dx) is its segment started dx+1 voxels
-//   (16 bytes each) in; the B operand is that tap's CI x CO block of the
-//   weight image, loaded once per CTA.
-//   Warp roles (352 threads): warp 0 lane 0 issues the bulk copies, lane 0
-//   of warps 1 and 10 issue the MMAs of alternate rows (warp 1 owns the
-//   TMEM allocation), warps
-//   2-9 run the epilogue on a double-buffered TMEM accumulator (warp w
-//   reads TMEM lanes 32 (w % 4).., warps 2-5 the first half of the output
-//   channels, warps 6-9 the second), so the epilogue of one tile overlaps
-//   the MMAs of the next.  Operand descriptors are built once and advanced
-//   by constant offsets.
+//   One tile = 128 consecutive voxels of one x row (M = 128), N = 3 CO (the
+//   three dy taps), K = 9 (dz, dx) taps x CI.  A work item is a column of
+//   tiles marching in y (rows y0..y1-1 of one z plane and x segment).  An
+//   input "segment" is 130 voxels (the tile plus one each side) of one input
+//   row, moved into shared memory by 1-D bulk copies, one per 8-channel
+//   plane.  A ring of RING row slots (3 segments each, z-1..z+1) holds the
+//   rows while the next ones load, so every input row is fetched once per
+//   work item.  The A operand of tap (dz, dx) is its segment started dx+1
+//   voxels (16 bytes each) in; the B operand is that tap's CI x 3 CO block of
+//   the weight image, loaded once per CTA.
+//   Warp roles: three producer threads (one per z plane), two MMA-issuing
+//   threads (alternate rows; the first one's warp owns the TMEM
+//   allocation), and two or three epilogue groups of four warps that take
+//   the output rows in turn from a ring of five TMEM tiles.
+//   What bounds it: with N = 96 an MMA reads 7 KB of operands from shared
+//   memory, 56 cycles at 128 bytes a clock (measured; the mathematics is
+//   48), so a row of 18 takes 1008 cycles; at 256^3, 32 -> 32 channels, that
+//   is 0.49 ms.  Measured 0.65 ms (0.82 ms before): one producer thread
+//   issued a row's 12 copies in about 1400 cycles, one MMA thread spends
+//   about 500 on a row's waits and descriptors, and every row's halo voxel in
+//   x sent its warp through the eight-image loop.
 //
 // wgrad_kernel<CX, CZ>: dW[tap][co][ci] = sum over voxels v of
 //   dZ[v][co] * X[v + tap][ci].  The reduction runs over voxels (K), both
@@ -40,6 +42,7 @@
 #include <cstdint>
 
 #include "ppf_nn.h"
+#include "ppf_pair.h"
 #include "ppf_ptx.h"
 
 namespace ppf {
@@ -96,53 +99,42 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-__device__ __forceinline__ uint4 pack8(const float *f) {
-    return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                      pack_bf16x2(f[6], f[7]));
+__device__ __forceinline__ uint4 pack8(const V2<float> *f) {
+    return make_uint4(pack_bf16x2(f[0].x(), f[0].y()), pack_bf16x2(f[1].x(), f[1].y()),
+                      pack_bf16x2(f[2].x(), f[2].y()), pack_bf16x2(f[3].x(), f[3].y()));
 }
 
-__device__ __forceinline__ void unpack8(uint4 q, float *f) {
+__device__ __forceinline__ void unpack8(uint4 q, V2<float> *f) {
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
+    for (int i = 0; i < 4; ++i) f[i] = V2<float>(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u));
 }
 
 // logistic function: sigma(z) = (1 + tanh(z/2)) / 2 with the hardware
 // tanh (tanh.approx.f32, relative error about 2^-11, well below the BF16
 // rounding of every value it feeds)
-__device__ __forceinline__ float sigmoidf(float z) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.5f * z));
-    return fmaf(0.5f, t, 0.5f);
+__device__ __forceinline__ V2<float> sigmoid2(V2<float> z) {
+    const V2<float> h = splat(0.5f) * z;
+    float t, u;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(h.x()));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(u) : "f"(h.y()));
+    return fma2(splat(0.5f), V2<float>(t, u), splat(0.5f));
 }
 
+// the halo images of voxel (x, y, z) in y and z (and their images in x); v[j]
+// is the voxel in channel plane j
 template <int NP>
-__device__ __forceinline__ void store_planes(uint16_t *base, int64_t Pst, int64_t p, const uint4 (&v)[NP]) {
-#pragma unroll
-    for (int j = 0; j < NP; ++j)
-        *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(base) + ((int64_t)j * Pst + p) * 16) = v[j];
-}
-
-// store at (x, y, z) and at every halo image of it
-template <int NP>
-__device__ __forceinline__ void store_with_images(const NNGeom &g, uint16_t *base, int x, int y, int z,
-                                                  const uint4 (&v)[NP]) {
-    store_planes<NP>(base, g.Pst, g.p(x, y, z), v);
+__device__ __noinline__ void store_images(const NNGeom &g, uint4 *base, int x, int y, int z, const uint4 (&v)[NP]) {
     const int ax = image_of(x, g.nx, g.bc), ay = image_of(y, g.ny, g.bc), az = image_of(z, g.nz, g.bc);
-    if (ax == kNone && ay == kNone && az == kNone) return;
-    for (int k = 1; k < 8; ++k) {
+    for (int k = 2; k < 8; ++k) {
         const int xx = (k & 1) ? ax : x, yy = (k & 2) ? ay : y, zz = (k & 4) ? az : z;
         if (xx == kNone || yy == kNone || zz == kNone) continue;
-        store_planes<NP>(base, g.Pst, g.p(xx, yy, zz), v);
+        const int64_t p = g.p(xx, yy, zz);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) base[(int64_t)j * g.Pst + p] = v[j];
     }
 }
 
-constexpr int kConvThreads = 352;   // producer warp, MMA warp, 8 epilogue warps, second MMA warp
-constexpr int kMmaWarp2 = 10;
-constexpr int kEpiThreads = 256;
 
 template <int CI, int CO>
 struct ConvCfg {
@@ -152,16 +144,26 @@ struct ConvCfg {
     static constexpr int SEGB = (CI / 8) * kSegPlane;    // one segment, all channel planes
     static constexpr int ROWB = 3 * SEGB;                // one slot: segments at z-1, z, z+1
     static constexpr int WB = 27 * CI * CO * 2;          // weight image
-    static constexpr int HALF = CO / 2;                  // output channels per epilogue warp
     static constexpr int OFF_W = RING * ROWB;
     static constexpr int OFF_BAR = OFF_W + WB;
     static constexpr int NBAR = 2 * RING + 2 * ND + 3;   // full, empty, dfull, dempty, wbar, drain x2
     static constexpr int OFF_SLOT = OFF_BAR + NBAR * 8;  // TMEM base, abort flag
-    static constexpr int OFF_RED = OFF_SLOT + 16;        // [8][HALF + 1] floats
-    static constexpr int OFF_BIAS = OFF_RED + 8 * (HALF + 1) * 4;   // CO floats
-    static constexpr int OFF_REDD = (OFF_BIAS + CO * 4 + 7) / 8 * 8;  // [4] doubles
-    static constexpr int SMEM = OFF_REDD + 4 * 8;
+    static constexpr int OFF_RED = OFF_SLOT + 16;        // [16][CO + 1] floats
+    static constexpr int OFF_BIAS = (OFF_RED + 16 * (CO + 1) * 4 + 15) / 16 * 16;   // CO floats
+    static constexpr int OFF_REDD = OFF_BIAS + CO * 4;   // [16] doubles
+    static constexpr int SMEM = OFF_REDD + 16 * 8;
     static constexpr int TMEM_COLS = ND * NCOL <= 256 ? 256 : 512;
+    // CTAs per SM: shared memory (228 KB per SM, 1 KB reserved per CTA), TMEM (512 columns per SM)
+    static constexpr int BY_SMEM = 233472 / (SMEM + 1024), BY_TMEM = 512 / TMEM_COLS;
+    static constexpr int CTAS = BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM;
+    static_assert(CTAS >= 1, "one CTA fits");
+    // epilogue groups of four warps: as many as the registers of the CTAs hold
+    // and as help (32 -> 32 channels at 256^3: 2 groups 652 us, 3 645, 4 672)
+    static constexpr int groups(int epi) { return CTAS > 1 || epi == EPI_DGRAD ? 2 : 3; }
+    // warps: a producer, an MMA issuer, the epilogue's, two more producers, another MMA issuer
+    static constexpr int producer2(int epi) { return 2 + 4 * groups(epi); }
+    static constexpr int mma2(int epi) { return producer2(epi) + 2; }
+    static constexpr int threads(int epi) { return 32 * (mma2(epi) + 1); }
     static_assert(CI % 16 == 0 && CO % 16 == 0 && CO <= 32, "channel counts");
     static_assert(ND * NCOL <= 512 && NCOL <= 256, "TMEM / MMA N");
     static_assert(OFF_W % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
@@ -193,9 +195,8 @@ __device__ __forceinline__ Item item_of(const NNGeom &g, int yc, int it) {
 // W[dz][dy][dx][co][ci] in[z+dz][row q][x+dx][ci]; output row y is
 // D_{y-1}[dy=-1] + D_y[dy=0] + D_{y+1}[dy=+1], summed by the epilogue.
 template <int CI, int CO, int EPI>
-__global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a) {
+__global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>::CTAS) conv_kernel(const __grid_constant__ ConvArgs a) {
     using C = ConvCfg<CI, CO>;
-    constexpr int HALF = C::HALF;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sb = smem_u32(smem);
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
         }
         for (int s = 0; s < C::ND; ++s) {
             mbar_init(dfull(s), 1);
-            mbar_init(dempty(s), kEpiThreads);
+            mbar_init(dempty(s), 3 * 4);         // three output rows read a tile, four warps each
         }
         mbar_init(wbar, 1);
         mbar_init(dbar, 1);
@@ -233,21 +234,30 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
     tc_fence_after();
     const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(tslot);
 
-    if (warp == 0) {
-        // ---------------- producer: bulk copies of input rows ----------------
+    if (warp == 0 || (warp >= C::producer2(EPI) && warp < C::mma2(EPI))) {
+        // ---------------- producers: bulk copies of input rows.  Issuing a copy
+        // takes one thread 115-150 cycles, so three threads share a row's, one
+        // per z plane; the first one also announces the row's bytes (copies that
+        // complete before that leave the phase open: its one arrival is the
+        // announcement) ----------------
         if (lane == 0) {
+            const int dz = warp == 0 ? 0 : warp - C::producer2(EPI) + 1;
             uint32_t issued_q[C::RING];
 #pragma unroll
             for (int s = 0; s < C::RING; ++s) issued_q[s] = 0xFFFFFFFFu;
-            mbar_expect_tx(wbar, C::WB);
-            bulk_load(wsm, a.wimg, C::WB, wbar);
+            if (dz == 0) {
+                mbar_expect_tx(wbar, C::WB);
+                bulk_load(wsm, a.wimg, C::WB, wbar);
+            }
             uint32_t q = 0;
             bool ok = true;
             for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
                 const Item w = item_of(g, a.yc, it);
-                for (int r = w.y0 - 1; r <= w.y1; ++r, ++q) {
+                const unsigned char *src = reinterpret_cast<const unsigned char *>(a.x) +
+                                           g.p(w.x0 - 1, w.y0 - 1, w.z + dz - 1) * 16;
+                for (int r = w.y0 - 1; r <= w.y1; ++r, ++q, src += (int64_t)g.X * 16) {
                     const uint32_t s = q % C::RING;
-                    // the producer runs ahead of the MMAs: its waits for a free slot
+                    // the producers run ahead of the MMAs: their waits for a free slot
                     // sleep between polls instead of taking issue slots
                     if (q >= (uint32_t)C::RING &&
                         !wait_backoff(empty(s), ((q / C::RING) + 1) & 1, a.limit_ns, abort_flag)) {
@@ -256,20 +266,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
                         break;
                     }
                     // test hook: the second row's barrier expects 16 bytes that never come
-                    mbar_expect_tx(full(s), C::ROWB + ((a.inject_stall && q == 1) ? 16u : 0u));
+                    if (dz == 0)
+                        mbar_expect_tx(full(s), 3 * (CI / 8) * kSegBytes + ((a.inject_stall && q == 1) ? 16u : 0u));
 #pragma unroll
                     for (int k = 0; k < C::RING; ++k)
                         if (k == (int)s) issued_q[k] = q;
+                    const uint32_t dst = ring + s * C::ROWB + dz * C::SEGB;
 #pragma unroll
-                    for (int dz = 0; dz < 3; ++dz) {
-                        const int64_t pv = g.p(w.x0 - 1, r, w.z + dz - 1);
-#pragma unroll
-                        for (int j = 0; j < CI / 8; ++j) {
-                            const unsigned char *src =
-                                reinterpret_cast<const unsigned char *>(a.x) + ((int64_t)j * g.Pst + pv) * 16;
-                            bulk_load(ring + s * C::ROWB + dz * C::SEGB + j * kSegPlane, src, kSegPlane, full(s));
-                        }
-                    }
+                    for (int j = 0; j < CI / 8; ++j)
+                        bulk_load(dst + j * kSegPlane, src + (int64_t)j * g.Pst * 16, kSegBytes, full(s));
                 }
             }
             // drain: every issued copy has landed before the CTA may exit
@@ -277,15 +282,15 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
             for (int s = 0; s < C::RING; ++s)
                 if (issued_q[s] != 0xFFFFFFFFu && !mbar_wait(full(s), (issued_q[s] / C::RING) & 1, a.limit_ns))
                     atomicOr(a.err, 4);
-            if (!mbar_wait(wbar, 0, a.limit_ns)) atomicOr(a.err, 4);
+            if (dz == 0 && !mbar_wait(wbar, 0, a.limit_ns)) atomicOr(a.err, 4);
         }
-    } else if (warp == 1 || warp == kMmaWarp2) {
-        // ---------------- MMA issuers: one D tile per input row; warp 1
-        // takes the even rows, warp 10 the odd ones, so that one thread's
-        // waits and bookkeeping overlap the other's MMAs ----------------
+    } else if (warp == 1 || warp == C::mma2(EPI)) {
+        // ---------------- MMA issuers: one D tile per input row; one thread takes
+        // the even rows, another the odd ones, so that one's waits and
+        // bookkeeping (about 500 cycles a row) overlap the other's MMAs ----------
         if (lane == 0) {
+            constexpr int NM = 9 * (CI / 16);              // MMAs of a row
             const uint32_t mine = warp == 1 ? 0u : 1u;
-            const uint32_t mydbar = warp == 1 ? dbar : dbar + 8;
             const uint32_t idesc = idesc_bf16(128, C::NCOL, false, false);
             // descriptors of slot 0 and of the weight image; every operand
             // below is one of these plus a byte offset / 16 (no carry: all
@@ -295,77 +300,88 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
             const uint64_t b0 = smem_desc(wsm, C::NCOL * 16, 128);
             bool ok = wait_or_abort(wbar, 0, a.limit_ns, abort_flag);
             if (!ok) fail(abort_flag, a.err, 1);
-            uint32_t q = 0;
-            for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
+            uint32_t total = 0;                            // input rows of the CTA's items
+            for (int it = blockIdx.x; it < a.items; it += gridDim.x) {
                 const Item w = item_of(g, a.yc, it);
-                for (int r = w.y0 - 1; r <= w.y1; ++r, ++q) {
-                    if ((q & 1u) != mine) continue;
-                    const uint32_t s = q % C::RING, ds = q % C::ND;
-                    if (!wait_or_abort(full(s), (q / C::RING) & 1, a.limit_ns, abort_flag) ||
-                        (q >= (uint32_t)C::ND &&
-                         !wait_or_abort(dempty(ds), ((q / C::ND) + 1) & 1, a.limit_ns, abort_flag))) {
-                        fail(abort_flag, a.err, 1);
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t d = tbase + ds * C::NCOL;
-                    const uint64_t ab = a0 + ((s * C::ROWB) >> 4);
-#pragma unroll
-                    for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-                        for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-                            for (int kk = 0; kk < CI / 16; ++kk) {
-                                const uint64_t ad = ab + ((dz * C::SEGB + dx * 16 + kk * 2 * kSegPlane) >> 4);
-                                const uint64_t bd = b0 + ((((dz * 3 + dx) * (CI / 8) + 2 * kk) * C::NCOL * 16) >> 4);
-                                mma_bf16(d, ad, bd, idesc, (dz | dx | kk) ? 1u : 0u);
-                            }
-                    mma_commit(empty(s));
-                    mma_commit(dfull(ds));
+                total += (uint32_t)(w.y1 - w.y0) + 2;
+            }
+            for (uint32_t q = mine; ok && q < total; q += 2) {
+                const uint32_t sl = q % C::RING, ds = q % C::ND;
+                if (!wait_or_abort(full(sl), (q / C::RING) & 1, a.limit_ns, abort_flag) ||
+                    (q >= (uint32_t)C::ND &&
+                     !wait_or_abort(dempty(ds), ((q / C::ND) + 1) & 1, a.limit_ns, abort_flag))) {
+                    fail(abort_flag, a.err, 1);
+                    ok = false;
+                    break;
                 }
+                tc_fence_after();
+                const uint32_t d = tbase + ds * C::NCOL;
+                const uint64_t ab = a0 + ((sl * C::ROWB) >> 4);
+#pragma unroll
+                for (int k = 0; k < NM; ++k) {             // (dz, dx, channel half)
+                    const int tap = k / (CI / 16), kk = k % (CI / 16), dz = tap / 3, dx = tap % 3;
+                    const uint64_t ad = ab + ((dz * C::SEGB + dx * 16 + kk * 2 * kSegPlane) >> 4);
+                    const uint64_t bd = b0 + (((tap * (CI / 8) + 2 * kk) * C::NCOL * 16) >> 4);
+                    mma_bf16(d, ad, bd, idesc, k ? 1u : 0u);
+                }
+                mma_commit(empty(sl));
+                mma_commit(dfull(ds));
             }
             // drain: all issued MMAs complete before TMEM is released
+            const uint32_t mydbar = dbar + 8 * mine;
             mma_commit(mydbar);
             if (!mbar_wait(mydbar, 0, a.limit_ns)) atomicOr(a.err, 4);
         }
     } else {
-        // ---------------- epilogue: warps 2-9; TMEM lane quarter = warp % 4,
-        // output channels [c0, c0 + HALF) by warp group ----------------
+        // ---------------- epilogue: groups of four warps take the output rows in
+        // turn (counted over the CTA's items), a warp the voxels of its TMEM lane
+        // quarter, warp % 4, with all channels ----
+        constexpr uint32_t NG = C::groups(EPI);
+        constexpr int NEW = 4 * NG;                        // epilogue warps
         const int ew = warp - 2;
+        const uint32_t grp = (uint32_t)ew >> 2;
         const int quarter = warp & 3;
-        const int c0 = (ew >> 2) * HALF;
         const int row = quarter * 32 + lane;
-        const uint32_t tl = tbase + ((uint32_t)(quarter * 32) << 16) + c0;
+        const uint32_t tl = tbase + ((uint32_t)(quarter * 32) << 16);
         constexpr bool STATE_OUT = EPI == EPI_STATE || EPI == EPI_LOSS;
-        const bool active = !STATE_OUT || c0 == 0;
-        float sums[HALF + 1];
+        constexpr int CH = STATE_OUT ? 4 : 16;             // channels loaded at a time
+        constexpr int NCH = STATE_OUT ? 1 : CO / 16;
+        constexpr int NSUM = EPI == EPI_DGRAD ? CO / 2 : EPI == EPI_LOSS ? 2 : 1;
+        V2<float> sums[NSUM];                              // per channel pair (EPI_DGRAD, EPI_LOSS)
+        float lsum = 0.f;                                  // the loss
 #pragma unroll
-        for (int c = 0; c <= HALF; ++c) sums[c] = 0.f;
+        for (int c = 0; c < NSUM; ++c) sums[c] = splat(0.f);
         double mass = 0.0;
-        uint32_t q = 0;
+        uint32_t q = 0, rows = 0;
         bool ok = true;
+        auto wait_d = [&](uint32_t t) {
+            return wait_backoff(dfull(t % C::ND), (t / C::ND) & 1, a.limit_ns, abort_flag);
+        };
         for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
             const Item w = item_of(g, a.yc, it);
-            const uint32_t qb = q;                 // input row y0 - 1
-            q += (uint32_t)(w.y1 - w.y0) + 2;
-            for (int y = w.y0; y < w.y1; ++y) {
-                const uint32_t qy = qb + (uint32_t)(y - w.y0) + 1;   // input row y
-                const int x = w.x0 + row, z = w.z;
-                const int64_t p = g.p(x, y, z);
+            const uint32_t qb = q, n = (uint32_t)(w.y1 - w.y0);  // input row y0 - 1; output rows
+            q += n + 2;
+            const int x = w.x0 + row, z = w.z;
+            // halo images: one in x is a second store; those in y and z (edge rows and
+            // planes) are left to store_images
+            const bool xedge = x == 0 || x == g.nx - 1, zedge = z == 0 || z == g.nz - 1;
+            const int dxi = xedge ? image_of(x, g.nx, g.bc) - x : 0;
+            const int64_t p0 = g.p(x, w.y0, z);
+            const int64_t s0 = STATE_OUT ? a.sg.at(x, w.y0, z) : 0;
+            for (uint32_t i = (grp + NG - rows % NG) % NG; i < n; i += NG) {
+                const int y = w.y0 + (int)i;
+                const uint32_t qy = qb + i + 1;            // input row y
+                const int64_t p = p0 + (int64_t)i * g.X;
                 // loads that do not depend on the accumulators go first
-                float zl[HALF];
-                float s0v[3] = {0.f, 0.f, 0.f}, s1v[3] = {0.f, 0.f, 0.f};
-                int64_t sa = 0;
+                uint4 zl[EPI == EPI_DGRAD ? CO / 8 : 1];
+                float s0v[3], s1v[3];
+                const int64_t sa = s0 + (int64_t)i * a.sg.P;
                 if (EPI == EPI_DGRAD) {
 #pragma unroll
-                    for (int j = 0; j < HALF / 8; ++j)
-                        unpack8(*reinterpret_cast<const uint4 *>(reinterpret_cast<const unsigned char *>(a.zlow) +
-                                                                  ((int64_t)(c0 / 8 + j) * g.Pst + p) * 16),
-                                zl + 8 * j);
+                    for (int j = 0; j < CO / 8; ++j)
+                        zl[j] = reinterpret_cast<const uint4 *>(a.zlow)[(int64_t)j * g.Pst + p];
                 }
-                if (STATE_OUT && active) {
-                    sa = a.sg.at(x, y, z);
+                if (STATE_OUT) {
                     s0v[0] = a.s0.eS[sa];
                     s0v[1] = a.s0.eL[sa];
                     s0v[2] = a.s0.c[sa];
@@ -375,156 +391,167 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv_kernel(const ConvArgs a)
                         s1v[2] = a.s1.c[sa];
                     }
                 }
-                if (!wait_backoff(dfull((qy - 1) % C::ND), ((qy - 1) / C::ND) & 1, a.limit_ns, abort_flag) ||
-                    !wait_backoff(dfull(qy % C::ND), (qy / C::ND) & 1, a.limit_ns, abort_flag) ||
-                    !wait_backoff(dfull((qy + 1) % C::ND), ((qy + 1) / C::ND) & 1, a.limit_ns, abort_flag)) {
+                if (!wait_d(qy - 1) || !wait_d(qy) || !wait_d(qy + 1)) {
                     fail(abort_flag, a.err, 1);
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                float v[HALF];
-                {
-                    // out[y] = sum_dy W_dy in[y + dy]: the dy = -1 block of
-                    // D_{y-1}, the dy = 0 block of D_y, the dy = +1 block of D_{y+1}
-                    const uint32_t t0 = tl + ((qy - 1) % C::ND) * C::NCOL;
-                    const uint32_t t1 = tl + (qy % C::ND) * C::NCOL + CO;
-                    const uint32_t t2 = tl + ((qy + 1) % C::ND) * C::NCOL + 2 * CO;
-                    if constexpr (HALF == 16) {
-                        float u0[16], u1[16], u2[16];
-                        tmem_ld16(t0, u0);
-                        tmem_ld16(t1, u1);
-                        tmem_ld16(t2, u2);
+                // out[y] = sum_dy W_dy in[y + dy]: the dy = -1 block of
+                // D_{y-1}, the dy = 0 block of D_y, the dy = +1 block of D_{y+1}
+                const uint32_t t0 = tl + ((qy - 1) % C::ND) * C::NCOL;
+                const uint32_t t1 = tl + (qy % C::ND) * C::NCOL + CO;
+                const uint32_t t2 = tl + ((qy + 1) % C::ND) * C::NCOL + 2 * CO;
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i] = (u0[i] + u1[i]) + u2[i];
-                    } else {
-                        float u0[8], u1[8], u2[8];
-                        tmem_ld8(t0, u0);
-                        tmem_ld8(t1, u1);
-                        tmem_ld8(t2, u2);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[i] = (u0[i] + u1[i]) + u2[i];
-                    }
-                }
-                tc_fence_before();
-                mbar_arrive(dempty((qy - 1) % C::ND));
-                if (y == w.y1 - 1) {
-                    mbar_arrive(dempty(qy % C::ND));
-                    mbar_arrive(dempty((qy + 1) % C::ND));
-                }
-
-                if (EPI == EPI_ACT || EPI == EPI_ACT_TRAIN) {
-                    uint4 o[HALF / 8], zz[HALF / 8];
-#pragma unroll
-                    for (int j = 0; j < HALF / 8; ++j) {
-                        float h[8], sv[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            h[i] = v[8 * j + i] + sbias[c0 + 8 * j + i];
-                            sv[i] = h[i] * sigmoidf(h[i]);
+                for (int ch = 0; ch < NCH; ++ch) {
+                    uint32_t u0[CH], u1[CH], u2[CH];
+                    tmem_ld(t0 + CH * ch, u0);
+                    tmem_ld(t1 + CH * ch, u1);
+                    tmem_ld(t2 + CH * ch, u2);
+                    tmem_wait_ld(u0, u1, u2);
+                    if (ch == NCH - 1) {
+                        // Every tile is released by three arrivals per thread: one from
+                        // each row that reads it, and at the item's ends, where fewer
+                        // rows do, the missing ones from the first that does.
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            mbar_arrive(dempty((qy - 1) % C::ND), i == 0 ? 3u : 1u);
+                            mbar_arrive(dempty(qy % C::ND), i == 0 ? (n > 1 ? 2u : 3u) : 1u);
+                            mbar_arrive(dempty((qy + 1) % C::ND), i + 1 == n ? 3u : i + 2 == n ? 2u : 1u);
                         }
-                        o[j] = pack8(sv);
-                        zz[j] = pack8(h);
                     }
-                    uint16_t *ob = reinterpret_cast<uint16_t *>(reinterpret_cast<unsigned char *>(a.out) +
-                                                                (int64_t)(c0 / 8) * g.Pst * 16);
-                    store_with_images<HALF / 8>(g, ob, x, y, z, o);
-                    if (EPI == EPI_ACT_TRAIN) {
-                        uint16_t *zb = reinterpret_cast<uint16_t *>(reinterpret_cast<unsigned char *>(a.zout) +
-                                                                    (int64_t)(c0 / 8) * g.Pst * 16);
-                        store_planes<HALF / 8>(zb, g.Pst, p, zz);
-                    }
-                } else if (EPI == EPI_DGRAD) {
-                    uint4 o[HALF / 8];
+                    auto pr = [](const uint32_t(&u)[CH], int k) {
+                        return V2<float>(__uint_as_float(u[2 * k]), __uint_as_float(u[2 * k + 1]));
+                    };
+                    V2<float> v[CH / 2];
 #pragma unroll
-                    for (int j = 0; j < HALF / 8; ++j) {
-                        float dd[8];
+                    for (int k = 0; k < CH / 2; ++k) v[k] = (pr(u0, k) + pr(u1, k)) + pr(u2, k);
+                    if (EPI == EPI_ACT || EPI == EPI_ACT_TRAIN) {
+                        uint4 o[2], zz[2];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const float zi = zl[8 * j + i];
-                            const float sg = sigmoidf(zi);
-                            dd[i] = v[8 * j + i] * sg * (1.0f + zi * (1.0f - sg));
-                            sums[8 * j + i] += dd[i];
+                        for (int j = 0; j < 2; ++j) {
+                            V2<float> h[4], sv[4];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                h[k] = v[4 * j + k] + ld2(sbias + 16 * ch + 8 * j + 2 * k);
+                                sv[k] = h[k] * sigmoid2(h[k]);
+                            }
+                            o[j] = pack8(sv);
+                            zz[j] = pack8(h);
                         }
-                        o[j] = pack8(dd);
-                    }
-                    uint16_t *ob = reinterpret_cast<uint16_t *>(reinterpret_cast<unsigned char *>(a.out) +
-                                                                (int64_t)(c0 / 8) * g.Pst * 16);
-                    store_with_images<HALF / 8>(g, ob, x, y, z, o);
-                } else if (EPI == EPI_STATE) {
-                    if (active) {
+                        uint4 *ob = reinterpret_cast<uint4 *>(a.out) + (int64_t)(2 * ch) * g.Pst;
+                        ob[p] = o[0];
+                        ob[g.Pst + p] = o[1];
+                        if (xedge) {
+                            ob[p + dxi] = o[0];
+                            ob[g.Pst + p + dxi] = o[1];
+                        }
+                        if (zedge || y == 0 || y == g.ny - 1) store_images<2>(g, ob, x, y, z, o);
+                        if (EPI == EPI_ACT_TRAIN) {
+                            uint4 *zb = reinterpret_cast<uint4 *>(a.zout) + (int64_t)(2 * ch) * g.Pst;
+                            zb[p] = zz[0];
+                            zb[g.Pst + p] = zz[1];
+                        }
+                    } else if (EPI == EPI_DGRAD) {
+                        uint4 o[2];
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) {
+                            V2<float> zi[4], dd[4];
+                            unpack8(zl[2 * ch + j], zi);
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const V2<float> sg = sigmoid2(zi[k]);
+                                dd[k] = v[4 * j + k] * sg * fma2(zi[k], splat(1.0f) - sg, splat(1.0f));
+                                sums[(8 * ch + 4 * j + k) % NSUM] = sums[(8 * ch + 4 * j + k) % NSUM] + dd[k];
+                            }
+                            o[j] = pack8(dd);
+                        }
+                        uint4 *ob = reinterpret_cast<uint4 *>(a.out) + (int64_t)(2 * ch) * g.Pst;
+                        ob[p] = o[0];
+                        ob[g.Pst + p] = o[1];
+                        if (xedge) {
+                            ob[p + dxi] = o[0];
+                            ob[g.Pst + p + dxi] = o[1];
+                        }
+                        if (zedge || y == 0 || y == g.ny - 1) store_images<2>(g, ob, x, y, z, o);
+                    } else if (EPI == EPI_STATE) {
                         const Geom &sg = a.sg;
-                        float nv[3];
-#pragma unroll
-                        for (int k = 0; k < 3; ++k) nv[k] = s0v[k] + a.oscale[k] * (v[k] + sbias[k]);
-                        // the stencil's face ghosts: written by the cell they mirror
-                        const int ax = image_of(x, sg.nx, sg.bc), ay = image_of(y, sg.ny, sg.bc),
-                                  az = image_of(z, sg.nz, sg.bc);
-                        a.s1.eS[sa] = nv[0];
-                        a.s1.eL[sa] = nv[1];
-                        a.s1.c[sa] = nv[2];
+                        const float nv[3] = {s0v[0] + a.oscale[0] * (v[0].x() + sbias[0]),
+                                             s0v[1] + a.oscale[1] * (v[0].y() + sbias[1]),
+                                             s0v[2] + a.oscale[2] * (v[1].x() + sbias[2])};
+                        auto put = [&](int64_t b) {
+                            a.s1.eS[b] = nv[0];
+                            a.s1.eL[b] = nv[1];
+                            a.s1.c[b] = nv[2];
+                        };
+                        put(sa);
                         mass += (double)nv[2];
-                        if (ax != kNone) {
-                            const int64_t b = sg.at(ax, y, z);
-                            a.s1.eS[b] = nv[0]; a.s1.eL[b] = nv[1]; a.s1.c[b] = nv[2];
+                        // the stencil's face ghosts: written by the cell they mirror
+                        if (xedge) put(sa + dxi);
+                        if (zedge || y == 0 || y == g.ny - 1) {
+                            const int ay = image_of(y, sg.ny, sg.bc), az = image_of(z, sg.nz, sg.bc);
+                            if (ay != kNone) put(sg.at(x, ay, z));
+                            if (az != kNone) put(sg.at(x, y, az));
                         }
-                        if (ay != kNone) {
-                            const int64_t b = sg.at(x, ay, z);
-                            a.s1.eS[b] = nv[0]; a.s1.eL[b] = nv[1]; a.s1.c[b] = nv[2];
-                        }
-                        if (az != kNone) {
-                            const int64_t b = sg.at(x, y, az);
-                            a.s1.eS[b] = nv[0]; a.s1.eL[b] = nv[1]; a.s1.c[b] = nv[2];
-                        }
-                    }
-                } else if (EPI == EPI_LOSS) {
-                    if (active) {
-                        float gr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                    } else if (EPI == EPI_LOSS) {
+                        const float vv[3] = {v[0].x(), v[0].y(), v[1].x()};
+                        float gr[3];
 #pragma unroll
                         for (int c = 0; c < 3; ++c) {
                             const float tg = (s1v[c] - s0v[c]) / a.oscale[c];
-                            const float diff = v[c] + sbias[c] - tg;
-                            sums[HALF] += a.lw[c] * diff * diff;
+                            const float diff = vv[c] + sbias[c] - tg;
+                            lsum += a.lw[c] * diff * diff;
                             gr[c] = 2.0f * a.lw[c] * diff;
-                            sums[c] += gr[c];
                         }
-                        const uint4 o[1] = {pack8(gr)};
-                        store_with_images<1>(g, a.out, x, y, z, o);
+                        const V2<float> gp[4] = {V2<float>(gr[0], gr[1]), V2<float>(gr[2], 0.f), splat(0.f), splat(0.f)};
+                        sums[0] = sums[0] + gp[0];
+                        sums[1 % NSUM] = sums[1 % NSUM] + gp[1];
+                        const uint4 o[1] = {pack8(gp)};
+                        uint4 *ob = reinterpret_cast<uint4 *>(a.out);
+                        ob[p] = o[0];
+                        if (xedge) ob[p + dxi] = o[0];
+                        if (zedge || y == 0 || y == g.ny - 1) store_images<1>(g, ob, x, y, z, o);
                     }
                 }
             }
+            rows += n;
         }
         if (EPI == EPI_STATE) {
-            // deterministic per-CTA FP64 sum of the new c (warps 2-5 hold it)
+            // deterministic per-CTA FP64 sum of the new c
             double* redd = reinterpret_cast<double *>(smem + C::OFF_REDD);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
-            if (lane == 0 && ew < 4) redd[ew] = mass;
-            asm volatile("bar.sync 1, %0;" ::"r"(kEpiThreads) : "memory");
-            if (ew == 0 && lane == 0 && a.mass_part)
-                a.mass_part[blockIdx.x] = ((redd[0] + redd[1]) + redd[2]) + redd[3];
+            if (lane == 0) redd[ew] = mass;
+            asm volatile("bar.sync 1, %0;" ::"r"(32 * NEW) : "memory");
+            if (ew == 0 && lane == 0 && a.mass_part) {
+                double t = 0;
+                for (int k = 0; k < NEW; ++k) t += redd[k];
+                a.mass_part[blockIdx.x] = t;
+            }
         }
         if (EPI == EPI_DGRAD || EPI == EPI_LOSS) {
-            // deterministic per-CTA sums: warp shuffle, then the four warps
-            // of each column group in a fixed order
+            // deterministic per-CTA sums: warp shuffle, then the warps in order
 #pragma unroll
-            for (int c = 0; c <= HALF; ++c) {
-                float sv = sums[c];
+            for (int c = 0; c < 2 * NSUM; ++c) {
+                float sv = (c & 1) ? sums[c / 2].y() : sums[c / 2].x();
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
-                if (lane == 0) red[ew * (HALF + 1) + c] = sv;
+                if (lane == 0) red[ew * (CO + 1) + c] = sv;
             }
-            asm volatile("bar.sync 1, %0;" ::"r"(kEpiThreads) : "memory");
+            if (lane == 0)
+                for (int c = 2 * NSUM; c < CO; ++c) red[ew * (CO + 1) + c] = 0.f;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+            if (lane == 0) red[ew * (CO + 1) + CO] = lsum;
+            asm volatile("bar.sync 1, %0;" ::"r"(32 * NEW) : "memory");
             if (ew == 0) {
                 float *dst = a.partials + (int64_t)blockIdx.x * (CO + 1);
-                for (int c = lane; c < CO; c += 32) {
-                    const int grp = c / HALF, cc = c % HALF;
-                    const float *r = red + grp * 4 * (HALF + 1) + cc;
-                    dst[c] = ((r[0] + r[HALF + 1]) + r[2 * (HALF + 1)]) + r[3 * (HALF + 1)];
+                for (int c = lane; c <= CO; c += 32) {
+                    float t = 0.f;
+                    for (int k = 0; k < NEW; ++k) t += red[k * (CO + 1) + c];
+                    dst[c] = t;
                 }
-                if (lane == 0)
-                    dst[CO] = ((red[HALF] + red[(HALF + 1) + HALF]) + red[2 * (HALF + 1) + HALF]) +
-                              red[3 * (HALF + 1) + HALF];
             }
         }
     }
@@ -545,7 +572,7 @@ struct WgCfg {
     static constexpr int NSLOT = NMB * SPB;
     static constexpr int SEGB = (CX / 8) * kSegPlane;
     static constexpr int XB = NSLOT * SEGB;
-    static constexpr int ZB = (CZ / 8) * kTileX * 16;
+    static constexpr int ZB = (CZ / 8) * kSegPlane;
     static constexpr int STB = XB + ZB;
     static constexpr int NST = 2;
     static constexpr int OFF_BAR = NST * STB;
@@ -608,20 +635,20 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
                 const int xt = tt % nxt, y = (tt / nxt) % g.ny, z = tt / (nxt * g.ny);
                 const int x0 = xt * kTileX;
                 const uint32_t stage = sb + st * C::STB;
-                mbar_expect_tx(full(st), 9 * C::SEGB + C::ZB);
+                mbar_expect_tx(full(st), (9 * (CX / 8) + CZ / 8) * kSegBytes);
                 for (int dz = 0; dz < 3; ++dz)
                     for (int dy = 0; dy < 3; ++dy) {
                         const int64_t pv = g.p(x0 - 1, y + dy - 1, z + dz - 1);
                         for (int j = 0; j < CX / 8; ++j)
                             bulk_load(stage + (dz * 3 + dy) * C::SEGB + j * kSegPlane,
                                       reinterpret_cast<const unsigned char *>(a.x) + ((int64_t)j * g.Pst + pv) * 16,
-                                      kSegPlane, full(st));
+                                      kSegBytes, full(st));
                     }
-                const int64_t pz = g.p(x0, y, z);
+                const int64_t pz = g.p(x0 - 1, y, z);     // (from the aligned voxel before the tile)
                 for (int j = 0; j < CZ / 8; ++j)
-                    bulk_load(stage + C::XB + j * kTileX * 16,
+                    bulk_load(stage + C::XB + j * kSegPlane,
                               reinterpret_cast<const unsigned char *>(a.dz) + ((int64_t)j * g.Pst + pz) * 16,
-                              kTileX * 16, full(st));
+                              kSegBytes, full(st));
             }
             // drain the copies of the last stages
             const uint32_t issued = n;
@@ -634,7 +661,7 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
             // MN-major operands: LBO = stride of 8-voxel K groups (128 B),
             // SBO = stride of 8-channel groups (a segment plane / a dZ plane)
             const uint64_t a0 = smem_desc(sb, 128, kSegPlane);
-            const uint64_t b0 = smem_desc(sb + C::XB, 128, kTileX * 16);
+            const uint64_t b0 = smem_desc(sb + C::XB + 16, 128, kSegPlane);
             uint32_t n = 0;
             for (int tt = t0; tt < t1; ++tt, ++n) {
                 const uint32_t st = n % C::NST;
@@ -704,7 +731,7 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
 
 template <int CI, int CO, int EPI>
 cudaError_t conv_launch(const ConvArgs &a, int grid, cudaStream_t s) {
-    conv_kernel<CI, CO, EPI><<<grid, kConvThreads, ConvCfg<CI, CO>::SMEM, s>>>(a);
+    conv_kernel<CI, CO, EPI><<<grid, ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>::SMEM, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -749,11 +776,7 @@ cudaError_t wgrad_attr() {
 
 template <int CI, int CO>
 int conv_per_sm() {
-    // shared memory (228 KB per SM, 1 KB reserved per CTA) and TMEM (512 columns per SM)
-    const int by_smem = 233472 / (ConvCfg<CI, CO>::SMEM + 1024);
-    const int by_tmem = 512 / ConvCfg<CI, CO>::TMEM_COLS;
-    const int n = by_smem < by_tmem ? by_smem : by_tmem;
-    return n < 1 ? 1 : n;
+    return ConvCfg<CI, CO>::CTAS;
 }
 
 int conv_ctas_per_sm(int ci, int co) {
