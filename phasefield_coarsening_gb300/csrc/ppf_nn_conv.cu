@@ -25,13 +25,18 @@
 //   about 500 on a row's waits and descriptors, and every row's halo voxel in
 //   x sent its warp through the eight-image loop.
 //
-// wgrad_kernel<CX, CZ>: dW[tap][co][ci] = sum over voxels v of
-//   dZ[v][co] * X[v + tap][ci].  The reduction runs over voxels (K), both
-//   operands are channel-contiguous (MN-major).  Per tile the nine (dz, dy)
-//   segments sit in fixed slots laid out back to back, so one M = 128 block
-//   covers 128/CX slots x CX channels at a uniform group stride; the three
-//   dx shifts are three start offsets.  Per CTA the partial dW stays in
-//   TMEM over all its tiles and is written once at the end.
+// wgrad_kernel<CX, CZ>: dW[tap][co][ci] = sum over voxels u of
+//   X[u][ci] * dZ[u - tap][co] (periodic).  The reduction runs over voxels
+//   (K), both operands are channel-contiguous (MN-major).  A CTA marches
+//   columns of 128-voxel rows in y.  A row r of X comes as its three z planes
+//   (M = 128: three slots of CX channels and zeros), a row y of dZ three times,
+//   shifted by dx = -1, 0, 1 (N = 3 CZ); row r meets dZ rows r+1, r, r-1, one
+//   accumulator per dy.  dW stays in TMEM over all the CTA's rows and is
+//   written once at the end.
+//   What bounds it: 24 MMAs a row, 56 cycles each (N = 96), 1344 cycles a row;
+//   loading nine X segments for every tile (40 copies) and 72 MMAs of N = 32
+//   (40 cycles each) it took about 5200 (146 us for 32 -> 32 channels on
+//   64 x 128 x 128).
 //
 // Every mbarrier wait is bounded by a time limit; on expiry the CTA sets
 // the error word, stops issuing work, drains its own copies and MMAs
@@ -567,48 +572,59 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
 
 template <int CX, int CZ>
 struct WgCfg {
-    static constexpr int SPB = 128 / CX;                  // slots per M block
-    static constexpr int NMB = (9 + SPB - 1) / SPB;       // M blocks
-    static constexpr int NSLOT = NMB * SPB;
-    static constexpr int SEGB = (CX / 8) * kSegPlane;
-    static constexpr int XB = NSLOT * SEGB;
-    static constexpr int ZB = (CZ / 8) * kSegPlane;
-    static constexpr int STB = XB + ZB;
-    static constexpr int NST = 2;
-    static constexpr int OFF_BAR = NST * STB;
-    static constexpr int NBAR = 2 * NST + 1;
+    static constexpr int PL = kTileX * 16;                // one 8-channel plane of a row
+    static constexpr int NX = 3, NZ = 5;                  // rows of X, of dZ in shared memory
+    static constexpr int XSEG = (CX / 8) * PL;            // one z plane of a row of X
+    static constexpr int XB = 16 * PL;                    // M = 128 channels: three planes, then zeros
+    static constexpr int ZSEG = (CZ / 8) * PL, ZB = 3 * ZSEG;
+    static constexpr int OFF_Z = NX * XB;
+    static constexpr int OFF_BAR = OFF_Z + NZ * ZB;
+    static constexpr int NBAR = 2 * NX + 1;
     static constexpr int OFF_SLOT = OFF_BAR + NBAR * 8;
     static constexpr int SMEM = OFF_SLOT + 16;
-    static constexpr int NACC = NMB * 3;
-    static constexpr int COLS = NACC * CZ;
-    static constexpr int TMEM_COLS = COLS <= 32 ? 32 : COLS <= 64 ? 64 : COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
-    static_assert(COLS <= 512, "TMEM columns");
-    static_assert(STB % 16 == 0, "alignment");
+    static constexpr int NCOL = 3 * CZ;                   // one accumulator: dx, co
+    static constexpr int TMEM_COLS = 3 * NCOL <= 256 ? 256 : 512;
+    static_assert(3 * NCOL <= 512 && 3 * XSEG <= XB, "TMEM columns, M");
 };
 
+// A CTA's rows t0 .. t1-1 (y fastest, then x tile, then z) in columns: rows
+// ya .. yb-1 of one column at a time.
+struct WgCol {
+    int x0, z, ya, yb;
+};
+
+__device__ __forceinline__ WgCol wg_col(const NNGeom &g, int t, int t1) {
+    const int nxt = g.nx / kTileX, col = t / g.ny;
+    WgCol c;
+    c.ya = t - col * g.ny;
+    c.yb = min(g.ny, c.ya + (t1 - t));
+    c.x0 = (col % nxt) * kTileX;
+    c.z = col / nxt;
+    return c;
+}
+
 template <int CX, int CZ>
-__global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
+__global__ void __launch_bounds__(256, 1) wgrad_kernel(const __grid_constant__ WgradArgs a) {
     using C = WgCfg<CX, CZ>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t sb = smem_u32(smem), bars = sb + C::OFF_BAR;
     auto full = [&](uint32_t s) { return bars + 8 * s; };
-    auto empty = [&](uint32_t s) { return bars + 8 * (C::NST + s); };
-    const uint32_t dbar = bars + 8 * (2 * C::NST);
+    auto empty = [&](uint32_t s) { return bars + 8 * (C::NX + s); };
+    const uint32_t dbar = bars + 8 * (2 * C::NX);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + C::OFF_SLOT);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + C::OFF_SLOT + 4);
     const NNGeom &g = a.g;
-    const int nxt = g.nx / kTileX;
     const int t0 = (int)((int64_t)a.ntiles * blockIdx.x / gridDim.x);
     const int t1 = (int)((int64_t)a.ntiles * (blockIdx.x + 1) / gridDim.x);
 
-    // unused slots (past the nine taps) read as zeros
-    for (int st = 0; st < C::NST; ++st)
-        for (int i = tid; i < (C::NSLOT - 9) * C::SEGB / 16; i += blockDim.x)
-            reinterpret_cast<uint4 *>(smem + st * C::STB + 9 * C::SEGB)[i] = make_uint4(0, 0, 0, 0);
+    // the channels of M past the three z planes read as zeros
+    for (int st = 0; st < C::NX; ++st)
+        for (int i = tid; i < (C::XB - 3 * C::XSEG) / 16; i += blockDim.x)
+            reinterpret_cast<uint4 *>(smem + st * C::XB + 3 * C::XSEG)[i] = make_uint4(0, 0, 0, 0);
     fence_proxy_async_smem();
     if (tid == 0) {
-        for (int s = 0; s < C::NST; ++s) {
+        for (int s = 0; s < C::NX; ++s) {
             mbar_init(full(s), 1);
             mbar_init(empty(s), 1);
         }
@@ -622,73 +638,96 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
     tc_fence_after();
     const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(tslot);
 
-    if (warp == 0) {
+    // Unit n (counted over the CTA's columns) is a row r of X, ya - 1 .. yb, in
+    // X slot n % NX, and with it row r + 1 of dZ, the z-th of the CTA's, in dZ
+    // slot z % NZ.  A dZ row is last used by the second unit after the one that
+    // loads it, so when unit n - NX is done, the dZ slot is free too (NZ = NX + 2).
+    if (warp == 0 || warp >= 6) {
+        // ---- producers: thread k loads z plane k - 1 of X and the dZ row shifted by
+        // 1 - k; the first one announces the unit's bytes ----
         if (lane == 0) {
-            uint32_t n = 0;
-            for (int tt = t0; tt < t1; ++tt, ++n) {
-                const uint32_t st = n % C::NST;
-                if (n >= (uint32_t)C::NST &&
-                    !wait_backoff(empty(st), ((n / C::NST) + 1) & 1, a.limit_ns, abort_flag)) {
-                    fail(abort_flag, a.err, 1);
-                    break;
-                }
-                const int xt = tt % nxt, y = (tt / nxt) % g.ny, z = tt / (nxt * g.ny);
-                const int x0 = xt * kTileX;
-                const uint32_t stage = sb + st * C::STB;
-                mbar_expect_tx(full(st), (9 * (CX / 8) + CZ / 8) * kSegBytes);
-                for (int dz = 0; dz < 3; ++dz)
-                    for (int dy = 0; dy < 3; ++dy) {
-                        const int64_t pv = g.p(x0 - 1, y + dy - 1, z + dz - 1);
-                        for (int j = 0; j < CX / 8; ++j)
-                            bulk_load(stage + (dz * 3 + dy) * C::SEGB + j * kSegPlane,
-                                      reinterpret_cast<const unsigned char *>(a.x) + ((int64_t)j * g.Pst + pv) * 16,
-                                      kSegBytes, full(st));
+            const int k = warp == 0 ? 0 : warp - 5;
+            uint32_t n = 0, zr = 0;
+            bool ok = true;
+            for (int t = t0; ok && t < t1;) {
+                const WgCol c = wg_col(g, t, t1);
+                for (int r = c.ya - 1; r <= c.yb; ++r, ++n) {
+                    const uint32_t st = n % C::NX;
+                    if (n >= (uint32_t)C::NX &&
+                        !wait_backoff(empty(st), ((n / C::NX) + 1) & 1, a.limit_ns, abort_flag)) {
+                        fail(abort_flag, a.err, 1);
+                        ok = false;
+                        break;
                     }
-                const int64_t pz = g.p(x0 - 1, y, z);     // (from the aligned voxel before the tile)
-                for (int j = 0; j < CZ / 8; ++j)
-                    bulk_load(stage + C::XB + j * kSegPlane,
-                              reinterpret_cast<const unsigned char *>(a.dz) + ((int64_t)j * g.Pst + pz) * 16,
-                              kSegBytes, full(st));
+                    const bool z = r + 1 < c.yb;
+                    if (k == 0) mbar_expect_tx(full(st), 3 * C::XSEG + (z ? C::ZB : 0));
+                    const unsigned char *xs = reinterpret_cast<const unsigned char *>(a.x) + g.p(c.x0, r, c.z + k - 1) * 16;
+#pragma unroll
+                    for (int j = 0; j < CX / 8; ++j)
+                        bulk_load(sb + st * C::XB + k * C::XSEG + j * C::PL, xs + (int64_t)j * g.Pst * 16, C::PL, full(st));
+                    if (z) {
+                        const unsigned char *zs = reinterpret_cast<const unsigned char *>(a.dz) +
+                                                  g.p(c.x0 + 1 - k, r + 1, c.z) * 16;
+                        const uint32_t dst = sb + C::OFF_Z + (zr % C::NZ) * C::ZB + k * C::ZSEG;
+#pragma unroll
+                        for (int j = 0; j < CZ / 8; ++j)
+                            bulk_load(dst + j * C::PL, zs + (int64_t)j * g.Pst * 16, C::PL, full(st));
+                        ++zr;
+                    }
+                }
+                t += c.yb - c.ya;
             }
-            // drain the copies of the last stages
-            const uint32_t issued = n;
-            for (uint32_t k = issued > (uint32_t)C::NST ? issued - C::NST : 0; k < issued; ++k)
-                if (!mbar_wait(full(k % C::NST), (k / C::NST) & 1, a.limit_ns)) atomicOr(a.err, 4);
+            // drain the copies of the last units
+            for (uint32_t i = n > (uint32_t)C::NX ? n - C::NX : 0; i < n; ++i)
+                if (!mbar_wait(full(i % C::NX), (i / C::NX) & 1, a.limit_ns)) atomicOr(a.err, 4);
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = idesc_bf16(128, CZ, true, true);
-            // MN-major operands: LBO = stride of 8-voxel K groups (128 B),
-            // SBO = stride of 8-channel groups (a segment plane / a dZ plane)
-            const uint64_t a0 = smem_desc(sb, 128, kSegPlane);
-            const uint64_t b0 = smem_desc(sb + C::XB + 16, 128, kSegPlane);
-            uint32_t n = 0;
-            for (int tt = t0; tt < t1; ++tt, ++n) {
-                const uint32_t st = n % C::NST;
-                if (!wait_or_abort(full(st), (n / C::NST) & 1, a.limit_ns, abort_flag)) {
+            const uint32_t idesc = idesc_bf16(128, C::NCOL, true, true);
+            // MN-major operands: LBO = stride of 8-voxel K groups (128 B), SBO =
+            // stride of 8-channel groups (a plane)
+            const uint64_t a0 = smem_desc(sb, 128, C::PL);
+            const uint64_t b0 = smem_desc(sb + C::OFF_Z, 128, C::PL);
+            uint32_t n = 0, zr = 0;                        // units; dZ rows of earlier columns
+            uint32_t begun = 0;                            // accumulators written so far (bits)
+            bool ok = true;
+            auto ready = [&](uint32_t u) {
+                if (ok && !wait_or_abort(full(u % C::NX), (u / C::NX) & 1, a.limit_ns, abort_flag)) {
                     fail(abort_flag, a.err, 1);
-                    break;
+                    ok = false;
                 }
-                tc_fence_after();
-                const uint32_t so = (st * C::STB) >> 4;
+            };
+            if (t0 < t1) ready(0);
+            for (int t = t0; ok && t < t1;) {
+                const WgCol c = wg_col(g, t, t1);
+                t += c.yb - c.ya;
+                for (int r = c.ya - 1; ok && r <= c.yb; ++r, ++n) {
+                    tc_fence_after();
+                    const uint64_t ax = a0 + (((n % C::NX) * C::XB) >> 4);
 #pragma unroll
-                for (int kb = 0; kb < kTileX / 16; ++kb) {
-                    const uint64_t bd = b0 + so + ((kb * 16 * 16) >> 4);
+                    for (int dy = 0; dy < 3; ++dy) {       // X row r meets dZ row y = r - (dy - 1)
+                        const int y = r + 1 - dy;
+                        // before the last MMAs of a unit, wait for the next one, so that its
+                        // MMAs follow at once
+                        if (dy == 2 && (r < c.yb || t < t1)) ready(n + 1);
+                        if (y < c.ya || y >= c.yb) continue;
+                        const uint64_t bz = b0 + ((((zr + (uint32_t)(y - c.ya)) % C::NZ) * C::ZB) >> 4);
+                        const uint32_t d = tbase + dy * C::NCOL;
+                        const uint32_t more = (begun >> dy) & 1u;
 #pragma unroll
-                    for (int mb = 0; mb < C::NMB; ++mb)
-#pragma unroll
-                        for (int dx = 0; dx < 3; ++dx) {
-                            const uint64_t ad = a0 + so + ((mb * C::SPB * C::SEGB + (kb * 16 + dx) * 16) >> 4);
-                            mma_bf16(tbase + (mb * 3 + dx) * CZ, ad, bd, idesc, (n > 0 || kb > 0) ? 1u : 0u);
-                        }
+                        for (int kb = 0; kb < kTileX / 16; ++kb)
+                            mma_bf16(d, ax + kb * 16, bz + kb * 16, idesc, kb ? 1u : more);
+                        begun |= 1u << dy;
+                    }
+                    mma_commit(empty(n % C::NX));
                 }
-                mma_commit(empty(st));
+                zr += (uint32_t)(c.yb - c.ya);
             }
             mma_commit(dbar);
         }
     }
     // epilogue: all four lane quarters; wait for the last MMA
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 6) {
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const bool have = t1 > t0;
@@ -699,24 +738,20 @@ __global__ void __launch_bounds__(192, 1) wgrad_kernel(const WgradArgs a) {
         }
         tc_fence_after();
         float *out = a.partials + (int64_t)blockIdx.x * 27 * CZ * CX;
-        for (int mb = 0; mb < C::NMB; ++mb) {
-            const int slot = mb * C::SPB + row / CX, ci = row % CX;
-            for (int dx = 0; dx < 3; ++dx) {
+        const int dz = row / CX, ci = row % CX;
+        for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
-                for (int c16 = 0; c16 < CZ / 16; ++c16) {
-                    float v[16];
-                    tmem_ld16(tbase + ((uint32_t)(quarter * 32) << 16) + (mb * 3 + dx) * CZ + 16 * c16, v);
-                    if (slot < 9) {
-                        const int tap = (slot / 3) * 9 + (slot % 3) * 3 + dx;
+            for (int c16 = 0; c16 < C::NCOL / 16; ++c16) {
+                float v[16];
+                tmem_ld16(tbase + ((uint32_t)(quarter * 32) << 16) + dy * C::NCOL + 16 * c16, v);
+                if (dz < 3) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i)
-                            out[((int64_t)tap * CZ + 16 * c16 + i) * CX + ci] = (ok && have) ? v[i] : 0.f;
+                    for (int i = 0; i < 16; ++i) {
+                        const int dx = (16 * c16 + i) / CZ, co = (16 * c16 + i) % CZ;
+                        out[((int64_t)(dz * 9 + dy * 3 + dx) * CZ + co) * CX + ci] = (ok && have) ? v[i] : 0.f;
                     }
                 }
             }
-        }
-    } else if (warp == 1) {
-        // the MMA warp's other lanes wait here too, so every role ends below
     }
     tc_fence_before();
     __syncthreads();
@@ -825,10 +860,10 @@ cudaError_t launch_conv(int ci, int co, int epi, const ConvArgs &a, int grid, cu
 }
 
 cudaError_t launch_wgrad(int cx, int cz, const WgradArgs &a, int grid, cudaStream_t s) {
-    if (cx == 16 && cz == 16) wgrad_kernel<16, 16><<<grid, 192, WgCfg<16, 16>::SMEM, s>>>(a);
-    else if (cx == 16 && cz == 32) wgrad_kernel<16, 32><<<grid, 192, WgCfg<16, 32>::SMEM, s>>>(a);
-    else if (cx == 32 && cz == 16) wgrad_kernel<32, 16><<<grid, 192, WgCfg<32, 16>::SMEM, s>>>(a);
-    else if (cx == 32 && cz == 32) wgrad_kernel<32, 32><<<grid, 192, WgCfg<32, 32>::SMEM, s>>>(a);
+    if (cx == 16 && cz == 16) wgrad_kernel<16, 16><<<grid, 256, WgCfg<16, 16>::SMEM, s>>>(a);
+    else if (cx == 16 && cz == 32) wgrad_kernel<16, 32><<<grid, 256, WgCfg<16, 32>::SMEM, s>>>(a);
+    else if (cx == 32 && cz == 16) wgrad_kernel<32, 16><<<grid, 256, WgCfg<32, 16>::SMEM, s>>>(a);
+    else if (cx == 32 && cz == 32) wgrad_kernel<32, 32><<<grid, 256, WgCfg<32, 32>::SMEM, s>>>(a);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }

@@ -192,20 +192,43 @@ __global__ void __launch_bounds__(kNT) sparse_kernel(Geom sg, float *c, const Ma
     }
 }
 
-// out[i] = sum_b part[b * stride + i] (fixed order, FP64 accumulation)
-__global__ void __launch_bounds__(kNT) reduce_kernel(const float *part, int nb, int stride, int n, float *out) {
-    for (int i = blockIdx.x * kNT + threadIdx.x; i < n; i += gridDim.x * kNT) {
-        double s = 0;
-        for (int b = 0; b < nb; ++b) s += (double)part[(int64_t)b * stride + i];
-        out[i] = (float)s;
-    }
-}
-
-__global__ void loss_kernel(const float *part, int nb, int stride, int idx, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0;
-        for (int b = 0; b < nb; ++b) s += (double)part[(int64_t)b * stride + idx];
-        *out = s;
+// out[i] = sum_b part[b * stride + i] for i < n, and with `loss` set also
+// *loss = sum_b part[b * stride + li], in a fixed order.  A block takes 32
+// values, its eight warps an eighth of the partial sums each: independent
+// loads in flight instead of one thread's chain (21 us for 152 partials of
+// 27 x 32 x 32 weights), and sums carried with their rounding errors in float
+// (Knuth's TwoSum, about 48 bits) instead of FP64, whose conversions and
+// additions alone would take 14 us.
+__global__ void __launch_bounds__(kNT) reduce_kernel(const float *part, int nb, int stride, int n, float *out, int li,
+                                                     double *loss) {
+    __shared__ float2 red[kNT / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto add = [](float2 &a, float x) {
+        const float s = a.x + x, bp = s - a.x;
+        a.y += (a.x - (s - bp)) + (x - bp);
+        a.x = s;
+    };
+    const int b0 = nb * warp / (kNT / 32), b1 = nb * (warp + 1) / (kNT / 32);
+    const int nv = n + (loss ? 1 : 0);
+    for (int i0 = blockIdx.x * 32; i0 < nv; i0 += gridDim.x * 32) {
+        const int i = i0 + lane, col = i < n ? i : li;
+        float2 s = make_float2(0.f, 0.f);
+        if (i < nv) {
+#pragma unroll 8
+            for (int b = b0; b < b1; ++b) add(s, part[(int64_t)b * stride + col]);
+        }
+        red[warp][lane] = s;
+        __syncthreads();
+        if (warp == 0 && i < nv) {
+            for (int w = 1; w < kNT / 32; ++w) {
+                const float2 o = red[w][lane];
+                add(s, o.x);
+                s.y += o.y;
+            }
+            if (i < n) out[i] = s.x + s.y;
+            else *loss = (double)s.x + (double)s.y;
+        }
+        __syncthreads();
     }
 }
 
@@ -261,6 +284,7 @@ struct ppf_surrogate {
     double *stage = nullptr;
     size_t scratch_elems = 0;
     int conv_grid[2][2] = {}, wgrad_grid = 0;
+    int yc[2][2] = {};           // rows per work item of the current shape
     int inject = 0;              // test hook: the next convolution's wait runs out
 };
 
@@ -306,6 +330,21 @@ int check_ctx(ppf_ctx *c) {
     return PPF_OK;
 }
 
+// Rows per work item: a CTA's rows are its items' plus two halo rows each, so
+// a length that gives the busiest CTA few of them (64 x 128 x 128 on 152
+// CTAs: items of 19 rows, 63 in all, where 4-row items made 84); of lengths
+// within 2 % the shortest, whose CTAs stay closer together in z and share
+// more of their input rows through the L2 (256^3: 32 rows 45.9 ms a cycle of
+// ten calls, 128 rows 46.9 ms).
+int pick_yc(const NNGeom &g, int grid) {
+    const int64_t cols = (int64_t)g.nz * (g.nx / kTileX);
+    auto rows = [&](int c) { return (cols * ((g.ny + c - 1) / c) + grid - 1) / grid * (c + 2); };
+    int64_t least = rows(g.ny);
+    for (int c = 1; c < g.ny; ++c) least = std::min(least, rows(c));
+    for (int c = 1;; ++c)
+        if (rows(c) * 50 <= least * 51) return c;
+}
+
 int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
     int rc = check_ctx(c);
     if (rc) return rc;
@@ -316,6 +355,8 @@ int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
         if ((rc = alloc_zero((void **)&s->feat, act_bytes(s->g, 16), c->stream))) return rc;
         for (auto &p : s->act)
             if ((rc = alloc_zero((void **)&p, act_bytes(s->g, s->W), c->stream))) return rc;
+        for (int p = 0; p < 2; ++p)
+            for (int q = 0; q < 2; ++q) s->yc[p][q] = pick_yc(s->g, s->conv_grid[p][q]);
         s->wz = c->nz;
         s->wy = c->ny;
         s->wx = c->nx;
@@ -338,13 +379,6 @@ int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
     return PPF_OK;
 }
 
-int pick_yc(const NNGeom &g, int grid) {
-    const int64_t nxt = g.nx / kTileX;
-    int yc = 32;
-    while (yc > 4 && (int64_t)g.nz * ((g.ny + yc - 1) / yc) * nxt < 8LL * grid) yc /= 2;
-    return yc;
-}
-
 Fields<const float> cur_fields(ppf_ctx *c) {
     return {(const float *)c->fld[c->cur_eta][0], (const float *)c->fld[c->cur_eta][1],
             (const float *)c->fld[c->cur_c][2]};
@@ -357,8 +391,7 @@ ConvArgs conv_args(ppf_surrogate *s, ppf_ctx *c, int layer, const uint16_t *x, c
     a.wimg = wimg;
     a.bias = s->params + s->boff[layer];
     a.sg = c->g;
-    const int grid = s->conv_grid[s->ci[layer] == 32][s->co[layer] == 32];
-    a.yc = pick_yc(s->g, grid);
+    a.yc = s->yc[s->ci[layer] == 32][s->co[layer] == 32];
     a.items = s->g.nz * ((s->g.ny + a.yc - 1) / a.yc) * (s->g.nx / kTileX);
     a.err = c->derr;
     a.limit_ns = c->wait_limit_ns;
@@ -407,9 +440,10 @@ int forward_hidden(ppf_surrogate *s, ppf_ctx *c, bool train) {
     return PPF_OK;
 }
 
-int reduce_into(ppf_surrogate *s, ppf_ctx *c, const float *part, int nb, int stride, int n, float *out) {
-    const int blocks = std::max(1, std::min((n + kNT - 1) / kNT, 4 * s->num_sms));
-    reduce_kernel<<<blocks, kNT, 0, c->stream>>>(part, nb, stride, n, out);
+int reduce_into(ppf_surrogate *s, ppf_ctx *c, const float *part, int nb, int stride, int n, float *out, int li = 0,
+                double *loss = nullptr) {
+    const int blocks = std::min((n + 32) / 32, 8 * s->num_sms);
+    reduce_kernel<<<blocks, kNT, 0, c->stream>>>(part, nb, stride, n, out, li, loss);
     SCU(cudaGetLastError());
     return PPF_OK;
 }
@@ -448,9 +482,7 @@ int loss_grad(ppf_surrogate *s, ppf_ctx *in, ppf_ctx *tg) {
         a.s1 = {const_cast<float *>(t.eS), const_cast<float *>(t.eL), const_cast<float *>(t.c)};
         if ((rc = run_conv(s, in, s->ci[5], 16, EPI_LOSS, a))) return rc;
         const int grid = s->conv_grid[s->ci[5] == 32][0];
-        if ((rc = reduce_into(s, in, s->bpart, grid, 17, 16, s->grads + s->boff[5]))) return rc;
-        loss_kernel<<<1, 32, 0, in->stream>>>(s->bpart, grid, 17, 16, s->dscal);
-        SCU(cudaGetLastError());
+        if ((rc = reduce_into(s, in, s->bpart, grid, 17, 16, s->grads + s->boff[5], 16, s->dscal))) return rc;
     }
     if ((rc = wgrad(s, in, 5, s->act[4], s->g16))) return rc;
     const uint16_t *cur = s->g16;
