@@ -71,7 +71,7 @@ struct ConvArgs {
     Fields<float> s1;       // EPI_STATE: state written; EPI_LOSS: target state (read)
     float oscale[3];        // output scale per state channel
     float lw[3];            // loss weight per channel, including 1/count
-    int yc;                 // rows per work item
+    int nyc;                // work items per column of ny rows, at most ny / 2
     int items;
     int *err;
     unsigned long long limit_ns;

@@ -143,7 +143,7 @@ __device__ __noinline__ void store_images(const NNGeom &g, uint4 *base, int x, i
 
 template <int CI, int CO>
 struct ConvCfg {
-    static constexpr int RING = CI == 32 ? 6 : 5;        // input-row slots in shared memory
+    static constexpr int RING = 6;                       // input-row slots in shared memory
     static constexpr int ND = 5;                         // TMEM tiles (one per input row)
     static constexpr int NCOL = 3 * CO;                  // one tile: contributions to rows y+1, y, y-1
     static constexpr int SEGB = (CI / 8) * kSegPlane;    // one segment, all channel planes
@@ -169,6 +169,15 @@ struct ConvCfg {
     static constexpr int producer2(int epi) { return 2 + 4 * groups(epi); }
     static constexpr int mma2(int epi) { return producer2(epi) + 2; }
     static constexpr int threads(int epi) { return 32 * (mma2(epi) + 1); }
+    // A parity wait is sound only if the phase before the awaited one is known to
+    // be complete; otherwise it returns at once.  The MMA issuers take alternate
+    // rows, so with an even RING the row that used a slot before is the issuer's
+    // own, whose data it has waited for; with RING = 5 it was the other issuer's,
+    // and an issuer could start on a row that had not arrived when an earlier
+    // row's copies were late by three rows.  For the epilogue's waits, items have
+    // at least two rows: over items of one row, three groups in turn lie nine
+    // tiles apart, more than the ND the tile ring remembers.
+    static_assert(RING % 2 == 0, "a slot's rows belong to one MMA issuer");
     static_assert(CI % 16 == 0 && CO % 16 == 0 && CO <= 32, "channel counts");
     static_assert(ND * NCOL <= 512 && NCOL <= 256, "TMEM / MMA N");
     static_assert(OFF_W % 16 == 0 && OFF_BAR % 8 == 0, "alignment");
@@ -178,17 +187,16 @@ struct Item {
     int z, x0, y0, y1;
 };
 
-__device__ __forceinline__ Item item_of(const NNGeom &g, int yc, int it) {
+__device__ __forceinline__ Item item_of(const NNGeom &g, int nyc, int it) {
     const int nxt = g.nx / kTileX;
-    const int nyc = (g.ny + yc - 1) / yc;
     Item r;
     const int xt = it % nxt;
     const int rest = it / nxt;
     const int yi = rest % nyc;
     r.z = rest / nyc;
     r.x0 = xt * kTileX;
-    r.y0 = yi * yc;
-    r.y1 = min(g.ny, r.y0 + yc);
+    r.y0 = yi * g.ny / nyc;
+    r.y1 = (yi + 1) * g.ny / nyc;
     return r;
 }
 
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
             uint32_t q = 0;
             bool ok = true;
             for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
-                const Item w = item_of(g, a.yc, it);
+                const Item w = item_of(g, a.nyc, it);
                 const unsigned char *src = reinterpret_cast<const unsigned char *>(a.x) +
                                            g.p(w.x0 - 1, w.y0 - 1, w.z + dz - 1) * 16;
                 for (int r = w.y0 - 1; r <= w.y1; ++r, ++q, src += (int64_t)g.X * 16) {
@@ -307,7 +315,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
             if (!ok) fail(abort_flag, a.err, 1);
             uint32_t total = 0;                            // input rows of the CTA's items
             for (int it = blockIdx.x; it < a.items; it += gridDim.x) {
-                const Item w = item_of(g, a.yc, it);
+                const Item w = item_of(g, a.nyc, it);
                 total += (uint32_t)(w.y1 - w.y0) + 2;
             }
             for (uint32_t q = mine; ok && q < total; q += 2) {
@@ -363,7 +371,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
             return wait_backoff(dfull(t % C::ND), (t / C::ND) & 1, a.limit_ns, abort_flag);
         };
         for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
-            const Item w = item_of(g, a.yc, it);
+            const Item w = item_of(g, a.nyc, it);
             const uint32_t qb = q, n = (uint32_t)(w.y1 - w.y0);  // input row y0 - 1; output rows
             q += n + 2;
             const int x = w.x0 + row, z = w.z;
@@ -401,6 +409,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
                     ok = false;
                     break;
                 }
+                __syncwarp();
                 tc_fence_after();
                 // out[y] = sum_dy W_dy in[y + dy]: the dy = -1 block of
                 // D_{y-1}, the dy = 0 block of D_y, the dy = +1 block of D_{y+1}
@@ -736,6 +745,7 @@ __global__ void __launch_bounds__(256, 1) wgrad_kernel(const __grid_constant__ W
             fail(abort_flag, a.err, 1);
             ok = false;
         }
+        __syncwarp();
         tc_fence_after();
         float *out = a.partials + (int64_t)blockIdx.x * 27 * CZ * CX;
         const int dz = row / CX, ci = row % CX;

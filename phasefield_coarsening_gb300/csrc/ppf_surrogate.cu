@@ -284,7 +284,7 @@ struct ppf_surrogate {
     double *stage = nullptr;
     size_t scratch_elems = 0;
     int conv_grid[2][2] = {}, wgrad_grid = 0;
-    int yc[2][2] = {};           // rows per work item of the current shape
+    int nyc[2][2] = {};          // work items per column of the current shape
     int inject = 0;              // test hook: the next convolution's wait runs out
 };
 
@@ -330,19 +330,19 @@ int check_ctx(ppf_ctx *c) {
     return PPF_OK;
 }
 
-// Rows per work item: a CTA's rows are its items' plus two halo rows each, so
-// a length that gives the busiest CTA few of them (64 x 128 x 128 on 152
-// CTAs: items of 19 rows, 63 in all, where 4-row items made 84); of lengths
-// within 2 % the shortest, whose CTAs stay closer together in z and share
-// more of their input rows through the L2 (256^3: 32 rows 45.9 ms a cycle of
-// ten calls, 128 rows 46.9 ms).
-int pick_yc(const NNGeom &g, int grid) {
+// Work items per column of ny rows, of at least two rows each: a CTA's rows
+// are its items' plus two halo rows each, so a count that gives the busiest CTA
+// few of them (64 x 128 x 128 on 152 CTAs: items of 18-19 rows, 63 in all,
+// where 4-row items made 84); of counts within 2 % the largest, whose CTAs stay
+// closer together in z and share more of their input rows through the L2
+// (256^3: 32 rows 45.9 ms a cycle of ten calls, 128 rows 46.9 ms).
+int pick_nyc(const NNGeom &g, int grid) {
     const int64_t cols = (int64_t)g.nz * (g.nx / kTileX);
-    auto rows = [&](int c) { return (cols * ((g.ny + c - 1) / c) + grid - 1) / grid * (c + 2); };
-    int64_t least = rows(g.ny);
-    for (int c = 1; c < g.ny; ++c) least = std::min(least, rows(c));
-    for (int c = 1;; ++c)
-        if (rows(c) * 50 <= least * 51) return c;
+    auto rows = [&](int k) { return (cols * k + grid - 1) / grid * ((g.ny + k - 1) / k + 2); };
+    int64_t least = rows(1);
+    for (int k = 2; k <= g.ny / 2; ++k) least = std::min(least, rows(k));
+    for (int k = g.ny / 2;; --k)
+        if (rows(k) * 50 <= least * 51) return k;
 }
 
 int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
@@ -356,7 +356,7 @@ int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
         for (auto &p : s->act)
             if ((rc = alloc_zero((void **)&p, act_bytes(s->g, s->W), c->stream))) return rc;
         for (int p = 0; p < 2; ++p)
-            for (int q = 0; q < 2; ++q) s->yc[p][q] = pick_yc(s->g, s->conv_grid[p][q]);
+            for (int q = 0; q < 2; ++q) s->nyc[p][q] = pick_nyc(s->g, s->conv_grid[p][q]);
         s->wz = c->nz;
         s->wy = c->ny;
         s->wx = c->nx;
@@ -391,8 +391,8 @@ ConvArgs conv_args(ppf_surrogate *s, ppf_ctx *c, int layer, const uint16_t *x, c
     a.wimg = wimg;
     a.bias = s->params + s->boff[layer];
     a.sg = c->g;
-    a.yc = s->yc[s->ci[layer] == 32][s->co[layer] == 32];
-    a.items = s->g.nz * ((s->g.ny + a.yc - 1) / a.yc) * (s->g.nx / kTileX);
+    a.nyc = s->nyc[s->ci[layer] == 32][s->co[layer] == 32];
+    a.items = s->g.nz * a.nyc * (s->g.nx / kTileX);
     a.err = c->derr;
     a.limit_ns = c->wait_limit_ns;
     for (int k = 0; k < 3; ++k) {
