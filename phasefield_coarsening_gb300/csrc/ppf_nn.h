@@ -6,7 +6,7 @@
 // (nz, ny, nx) domain with a one-voxel halo is stored as C/8 planes of
 // 16-byte voxels (8 BF16 channels each):
 //   byte (j, x, y, z) = (j * Pst + p(x, y, z)) * 16,  p = (z+1) YX + (y+1) X + (x+1)
-// with X = nx+2, YX = (ny+2)(nx+2), Pst >= (nz+2) YX.  A run of voxels
+// with X = nx+2 rounded up to 8, YX = (ny+2) X, Pst >= (nz+2) YX.  A run of voxels
 // along x is then a run of 16-byte rows, which is exactly the no-swizzle
 // core-matrix layout of the tensor-core operands: shifting a convolution
 // tap by one voxel in x moves an operand's start address by 16 bytes.
@@ -88,9 +88,7 @@ struct WgradArgs {
     unsigned long long limit_ns;
 };
 
-int conv_smem_bytes(int ci, int co);
 int conv_ctas_per_sm(int ci, int co);
-int wgrad_smem_bytes(int cx, int cz);
 cudaError_t conv_setup(int max_smem_optin);
 cudaError_t launch_conv(int ci, int co, int epi, const ConvArgs &a, int grid, cudaStream_t s);
 cudaError_t launch_wgrad(int cx, int cz, const WgradArgs &a, int grid, cudaStream_t s);

@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
         float lsum = 0.f;                                  // the loss
 #pragma unroll
         for (int c = 0; c < NSUM; ++c) sums[c] = splat(0.f);
-        double mass = 0.0;
+        Mass1 msum;
         uint32_t q = 0, rows = 0;
         bool ok = true;
         auto wait_d = [&](uint32_t t) {
@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
                             a.s1.c[b] = nv[2];
                         };
                         put(sa);
-                        mass += (double)nv[2];
+                        msum.add(nv[2]);
                         // the stencil's face ghosts: written by the cell they mirror
                         if (xedge) put(sa + dxi);
                         if (zedge || y == 0 || y == g.ny - 1) {
@@ -533,7 +533,8 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
         }
         if (EPI == EPI_STATE) {
             // deterministic per-CTA FP64 sum of the new c
-            double* redd = reinterpret_cast<double *>(smem + C::OFF_REDD);
+            double *redd = reinterpret_cast<double *>(smem + C::OFF_REDD);
+            double mass = msum.get();
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) mass += __shfl_xor_sync(0xffffffffu, mass, o);
             if (lane == 0) redd[ew] = mass;
@@ -830,22 +831,6 @@ int conv_ctas_per_sm(int ci, int co) {
     if (ci == 32 && co == 16) return conv_per_sm<32, 16>();
     if (ci == 32 && co == 32) return conv_per_sm<32, 32>();
     return 1;
-}
-
-int conv_smem_bytes(int ci, int co) {
-    if (ci == 16 && co == 16) return ConvCfg<16, 16>::SMEM;
-    if (ci == 16 && co == 32) return ConvCfg<16, 32>::SMEM;
-    if (ci == 32 && co == 16) return ConvCfg<32, 16>::SMEM;
-    if (ci == 32 && co == 32) return ConvCfg<32, 32>::SMEM;
-    return -1;
-}
-
-int wgrad_smem_bytes(int cx, int cz) {
-    if (cx == 16 && cz == 16) return WgCfg<16, 16>::SMEM;
-    if (cx == 16 && cz == 32) return WgCfg<16, 32>::SMEM;
-    if (cx == 32 && cz == 16) return WgCfg<32, 16>::SMEM;
-    if (cx == 32 && cz == 32) return WgCfg<32, 32>::SMEM;
-    return -1;
 }
 
 cudaError_t conv_setup(int max_smem_optin) {

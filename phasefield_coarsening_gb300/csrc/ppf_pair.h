@@ -63,4 +63,72 @@ __device__ __forceinline__ V2<double> ld2(const double *p) { return V2<double>(*
 __device__ __forceinline__ void st2(float *p, V2<float> v) { *reinterpret_cast<float2 *>(p) = v.v; }
 __device__ __forceinline__ void st2(double *p, V2<double> v) { *reinterpret_cast<double2 *>(p) = make_double2(v.a, v.b); }
 
+// sums of pairs of floats carried with their rounding errors (Knuth's TwoSum)
+__device__ __forceinline__ V2<float> two_sum(V2<float> a, V2<float> x, V2<float> &err) {
+    const V2<float> s = a + x;
+    const V2<float> bp = s - a;
+    err = (a - (s - bp)) + (x - bp);
+    return s;
+}
+
+__device__ __forceinline__ float two_sum1(float a, float x, float &err) {
+    const float s = a + x;
+    const float bp = s - a;
+    err = (a - (s - bp)) + (x - bp);
+    return s;
+}
+
+template <typename T>
+struct Sum;   // a pair of running sums, about 48 bits or better
+template <>
+struct Sum<float> {
+    V2<float> hi = splat(0.f), lo = splat(0.f);
+    __device__ __forceinline__ void add(V2<float> x) {
+        V2<float> e;
+        hi = two_sum(hi, x, e);
+        lo = lo + e;
+    }
+    __device__ __forceinline__ double get() const {
+        float e;
+        const float h = two_sum1(hi.x(), hi.y(), e);
+        return (double)h + (double)(lo.x() + lo.y() + e);
+    }
+};
+template <>
+struct Sum<double> {
+    V2<double> s = splat(0.0);
+    __device__ __forceinline__ void add(V2<double> x) { s = s + x; }
+    __device__ __forceinline__ double get() const { return s.x() + s.y(); }
+};
+
+template <typename T>
+struct Mass : Sum<double> {};   // FP64: the plain sum
+template <>
+struct Mass<float> {            // FP32: three parts
+    V2<float> hi = splat(0.f), mid = splat(0.f), lo = splat(0.f);
+    __device__ __forceinline__ void add(V2<float> x) {
+        V2<float> e, f;
+        hi = two_sum(hi, x, e);
+        mid = two_sum(mid, e, f);
+        lo = lo + f;
+    }
+    __device__ __forceinline__ double get() const {
+        float e, f, q;
+        const float h = two_sum1(hi.x(), hi.y(), e);
+        const float m = two_sum1(two_sum1(mid.x(), mid.y(), f), e, q);
+        return (double)h + ((double)m + (double)(lo.x() + lo.y() + f + q));
+    }
+};
+
+struct Mass1 {   // Mass<float> of single floats
+    float hi = 0.f, mid = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        float e, f;
+        hi = two_sum1(hi, x, e);
+        mid = two_sum1(mid, e, f);
+        lo += f;
+    }
+    __device__ __forceinline__ double get() const { return (double)hi + ((double)mid + (double)lo); }
+};
+
 }  // namespace ppf

@@ -265,65 +265,8 @@ cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[
 // accumulation per cell is what bounded the FP32 form (one conversion and
 // one addition per cell, each 1/64 of the FP32 rate); the FP64 state's form
 // in FP64 arithmetic is bound by the FP64 pipe, so it has few operations
-// (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 54 us (186 us with one cell per thread
-// and FP64 sums of the solute mass); 64^3: 7 us (33 us).
-
-// sums of pairs of floats carried with their rounding errors (Knuth's TwoSum)
-__device__ __forceinline__ V2<float> two_sum(V2<float> a, V2<float> x, V2<float> &err) {
-    const V2<float> s = a + x;
-    const V2<float> bp = s - a;
-    err = (a - (s - bp)) + (x - bp);
-    return s;
-}
-
-__device__ __forceinline__ float two_sum1(float a, float x, float &err) {
-    const float s = a + x;
-    const float bp = s - a;
-    err = (a - (s - bp)) + (x - bp);
-    return s;
-}
-
-template <typename T>
-struct Sum;   // a pair of running sums, about 48 bits or better
-template <>
-struct Sum<float> {
-    V2<float> hi = splat(0.f), lo = splat(0.f);
-    __device__ __forceinline__ void add(V2<float> x) {
-        V2<float> e;
-        hi = two_sum(hi, x, e);
-        lo = lo + e;
-    }
-    __device__ __forceinline__ double get() const {
-        float e;
-        const float h = two_sum1(hi.x(), hi.y(), e);
-        return (double)h + (double)(lo.x() + lo.y() + e);
-    }
-};
-template <>
-struct Sum<double> {
-    V2<double> s = splat(0.0);
-    __device__ __forceinline__ void add(V2<double> x) { s = s + x; }
-    __device__ __forceinline__ double get() const { return s.x() + s.y(); }
-};
-
-template <typename T>
-struct Mass : Sum<double> {};   // FP64: the plain sum
-template <>
-struct Mass<float> {            // FP32: three parts
-    V2<float> hi = splat(0.f), mid = splat(0.f), lo = splat(0.f);
-    __device__ __forceinline__ void add(V2<float> x) {
-        V2<float> e, f;
-        hi = two_sum(hi, x, e);
-        mid = two_sum(mid, e, f);
-        lo = lo + f;
-    }
-    __device__ __forceinline__ double get() const {
-        float e, f, q;
-        const float h = two_sum1(hi.x(), hi.y(), e);
-        const float m = two_sum1(two_sum1(mid.x(), mid.y(), f), e, q);
-        return (double)h + ((double)m + (double)(lo.x() + lo.y() + f + q));
-    }
-};
+// (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 54 us (186 us with
+// one cell per thread and FP64 sums of the solute mass); 64^3: 7 us (33 us).
 
 // 1/x of a pair: the hardware's estimate (about 1 ulp) and a Newton step
 __device__ __forceinline__ V2<float> recip(V2<float> x) {

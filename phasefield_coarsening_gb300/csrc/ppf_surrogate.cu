@@ -36,6 +36,7 @@
 #include "ppf_ctx.h"
 #include "ppf_internal.h"
 #include "ppf_nn.h"
+#include "ppf_pair.h"
 
 using namespace ppf;
 using namespace ppf::nn;
@@ -59,14 +60,6 @@ int serr(int code, const char *fmt, ...) {
         cudaError_t e_ = (x);                                                                    \
         if (e_ != cudaSuccess) return serr(PPF_ECUDA, "%s: %s", #x, cudaGetErrorString(e_));     \
     } while (0)
-
-__device__ __forceinline__ int face_images(int x, int n, int bc, int (&o)[3]) {
-    int k = 0;
-    o[k++] = x;
-    if (x == 0) o[k++] = bc == 0 ? n : -1;
-    if (x == n - 1) o[k++] = bc == 0 ? -1 : n;
-    return k;
-}
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -96,100 +89,188 @@ __device__ __forceinline__ void block_sum_to(double s, double *out) {
 // BF16 features (etaS, etaL, composition feature; channels 8..15 live in
 // the second plane, zero from allocation and never written), with every
 // halo image; also the per-CTA FP64 sum of c (the mass before the call).
-// One block per x row (grid-stride over rows).
+// Bound by HBM: 12 bytes read and 16 written per cell.  A warp takes 128
+// voxels of a row, lane after lane, so that each 16-byte store instruction
+// fills whole lines; images are stored only by the rows and voxels that have
+// them, and the mass is summed in three floats per thread: a conversion and
+// an addition in FP64 per cell took longer than the memory traffic.  256^3:
+// 78 us, was 152 us.
 __global__ void __launch_bounds__(kNT) features_kernel(Geom sg, Fields<const float> s, NNGeom g, uint16_t *act,
                                                        float cS, float cL, float kc, double *mass_part) {
-    double m = 0;
-    const int nrows = g.ny * g.nz;
-    for (int rr = blockIdx.x; rr < nrows; rr += gridDim.x) {
-        const int y = rr % g.ny, z = rr / g.ny;
-        const int ay = image_of(y, g.ny, g.bc), az = image_of(z, g.nz, g.bc);
-        const int64_t a0 = sg.at(0, y, z);
-        for (int x = threadIdx.x; x < g.nx; x += kNT) {
-            const float eS = s.eS[a0 + x], eL = s.eL[a0 + x], c = s.c[a0 + x];
-            m += (double)c;
-            const float s2 = eS * eS, l2 = eL * eL;
+    Mass<float> m;
+    uint4 *out = reinterpret_cast<uint4 *>(act);
+    const int lane = threadIdx.x & 31;
+    const int per = g.nx / kTileX;
+    const int nw = g.nz * g.ny * per;
+    for (int w = blockIdx.x * (kNT / 32) + (threadIdx.x >> 5); w < nw; w += gridDim.x * (kNT / 32)) {
+        const int row = w / per, x0 = (w - row * per) * kTileX + lane;
+        const int z = row / g.ny, y = row - z * g.ny;
+        const int64_t a0 = sg.at(x0, y, z);
+        float eS[4], eL[4], c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            eS[k] = s.eS[a0 + 32 * k];
+            eL[k] = s.eL[a0 + 32 * k];
+            c[k] = s.c[a0 + 32 * k];
+        }
+        m.add(V2<float>(c[0], c[1]));
+        m.add(V2<float>(c[2], c[3]));
+        uint4 v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float s2 = eS[k] * eS[k], l2 = eL[k] * eL[k];
             const float h = s2 / fmaxf(s2 + l2, 1e-30f);
-            const float f2 = (c - (cL + (cS - cL) * h)) * kc;
+            const float f2 = (c[k] - (cL + (cS - cL) * h)) * kc;
             // what BF16 drops of etaS and etaL, scaled into range: with
             // channels 0-1 the network sees both fields to ~16 bits
-            const uint32_t hi = pack2(eS, eL);
-            const float rS = (eS - __uint_as_float(hi << 16)) * 256.0f;
-            const float rL = (eL - __uint_as_float(hi & 0xFFFF0000u)) * 256.0f;
-            const uint4 v = make_uint4(hi, pack2(f2, rS), pack2(rL, 0.f), 0u);
-            const int ax = image_of(x, g.nx, g.bc);
-            for (int k = 0; k < 8; ++k) {
-                const int xx = (k & 1) ? ax : x, yy = (k & 2) ? ay : y, zz = (k & 4) ? az : z;
-                if (xx == kNone || yy == kNone || zz == kNone) continue;
-                *reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(act) + g.p(xx, yy, zz) * 16) = v;
+            const uint32_t hi = pack2(eS[k], eL[k]);
+            const float rS = (eS[k] - __uint_as_float(hi << 16)) * 256.0f;
+            const float rL = (eL[k] - __uint_as_float(hi & 0xFFFF0000u)) * 256.0f;
+            v[k] = make_uint4(hi, pack2(f2, rS), pack2(rL, 0.f), 0u);
+        }
+        const int ay = image_of(y, g.ny, g.bc), az = image_of(z, g.nz, g.bc);
+        for (int q = 0; q < 4; ++q) {
+            const int yy = (q & 1) ? ay : y, zz = (q & 2) ? az : z;
+            if (yy == kNone || zz == kNone) continue;
+            uint4 *o = out + g.p(0, yy, zz);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int x = x0 + 32 * k;
+                o[x] = v[k];
+                const int ax = image_of(x, g.nx, g.bc);
+                if (ax != kNone) o[ax] = v[k];
             }
         }
     }
-    block_sum_to(m, mass_part + blockIdx.x);
-}
-
-// FP64 per-CTA sums of c over the interior, one block per x row
-__global__ void __launch_bounds__(kNT) csum_kernel(Geom sg, const float *c, double *partials) {
-    double m = 0;
-    const int nrows = sg.ny * sg.nz;
-    for (int rr = blockIdx.x; rr < nrows; rr += gridDim.x) {
-        const float *row = c + sg.at(0, rr % sg.ny, rr / sg.ny);
-        for (int x = threadIdx.x; x < sg.nx; x += kNT) m += (double)row[x];
-    }
-    block_sum_to(m, partials + blockIdx.x);
+    block_sum_to(m.get(), mass_part + blockIdx.x);
 }
 
 // The projection moves sum(c) by R = round((target - sum) / 2^-24) units of
 // 2^-24: every cell by `base` units and `rem` cells by one more, where
-// base = floor(R / n), rem = R - base n in [0, n); the cells taking the
-// extra unit are i_k = ceil((k+1) n / rem) - 1, k < rem (evenly spread: the
-// cells where floor((i+1) rem / n) steps up).
+// base = floor(R / n), rem = R - base n in [0, n); the extra unit goes to
+// the cells i where floor(i rem / n) steps up, (i rem mod n) + rem >= n,
+// evenly spread.
 struct MassPlan {
     double target, sum;
+};
+
+struct Shift {
     long long base, rem;
 };
 
-__global__ void plan_kernel(MassPlan *mp, long long n) {
-    const double d = (mp->target - mp->sum) * 16777216.0;   // in units of 2^-24
+__device__ __forceinline__ Shift shift_of(const MassPlan &mp, long long n) {
+    const double d = (mp.target - mp.sum) * 16777216.0;     // in units of 2^-24
     long long R = 0;
     if (fabs(d) < 4.0e18) R = llrint(d);                     // non-finite or absurd: leave c alone
-    long long base = R / n, rem = R % n;
-    if (rem < 0) {
-        rem += n;
-        base -= 1;
+    Shift s{R / n, R % n};
+    if (s.rem < 0) {
+        s.rem += n;
+        s.base -= 1;
     }
-    mp->base = base;
-    mp->rem = rem;
+    return s;
 }
 
-__device__ __forceinline__ void put_c(const Geom &sg, float *c, int x, int y, int z, double add) {
-    const int64_t a = sg.at(x, y, z);
-    const float v = (float)((double)c[a] + add);
-    c[a] = v;
-    const int ax = image_of(x, sg.nx, sg.bc), ay = image_of(y, sg.ny, sg.bc), az = image_of(z, sg.nz, sg.bc);
-    if (ax != kNone) c[sg.at(ax, y, z)] = v;
-    if (ay != kNone) c[sg.at(x, ay, z)] = v;
-    if (az != kNone) c[sg.at(x, y, az)] = v;
+constexpr float kUnit = 5.9604644775390625e-08f;             // 2^-24
+
+// (a call, so that its FP64 operations are not predicated into the loop: at
+// 1/64 of the FP32 rate they cost the same whether they take effect or not)
+__device__ __noinline__ float add_wide(float v, long long base) {
+    return (float)((double)v + (double)base * (double)kUnit);
 }
 
-__global__ void __launch_bounds__(kNT) dense_kernel(Geom sg, float *c, const MassPlan *mp) {
-    const long long base = mp->base;
-    if (base == 0) return;
-    const double add = (double)base * 5.9604644775390625e-08;
-    const int nrows = sg.ny * sg.nz;
-    for (int rr = blockIdx.x; rr < nrows; rr += gridDim.x) {
-        const int y = rr % sg.ny, z = rr / sg.ny;
-        for (int x = threadIdx.x; x < sg.nx; x += kNT) put_c(sg, c, x, y, z, add);
+// One pass over the rows of c, a warp per row and four cells per lane:
+// APPLY adds each cell its `base` units of 2^-24 and then, rounded by itself,
+// the extra one (both exact in FP32 up to 2^24 units), SUM leaves the per-CTA FP64 sums
+// of the resulting c, three floats per thread (more than an FP64 running sum
+// keeps).  Bound by memory, mostly the L2, which holds the 67 MB of c at
+// 256^3: 41 us with both, 6 us adding few units.  A pass of its own for the
+// sum (79 us: an FP64 conversion and addition per cell), one over all cells
+// for `base` (21 us) and one scattered over `rem` cells (58 us) did the same
+// before.  Products of 64 bits: rows x rem stays below 2^63 for any domain
+// that fits in memory.  N holds a cell's i rem mod n plus rem: 32 bits below
+// 2^31 cells.
+template <typename N, bool APPLY, bool SUM>
+__global__ void __launch_bounds__(kNT) mass_kernel(Geom sg, float *c, const MassPlan *mp, double *partials) {
+    __shared__ Shift sh;
+    const long long n = (long long)sg.nx * sg.ny * sg.nz;
+    Shift s{0, 0};
+    if (APPLY) {
+        if (threadIdx.x == 0) sh = shift_of(*mp, n);
+        __syncthreads();
+        s = sh;
+        if (!SUM && s.base == 0 && s.rem == 0) return;
     }
-}
-
-__global__ void __launch_bounds__(kNT) sparse_kernel(Geom sg, float *c, const MassPlan *mp, long long n) {
-    const long long rem = mp->rem;
-    for (long long k = blockIdx.x * (long long)kNT + threadIdx.x; k < rem; k += (long long)gridDim.x * kNT) {
-        const long long i = ((k + 1) * n + rem - 1) / rem - 1;
-        const int x = (int)(i % sg.nx), y = (int)((i / sg.nx) % sg.ny), z = (int)(i / ((long long)sg.nx * sg.ny));
-        put_c(sg, c, x, y, z, 5.9604644775390625e-08);
+    const bool narrow = s.base >= -(1 << 24) && s.base <= (1 << 24);
+    const float add = (float)s.base * kUnit;
+    const int lane = threadIdx.x & 31, nwarps = gridDim.x * (kNT / 32);
+    const int nrows = sg.ny * sg.nz, row0 = blockIdx.x * (kNT / 32) + (threadIdx.x >> 5);
+    // i rem mod n of the thread's next row, kept by additions, and its
+    // advances: the next row's, 128 cells'
+    const N nn = (N)n, rem = (N)s.rem;
+    auto mod_add = [&](N &u, N d) {
+        u += d;
+        const bool over = u >= nn;
+        if (over) u -= nn;
+        return over;
+    };
+    N trow = 0, rrow = 0, r128 = 0;
+    if (APPLY) {
+        const long long per_row = sg.nx * s.rem % n;
+        trow = (N)(row0 * per_row % n);
+        mod_add(trow, (N)(4 * lane * s.rem % n));
+        rrow = (N)(nwarps * per_row % n);
+        r128 = (N)(128 * s.rem % n);
     }
+    Mass<float> m;
+    for (int row = row0; row < nrows; row += nwarps) {
+        const int z = row / sg.ny, y = row - z * sg.ny;
+        const int64_t a0 = sg.at(0, y, z);
+        const int ay = image_of(y, sg.ny, sg.bc), az = image_of(z, sg.nz, sg.bc);
+        N t = trow;
+        mod_add(trow, rrow);
+        for (int x = 4 * lane; x < sg.nx; x += 128) {
+            unsigned extra = 0;                              // bit k: cell x + k takes one unit more
+            if (APPLY) {
+                N u = t;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) extra |= (unsigned)mod_add(u, rem) << k;
+                mod_add(t, r128);
+                if (!SUM && s.base == 0 && !extra) continue;
+            }
+            // rows start on 32 bytes and are padded to 8 cells past the last
+            // halo cell: the load stays inside the row
+            const float4 q = *reinterpret_cast<const float4 *>(c + a0 + x);
+            float v[4] = {q.x, q.y, q.z, q.w};
+            const int nk = min(4, sg.nx - x);
+            if (APPLY) {
+                if (narrow) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[k] += add;
+                } else {
+                    for (int k = 0; k < 4; ++k) v[k] = add_wide(v[k], s.base);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) v[k] += extra >> k & 1 ? kUnit : 0.f;
+                auto put = [&](int64_t a) {
+                    if (nk == 4) {
+                        *reinterpret_cast<float4 *>(c + a) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+                        for (int k = 0; k < nk; ++k) c[a + k] = v[k];
+                    }
+                };
+                put(a0 + x);
+                if (ay != kNone) put(sg.at(x, ay, z));
+                if (az != kNone) put(sg.at(x, y, az));
+                if (x == 0) c[sg.at(image_of(0, sg.nx, sg.bc), y, z)] = v[0];
+                if (x + nk == sg.nx && sg.nx > 1) c[sg.at(image_of(sg.nx - 1, sg.nx, sg.bc), y, z)] = v[nk - 1];
+            }
+            if (SUM) {
+                m.add(V2<float>(v[0], nk > 1 ? v[1] : 0.f));
+                m.add(V2<float>(nk > 2 ? v[2] : 0.f, nk > 3 ? v[3] : 0.f));
+            }
+        }
+    }
+    if (SUM) block_sum_to(m.get(), partials + blockIdx.x);
 }
 
 // out[i] = sum_b part[b * stride + i] for i < n, and with `loss` set also
@@ -413,7 +494,10 @@ int run_conv(ppf_surrogate *s, ppf_ctx *c, int ci, int co, int epi, const ConvAr
 
 MassPlan *plan_of(ppf_ctx *c) { return reinterpret_cast<MassPlan *>(c->dres + 16); }
 
-int row_blocks(const ppf_ctx *c) { return (int)std::min<int64_t>((int64_t)c->ny * c->nz, 8LL * c->num_sms); }
+// blocks of the kernels that take a warp per row
+int row_blocks(const ppf_ctx *c) {
+    return (int)std::min<int64_t>(((int64_t)c->ny * c->nz + kNT / 32 - 1) / (kNT / 32), 8LL * c->num_sms);
+}
 
 // features of the current state; the mass before the call goes to the plan's target
 int features(ppf_surrogate *s, ppf_ctx *c) {
@@ -514,33 +598,31 @@ int pack_all(ppf_surrogate *s, cudaStream_t st) {
     return PPF_OK;
 }
 
-int mass_sum(ppf_ctx *c, double *out) {
+// move sum(c) onto the plan's target; `have_sum`: the plan's sum is already
+// that of the current state
+template <typename N>
+int project_n(ppf_ctx *c, bool have_sum) {
+    MassPlan *mp = plan_of(c);
+    float *cc = (float *)c->fld[c->cur_c][2];
     const int nb = row_blocks(c);
     int rc = ensure_partials(c, nb);
     if (rc) return rc;
-    csum_kernel<<<nb, kNT, 0, c->stream>>>(c->g, (const float *)c->fld[c->cur_c][2], c->partials);
+    if (!have_sum) {
+        mass_kernel<N, false, true><<<nb, kNT, 0, c->stream>>>(c->g, cc, mp, c->partials);
+        SCU(cudaGetLastError());
+        SCU(launch_final_sum(c->partials, nb, 1, 1, &mp->sum, c->stream));
+    }
+    mass_kernel<N, true, true><<<nb, kNT, 0, c->stream>>>(c->g, cc, mp, c->partials);
     SCU(cudaGetLastError());
-    SCU(launch_final_sum(c->partials, nb, 1, 1, out, c->stream));
+    SCU(launch_final_sum(c->partials, nb, 1, 1, &mp->sum, c->stream));
+    mass_kernel<N, true, false><<<nb, kNT, 0, c->stream>>>(c->g, cc, mp, nullptr);
+    SCU(cudaGetLastError());
     return PPF_OK;
 }
 
-// move sum(c) onto the plan's target; `have_sum`: the plan's sum is already
-// that of the current state
 int project(ppf_ctx *c, bool have_sum) {
-    MassPlan *mp = plan_of(c);
     const long long n = (long long)c->nz * c->ny * c->nx;
-    float *cc = (float *)c->fld[c->cur_c][2];
-    for (int pass = 0; pass < 2; ++pass) {
-        if (pass > 0 || !have_sum) {
-            int rc = mass_sum(c, &mp->sum);
-            if (rc) return rc;
-        }
-        plan_kernel<<<1, 1, 0, c->stream>>>(mp, n);
-        dense_kernel<<<row_blocks(c), kNT, 0, c->stream>>>(c->g, cc, mp);
-        sparse_kernel<<<4 * c->num_sms, kNT, 0, c->stream>>>(c->g, cc, mp, n);
-        SCU(cudaGetLastError());
-    }
-    return PPF_OK;
+    return n < (1LL << 31) ? project_n<unsigned>(c, have_sum) : project_n<unsigned long long>(c, have_sum);
 }
 
 }  // namespace
