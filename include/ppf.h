@@ -175,10 +175,14 @@ typedef struct ppf_particle_stats {
 } ppf_particle_stats;
 
 /* `volumes` (may be NULL) receives up to `capacity` particle volumes in
- * cells, in no particular order; *nvolumes (may be NULL) the particle count.
- * Device scratch of about 8 bytes per cell is allocated on the first call. */
+ * cells, in ascending order; *nvolumes (may be NULL) the particle count.
+ * Device scratch of about 6 bytes per cell is allocated on the first call. */
 int ppf_particles(ppf_ctx *ctx, double threshold, ppf_particle_stats *out, int64_t *volumes, int64_t capacity,
                   int64_t *nvolumes);
+/* The first n volumes of the last ppf_particles call on this context, which
+ * keeps up to its `capacity` of them (also when its `volumes` is NULL, so that
+ * the array can be made once their number is known). */
+int ppf_particle_volumes(ppf_ctx *ctx, int64_t *volumes, int64_t n);
 
 /* Launch choices of the fused step kernel.  No counterpart in the
  * reference (whose only tuning is the no-op cache blocking of

@@ -28,8 +28,8 @@ EXPORTS = (
     "ppf_params_default", "ppf_params_derive", "ppf_create", "ppf_destroy", "ppf_get_dims", "ppf_set_stream",
     "ppf_upload", "ppf_download", "ppf_upload_device", "ppf_download_device", "ppf_step", "ppf_step_c_only",
     "ppf_reduce", "ppf_sync", "ppf_set_wait_limit", "ppf_debug_inject", "ppf_get_tune", "ppf_set_tune",
-    "ppf_autotune", "ppf_observe_noalloc", "ppf_particles", "ppf_ensemble_create", "ppf_ensemble_destroy",
-    "ppf_ensemble_domain", "ppf_ensemble_upload", "ppf_ensemble_download", "ppf_ensemble_upload_all",
+    "ppf_autotune", "ppf_observe_noalloc", "ppf_particles", "ppf_particle_volumes", "ppf_ensemble_create",
+    "ppf_ensemble_destroy", "ppf_ensemble_domain", "ppf_ensemble_upload", "ppf_ensemble_download", "ppf_ensemble_upload_all",
     "ppf_ensemble_download_all", "ppf_ensemble_step",
     "ppf_ensemble_reduce", "ppf_ensemble_sync", "ppf_ensemble_get_tune", "ppf_ensemble_set_tune",
     "ppf_ensemble_autotune", "ppf_slabs_plan", "ppf_slabs_create", "ppf_slabs_destroy", "ppf_slabs_upload",
@@ -135,6 +135,7 @@ def lib() -> ctypes.CDLL:
         L.ppf_get_tune.argtypes = [ctypes.c_void_p, ctypes.POINTER(Tune)]
         L.ppf_set_tune.argtypes = [ctypes.c_void_p, ctypes.POINTER(Tune)]
         L.ppf_autotune.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(Tune)]
+        L.ppf_particle_volumes.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64]
         L.ppf_particles.argtypes = [ctypes.c_void_p, ctypes.c_double, ctypes.POINTER(ParticleStats),
                                     ctypes.c_void_p, ctypes.c_int64, ctypes.POINTER(ctypes.c_int64)]
         L.ppf_get_dims.argtypes = [ctypes.c_void_p] + [ctypes.POINTER(ctypes.c_int)] * 3
@@ -305,11 +306,10 @@ class Simulation:
         n = ctypes.c_int64(0)
         if volumes:
             cap = int(np.prod(self.shape)) // 2 + 1
-            buf = np.zeros(cap, dtype=np.int64)
-            _check(lib().ppf_particles(self._h, float(threshold), ctypes.byref(st), buf.ctypes.data, cap,
-                                       ctypes.byref(n)))
+            _check(lib().ppf_particles(self._h, float(threshold), ctypes.byref(st), None, cap, ctypes.byref(n)))
             d = st.as_dict()
-            d["volumes"] = np.sort(buf[:min(n.value, cap)])
+            d["volumes"] = np.empty(min(n.value, cap), dtype=np.int64)
+            _check(lib().ppf_particle_volumes(self._h, d["volumes"].ctypes.data, len(d["volumes"])))
             return d
         _check(lib().ppf_particles(self._h, float(threshold), ctypes.byref(st), None, 0, ctypes.byref(n)))
         return st.as_dict()

@@ -229,8 +229,7 @@ extern "C" int ppf_destroy(ppf_ctx *c) {
     if (c->staging) cudaFree(c->staging);
     if (c->partials) cudaFree(c->partials);
     if (c->dres) cudaFree(c->dres);
-    if (c->plab) cudaFree(c->plab);
-    if (c->pvol) cudaFree(c->pvol);
+    if (c->pscratch) cudaFree(c->pscratch);
     if (c->plist) cudaFree(c->plist);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
@@ -705,35 +704,35 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     if (volumes && capacity < 0) return seterr(PPF_EINVAL, "negative capacity");
     const int64_t cells = (int64_t)c->nz * c->ny * c->nx;
     if (cells >= ((int64_t)1 << 31)) return seterr(PPF_EINVAL, "particle labels hold at most 2^31-1 cells");
-    // labels, and behind them the bit of every cell
-    if (!c->plab) CU(cudaMalloc(&c->plab, ((size_t)cells + (size_t)particle_words(c->g)) * sizeof(int)));
-    if (!c->pvol) CU(cudaMalloc(&c->pvol, (size_t)cells * sizeof(int)));
-    int64_t cap = volumes ? capacity : 0;
-    if (cap > 0 && cap > c->plist_cap) {
+    ParticleScratch ps = particle_scratch(c->g, c->pscratch);
+    if (!c->pscratch) {
+        CU(cudaMalloc(&c->pscratch, (size_t)ps.ints * sizeof(int)));
+        ps = particle_scratch(c->g, c->pscratch);
+    }
+    int64_t cap = capacity > 0 ? capacity : 0;
+    c->pkept = 0;
+    if (cap > ps.nodes) cap = ps.nodes;
+    if (cap > c->plist_cap) {
         if (c->plist) cudaFree(c->plist);
         c->plist = nullptr;
         c->plist_cap = 0;
-        CU(cudaMalloc(&c->plist, (size_t)cap * sizeof(int64_t) + 64));
+        CU(cudaMalloc(&c->plist, (size_t)cap * 2 * sizeof(int)));
         c->plist_cap = cap;
     }
     int nb = (int)((cells + 255) / 256);
     if (nb > 8 * c->num_sms) nb = 8 * c->num_sms;
-    int rc = ensure_partials(c, 5 * nb + 8);
+    int rc = ensure_partials(c, 5 * nb + 3 * c->num_sms);
     if (rc) return rc;
-    unsigned long long *nlist = c->plist ? (unsigned long long *)(c->plist + c->plist_cap) : nullptr;
     double *dout = c->dres + 8;
+    int *const vols = cap > 0 ? c->plist : nullptr;
     if (c->prec == PPF_F32)
-        CU(launch_particles<float>(c->g, (const float *)c->fld[c->cur_eta][0], threshold, c->plab, c->pvol,
-                                   (unsigned *)c->plab + cells, c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist, c->derr,
-                                   c->stream));
+        CU(launch_particles<float>(c->g, (const float *)c->fld[c->cur_eta][0], threshold, ps, c->partials, nb, c->num_sms,
+                                   c->p.dx, dout, vols, cap, c->derr, c->stream));
     else
-        CU(launch_particles<double>(c->g, (const double *)c->fld[c->cur_eta][0], threshold, c->plab, c->pvol,
-                                    (unsigned *)c->plab + cells, c->partials, nb, c->p.dx, dout, cap > 0 ? c->plist : nullptr, cap, nlist,
-                                    c->derr, c->stream));
+        CU(launch_particles<double>(c->g, (const double *)c->fld[c->cur_eta][0], threshold, ps, c->partials, nb,
+                                    c->num_sms, c->p.dx, dout, vols, cap, c->derr, c->stream));
     double h[5];
-    unsigned long long hn = 0;
     CU(cudaMemcpyAsync(h, dout, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    if (cap > 0) CU(cudaMemcpyAsync(&hn, nlist, sizeof hn, cudaMemcpyDeviceToHost, c->stream));
     rc = check_device_error(c);
     if (rc) return rc;
     const double dx = c->p.dx;
@@ -743,10 +742,21 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     out->largest_volume = h[3] * dx * dx * dx;
     out->interface_area = h[4] * dx * dx;
     if (nvolumes) *nvolumes = (int64_t)h[0];
-    if (cap > 0) {
-        const int64_t m = (int64_t)hn < cap ? (int64_t)hn : cap;
-        CU(cudaMemcpy(volumes, c->plist, (size_t)m * sizeof(int64_t), cudaMemcpyDeviceToHost));
+    const int64_t m = (int64_t)h[0] < cap ? (int64_t)h[0] : cap;
+    if (m > 0) {
+        CU(launch_sort_volumes(c->plist, c->plist + cap, m, (int64_t)h[3], ps, &c->psorted, c->stream));
+        c->pkept = m;
+        if (volumes) return ppf_particle_volumes(c, volumes, m);
     }
+    return PPF_OK;
+}
+
+extern "C" int ppf_particle_volumes(ppf_ctx *c, int64_t *volumes, int64_t n) {
+    if (!c || !volumes) return seterr(PPF_EINVAL, "null argument");
+    if (n < 0 || n > c->pkept) return seterr(PPF_EINVAL, "the last particle analysis kept %lld volumes", (long long)c->pkept);
+    if (n == 0) return PPF_OK;
+    CU(cudaMemcpyAsync(volumes, c->psorted, (size_t)n * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaStreamSynchronize(c->stream));
     return PPF_OK;
 }
 

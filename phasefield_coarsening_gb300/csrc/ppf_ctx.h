@@ -34,9 +34,11 @@ struct ppf_ctx {
     ppf::StepTune tune;        // launch choices of the fused step (grid, z chunk, unroll)
     unsigned long long wait_limit_ns;
     int inject;           // test hook: PPF_INJECT_*
-    int *plab, *pvol;     // particle labels / volumes (allocated on first use)
-    int64_t *plist;       // particle volume list (device), plist_cap entries
+    int *pscratch;        // particle analysis (allocated on first use)
+    int *plist;           // particle volumes (device), twice plist_cap entries
     int64_t plist_cap;
+    int64_t *psorted;     // the last analysis' first pkept volumes in order (in pscratch)
+    int64_t pkept;
     int64_t steps;
     int uploaded;
     ppf::Coef<float> kf;

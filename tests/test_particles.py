@@ -138,3 +138,27 @@ def test_gpu_particles_of_a_spiral(bc):
         o = oracle.particles(f, bc=bc)
         assert g["count"] == o["count"] and np.array_equal(g["volumes"], o["volumes"])
         assert g["interface_area"] == o["interface_area"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(19, 35, 300), (40, 33, 40), (70, 18, 20), (8, 16, 128), (9, 17, 129)])
+@pytest.mark.parametrize("bc", [0, 1])
+@pytest.mark.parametrize("fill", [0.2, 0.31, 0.5])
+def test_gpu_particles_over_bricks(shape, bc, fill):
+    """Domains of one and of several labelling bricks in every direction, whole
+    and ragged; fewer volumes asked for than there are particles."""
+    import ctypes
+    r = np.random.default_rng(int(100 * fill) + sum(shape) + bc)
+    e = np.where(r.random(shape) < fill, 0.9, 0.1)
+    o = oracle.particles(e, bc=bc)
+    with ppf.Simulation(shape, bc=bc) as s:
+        s.upload(e, 1.0 - e, np.full(shape, 0.7))
+        g = s.particles(volumes=True)
+        few = max(1, o["count"] // 3)
+        some = np.full(few + 1, -1, np.int64)
+        st, n = ppf.ParticleStats(), ctypes.c_int64(0)
+        assert ppf.lib().ppf_particles(s._h, 0.5, ctypes.byref(st), some.ctypes.data, few, ctypes.byref(n)) == 0
+    assert g["count"] == o["count"] and np.array_equal(g["volumes"], o["volumes"])
+    assert g["interface_area"] == o["interface_area"] and g["solid_volume"] == o["solid_volume"]
+    assert n.value == o["count"] and some[few] == -1
+    assert np.all(np.diff(some[:few]) >= 0) and np.all(np.isin(some[:few], o["volumes"]))
