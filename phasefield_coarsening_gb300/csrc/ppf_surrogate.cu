@@ -273,72 +273,97 @@ __global__ void __launch_bounds__(kNT) mass_kernel(Geom sg, float *c, const Mass
     if (SUM) block_sum_to(m.get(), partials + blockIdx.x);
 }
 
-// out[i] = sum_b part[b * stride + i] for i < n, and with `loss` set also
-// *loss = sum_b part[b * stride + li], in a fixed order.  A block takes 32
-// values, its eight warps an eighth of the partial sums each: independent
-// loads in flight instead of one thread's chain (21 us for 152 partials of
-// 27 x 32 x 32 weights), and sums carried with their rounding errors in float
-// (Knuth's TwoSum, about 48 bits) instead of FP64, whose conversions and
-// additions alone would take 14 us.
-__global__ void __launch_bounds__(kNT) reduce_kernel(const float *part, int nb, int stride, int n, float *out, int li,
-                                                     double *loss) {
+// The partial sums of a training step: per job, out[i] = sum_b
+// part[b * stride + i] for i < n, in a fixed order; job 0 also has the loss
+// behind its n values.  Blocks first[j] .. first[j + 1] - 1 have job j.
+constexpr int kJobs = 2 * kLayers;
+struct ReduceJobs {
+    const float *part[kJobs];
+    float *out[kJobs];
+    int nb[kJobs], stride[kJobs], n[kJobs], first[kJobs + 1];
+    double *loss;
+};
+
+// A block takes 32 values, its eight warps an eighth of the partial sums each:
+// independent loads in flight instead of one thread's chain (21 us for 152
+// partials of 27 x 32 x 32 weights), and sums carried with their rounding
+// errors in float (Knuth's TwoSum, about 48 bits) instead of FP64, whose
+// conversions and additions alone would take 14 us.  All jobs of a step in one
+// launch: 24 us for the 84 MB of a width-32 network (62 us in twelve launches).
+__global__ void __launch_bounds__(kNT) reduce_kernel(const __grid_constant__ ReduceJobs q) {
     __shared__ float2 red[kNT / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    auto add = [](float2 &a, float x) {
-        const float s = a.x + x, bp = s - a.x;
-        a.y += (a.x - (s - bp)) + (x - bp);
-        a.x = s;
-    };
+    int j = 0;
+    while ((int)blockIdx.x >= q.first[j + 1]) ++j;
+    const int nb = q.nb[j], n = q.n[j];
+    const int nv = n + (j == 0 ? 1 : 0);
     const int b0 = nb * warp / (kNT / 32), b1 = nb * (warp + 1) / (kNT / 32);
-    const int nv = n + (loss ? 1 : 0);
-    for (int i0 = blockIdx.x * 32; i0 < nv; i0 += gridDim.x * 32) {
-        const int i = i0 + lane, col = i < n ? i : li;
-        float2 s = make_float2(0.f, 0.f);
-        if (i < nv) {
+    const int i = ((int)blockIdx.x - q.first[j]) * 32 + lane;
+    const float *part = q.part[j] + i;
+    float2 s = make_float2(0.f, 0.f);
+    auto add = [](float2 &a, float x) {
+        float e;
+        a.x = two_sum1(a.x, x, e);
+        a.y += e;
+    };
+    if (i < nv) {
 #pragma unroll 8
-            for (int b = b0; b < b1; ++b) add(s, part[(int64_t)b * stride + col]);
+        for (int b = b0; b < b1; ++b) add(s, part[(int64_t)b * q.stride[j]]);
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < nv) {
+        for (int w = 1; w < kNT / 32; ++w) {
+            const float2 o = red[w][lane];
+            add(s, o.x);
+            s.y += o.y;
         }
-        red[warp][lane] = s;
-        __syncthreads();
-        if (warp == 0 && i < nv) {
-            for (int w = 1; w < kNT / 32; ++w) {
-                const float2 o = red[w][lane];
-                add(s, o.x);
-                s.y += o.y;
-            }
-            if (i < n) out[i] = s.x + s.y;
-            else *loss = (double)s.x + (double)s.y;
-        }
-        __syncthreads();
+        if (i < n) q.out[j][i] = s.x + s.y;
+        else *q.loss = (double)s.x + (double)s.y;
     }
 }
 
-__global__ void __launch_bounds__(kNT) adam_kernel(int64_t n, float *p, const float *g, float *m, float *v, float lr,
-                                                   float b1, float b2, float eps, float c1, float c2) {
-    for (int64_t i = blockIdx.x * (int64_t)kNT + threadIdx.x; i < n; i += (int64_t)gridDim.x * kNT) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    }
-}
+// Where a layer's weights stand among the parameters, and their BF16 images.
+struct PackTable {
+    int64_t n;                   // parameters
+    int64_t woff[kLayers];
+    int ci[kLayers], co[kLayers];
+    uint16_t *wf[kLayers], *wb[kLayers];
+};
 
 // W[27][co][ci] (FP32, tap = 9 dz + 3 dy + dx over 0..2) -> the BF16
 // B-operand images of the convolution kernel, [dz][dx][ci/8][dy][co][8]
 // (one MMA's N = 3 co rows are the three dy taps), forward and for the
 // input-gradient convolution (taps reversed, ci and co swapped).
-__global__ void __launch_bounds__(kNT) pack_kernel(const float *W, int ci, int co, uint16_t *wf, uint16_t *wb) {
-    const int n = 27 * ci * co;
-    for (int i = blockIdx.x * kNT + threadIdx.x; i < n; i += gridDim.x * kNT) {
-        const int c_in = i % ci, c_out = (i / ci) % co, tap = i / (ci * co);
-        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-        const __nv_bfloat16 h = __float2bfloat16_rn(W[i]);
-        const uint16_t u = *reinterpret_cast<const uint16_t *>(&h);
-        wf[((((int64_t)(dz * 3 + dx) * (ci / 8) + c_in / 8) * 3 + dy) * co + c_out) * 8 + (c_in & 7)] = u;
-        const int rz = 2 - dz, ry = 2 - dy, rx = 2 - dx;
-        wb[((((int64_t)(rz * 3 + rx) * (co / 8) + c_out / 8) * 3 + ry) * ci + c_in) * 8 + (c_out & 7)] = u;
+__device__ __forceinline__ void pack_weight(const PackTable &t, int64_t p, float w) {
+    int l = kLayers - 1;
+    while (p < t.woff[l]) --l;
+    const int i = (int)(p - t.woff[l]), ci = t.ci[l], co = t.co[l];
+    if (i >= 27 * ci * co) return;                           // a bias
+    const int c_in = i % ci, c_out = (i / ci) % co, tap = i / (ci * co);
+    const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
+    const __nv_bfloat16 h = __float2bfloat16_rn(w);
+    const uint16_t u = *reinterpret_cast<const uint16_t *>(&h);
+    t.wf[l][((((int64_t)(dz * 3 + dx) * (ci / 8) + c_in / 8) * 3 + dy) * co + c_out) * 8 + (c_in & 7)] = u;
+    const int rz = 2 - dz, ry = 2 - dy, rx = 2 - dx;
+    t.wb[l][((((int64_t)(rz * 3 + rx) * (co / 8) + c_out / 8) * 3 + ry) * ci + c_in) * 8 + (c_out & 7)] = u;
+}
+
+__global__ void __launch_bounds__(kNT) pack_kernel(const __grid_constant__ PackTable t, const float *p) {
+    for (int64_t i = blockIdx.x * (int64_t)kNT + threadIdx.x; i < t.n; i += (int64_t)gridDim.x * kNT) pack_weight(t, i, p[i]);
+}
+
+__global__ void __launch_bounds__(kNT) adam_kernel(const __grid_constant__ PackTable t, float *p, const float *g, float *m,
+                                                   float *v, float lr, float b1, float b2, float eps, float c1, float c2) {
+    for (int64_t i = blockIdx.x * (int64_t)kNT + threadIdx.x; i < t.n; i += (int64_t)gridDim.x * kNT) {
+        const float gi = g[i];
+        const float mi = b1 * m[i] + (1.f - b1) * gi;
+        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
+        m[i] = mi;
+        v[i] = vi;
+        const float w = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        p[i] = w;
+        pack_weight(t, i, w);
     }
 }
 
@@ -358,6 +383,8 @@ struct ppf_surrogate {
     NNGeom g{};
     uint16_t *feat = nullptr, *act[5] = {}, *zp[5] = {}, *g16 = nullptr, *gw[2] = {};
     bool train_ready = false;    // g16, gw, zp allocated for the current shape
+    // per-CTA sums of all layers (training): weight gradients, bias gradients
+    // and the loss, summed up in one launch at the end of the backward pass
     float *wpart = nullptr, *bpart = nullptr;
     double *mpart = nullptr;     // per-CTA sums of c after a call (output layer)
     double *dscal = nullptr;     // [0] loss
@@ -450,6 +477,8 @@ int ensure_ws(ppf_surrogate *s, ppf_ctx *c, bool train) {
             if (!rc) rc = alloc_zero((void **)&p, act_bytes(s->g, s->W), c->stream);
         for (auto &p : s->zp)
             if (!rc) rc = alloc_zero((void **)&p, act_bytes(s->g, s->W), c->stream);
+        if (!rc && !s->wpart && cudaMalloc(&s->wpart, (size_t)s->wgrad_grid * s->nparams * sizeof(float)) != cudaSuccess)
+            rc = serr(PPF_ENOMEM, "no memory for the weight gradients' partial sums");
         if (rc) {
             cudaDeviceSynchronize();
             free_train(s);
@@ -524,26 +553,45 @@ int forward_hidden(ppf_surrogate *s, ppf_ctx *c, bool train) {
     return PPF_OK;
 }
 
-int reduce_into(ppf_surrogate *s, ppf_ctx *c, const float *part, int nb, int stride, int n, float *out, int li = 0,
-                double *loss = nullptr) {
-    const int blocks = std::min((n + 32) / 32, 8 * s->num_sms);
-    reduce_kernel<<<blocks, kNT, 0, c->stream>>>(part, nb, stride, n, out, li, loss);
-    SCU(cudaGetLastError());
-    return PPF_OK;
-}
+// per-CTA sums of a layer's weight gradients, and of its bias gradients (CO + 1 per CTA)
+float *wpart_of(ppf_surrogate *s, int layer) { return s->wpart + s->wgrad_grid * s->woff[layer]; }
+float *bpart_of(ppf_surrogate *s, int layer) { return s->bpart + (size_t)layer * 2 * s->num_sms * 33; }
 
 int wgrad(ppf_surrogate *s, ppf_ctx *c, int layer, const uint16_t *x, const uint16_t *dz) {
     WgradArgs w{};
     w.g = s->g;
     w.x = x;
     w.dz = dz;
-    w.partials = s->wpart;
+    w.partials = wpart_of(s, layer);
     w.ntiles = s->g.nz * s->g.ny * (s->g.nx / kTileX);
     w.err = c->derr;
     w.limit_ns = c->wait_limit_ns;
     SCU(launch_wgrad(s->ci[layer], s->co[layer], w, s->wgrad_grid, c->stream));
-    const int n = 27 * s->ci[layer] * s->co[layer];
-    return reduce_into(s, c, s->wpart, s->wgrad_grid, n, n, s->grads + s->woff[layer]);
+    return PPF_OK;
+}
+
+int reduce_all(ppf_surrogate *s, ppf_ctx *c, const int (&bias_grid)[kLayers]) {
+    ReduceJobs q{};
+    q.loss = s->dscal;
+    int blocks = 0, j = 0;
+    auto job = [&](const float *part, float *out, int nb, int stride, int n) {
+        q.part[j] = part;
+        q.out[j] = out;
+        q.nb[j] = nb;
+        q.stride[j] = stride;
+        q.n[j] = n;
+        q.first[j] = blocks;
+        blocks += (n + (j == 0 ? 1 : 0) + 31) / 32;
+        q.first[++j] = blocks;
+    };
+    for (int l = kLayers - 1; l >= 0; --l) job(bpart_of(s, l), s->grads + s->boff[l], bias_grid[l], s->co[l] + 1, s->co[l]);
+    for (int l = 0; l < kLayers; ++l) {
+        const int n = 27 * s->ci[l] * s->co[l];
+        job(wpart_of(s, l), s->grads + s->woff[l], s->wgrad_grid, n, n);
+    }
+    reduce_kernel<<<blocks, kNT, 0, c->stream>>>(q);
+    SCU(cudaGetLastError());
+    return PPF_OK;
 }
 
 // loss and gradients of all parameters for one (input, target) pair
@@ -556,17 +604,17 @@ int loss_grad(ppf_surrogate *s, ppf_ctx *in, ppf_ctx *tg) {
     if (in->bc != PPF_BC_PERIODIC) return serr(PPF_EINVAL, "training runs on periodic domains");
     if (tg->stream != in->stream) SCU(cudaStreamSynchronize(tg->stream));
     if ((rc = forward_hidden(s, in, true))) return rc;
+    int bias_grid[kLayers];      // CTAs that sum a layer's bias gradients
     // output layer + loss: dZ5 -> g16
     {
         ConvArgs a = conv_args(s, in, 5, s->act[4], s->wf[5]);
         a.out = s->g16;
-        a.partials = s->bpart;
+        a.partials = bpart_of(s, 5);
         a.s0 = cur_fields(in);
         Fields<const float> t = cur_fields(tg);
         a.s1 = {const_cast<float *>(t.eS), const_cast<float *>(t.eL), const_cast<float *>(t.c)};
         if ((rc = run_conv(s, in, s->ci[5], 16, EPI_LOSS, a))) return rc;
-        const int grid = s->conv_grid[s->ci[5] == 32][0];
-        if ((rc = reduce_into(s, in, s->bpart, grid, 17, 16, s->grads + s->boff[5], 16, s->dscal))) return rc;
+        bias_grid[5] = s->conv_grid[s->ci[5] == 32][0];
     }
     if ((rc = wgrad(s, in, 5, s->act[4], s->g16))) return rc;
     const uint16_t *cur = s->g16;
@@ -576,25 +624,34 @@ int loss_grad(ppf_surrogate *s, ppf_ctx *in, ppf_ctx *tg) {
         ConvArgs a = conv_args(s, in, l, cur, s->wb[l]);
         a.out = out;
         a.zlow = s->zp[l - 1];
-        a.partials = s->bpart;
+        a.partials = bpart_of(s, l - 1);
         const int ci = s->co[l], co = s->ci[l];
         if ((rc = run_conv(s, in, ci, co, EPI_DGRAD, a))) return rc;
-        if ((rc = reduce_into(s, in, s->bpart, s->conv_grid[ci == 32][co == 32], co + 1, co,
-                              s->grads + s->boff[l - 1])))
-            return rc;
+        bias_grid[l - 1] = s->conv_grid[ci == 32][co == 32];
         if ((rc = wgrad(s, in, l - 1, l - 1 == 0 ? s->feat : s->act[l - 2], out))) return rc;
         cur = out;
     }
-    return PPF_OK;
+    return reduce_all(s, in, bias_grid);
 }
 
-int pack_all(ppf_surrogate *s, cudaStream_t st) {
+PackTable pack_table(const ppf_surrogate *s) {
+    PackTable t{};
+    t.n = s->nparams;
     for (int l = 0; l < kLayers; ++l) {
-        const int n = 27 * s->ci[l] * s->co[l];
-        pack_kernel<<<(n + kNT - 1) / kNT, kNT, 0, st>>>(s->params + s->woff[l], s->ci[l], s->co[l], s->wf[l],
-                                                        s->wb[l]);
-        SCU(cudaGetLastError());
+        t.woff[l] = s->woff[l];
+        t.ci[l] = s->ci[l];
+        t.co[l] = s->co[l];
+        t.wf[l] = s->wf[l];
+        t.wb[l] = s->wb[l];
     }
+    return t;
+}
+
+int param_blocks(const ppf_surrogate *s) { return (int)std::min<int64_t>((s->nparams + kNT - 1) / kNT, 4LL * s->num_sms); }
+
+int pack_all(ppf_surrogate *s, cudaStream_t st) {
+    pack_kernel<<<param_blocks(s), kNT, 0, st>>>(pack_table(s), s->params);
+    SCU(cudaGetLastError());
     return PPF_OK;
 }
 
@@ -686,8 +743,7 @@ extern "C" int ppf_surrogate_create(const ppf_surrogate_config *cfg, ppf_surroga
     const size_t pb = (size_t)s->nparams * sizeof(float);
     bool ok = cudaMalloc(&s->params, pb) == cudaSuccess && cudaMalloc(&s->grads, pb) == cudaSuccess &&
               cudaMalloc(&s->mom1, pb) == cudaSuccess && cudaMalloc(&s->mom2, pb) == cudaSuccess &&
-              cudaMalloc(&s->wpart, (size_t)s->wgrad_grid * 27 * 32 * 32 * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&s->bpart, (size_t)2 * s->num_sms * 33 * sizeof(float)) == cudaSuccess &&
+              cudaMalloc(&s->bpart, (size_t)kLayers * 2 * s->num_sms * 33 * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&s->mpart, (size_t)2 * s->num_sms * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&s->dscal, 8 * sizeof(double)) == cudaSuccess;
     for (int l = 0; ok && l < kLayers; ++l)
@@ -780,11 +836,9 @@ extern "C" int ppf_surrogate_train_step(ppf_surrogate *s, ppf_ctx *input, ppf_ct
     s->adam_t++;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)s->adam_t), c2 = 1.f - powf(b2, (float)s->adam_t);
-    const int nb = (int)std::min<int64_t>((s->nparams + kNT - 1) / kNT, 4LL * s->num_sms);
-    adam_kernel<<<nb, kNT, 0, input->stream>>>(s->nparams, s->params, s->grads, s->mom1, s->mom2, (float)lr, b1, b2,
-                                               1e-8f, c1, c2);
+    adam_kernel<<<param_blocks(s), kNT, 0, input->stream>>>(pack_table(s), s->params, s->grads, s->mom1, s->mom2, (float)lr,
+                                                            b1, b2, 1e-8f, c1, c2);
     SCU(cudaGetLastError());
-    if ((rc = pack_all(s, input->stream))) return rc;
     if (loss) {
         SCU(cudaMemcpyAsync(loss, s->dscal, sizeof(double), cudaMemcpyDeviceToHost, input->stream));
         SCU(cudaStreamSynchronize(input->stream));
