@@ -87,6 +87,32 @@ __device__ __forceinline__ bool wait_backoff(uint32_t bar, uint32_t parity, unsi
     }
 }
 
+// Programmatic dependent launch: a convolution or weight-gradient kernel starts
+// while the CTAs of the one before finish, sets itself up, and waits here until
+// that one is complete and its results are visible.  The next kernel may start
+// only after this point, so at most two are in flight.  (64 x 128 x 128, width
+// 32: @T1@ us a training step, 1223 us without.)
+__device__ __forceinline__ void grid_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// launch with that attribute
+template <typename Args>
+cudaError_t launch_pdl(void (*kern)(Args), int grid, int block, int smem, const Args &a, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
 __device__ __forceinline__ void fail(volatile int *abort_flag, int *err, int code) {
     *abort_flag = 1;
     atomicOr(err, code);
@@ -162,6 +188,9 @@ struct ConvCfg {
     static constexpr int BY_SMEM = 233472 / (SMEM + 1024), BY_TMEM = 512 / TMEM_COLS;
     static constexpr int CTAS = BY_SMEM < BY_TMEM ? BY_SMEM : BY_TMEM;
     static_assert(CTAS >= 1, "one CTA fits");
+    // what a launch asks for: enough that no more CTAs than that share an SM
+    // (a CTA beyond the TMEM of an SM would sit there until another one ends)
+    static constexpr int LAUNCH_SMEM = CTAS == 1 && BY_SMEM > 1 ? 233472 / 2 : SMEM;
     // epilogue groups of four warps: as many as the registers of the CTAs hold
     // and as help (32 -> 32 channels at 256^3: 2 groups 652 us, 3 645, 4 672)
     static constexpr int groups(int epi) { return CTAS > 1 || epi == EPI_DGRAD ? 2 : 3; }
@@ -240,8 +269,13 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
         mbar_init(dbar + 8, 1);
         *abort_flag = 0;
         mbar_init_fence();
+        mbar_expect_tx(wbar, C::WB);
+        bulk_load(wsm, a.wimg, C::WB, wbar);
     }
     if (warp == 1) tmem_alloc(smem_u32(tslot), C::TMEM_COLS);
+    // Everything above reads parameters only, which no kernel of the same pass
+    // writes: it may run while the kernel before still does.
+    grid_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -258,10 +292,6 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
             uint32_t issued_q[C::RING];
 #pragma unroll
             for (int s = 0; s < C::RING; ++s) issued_q[s] = 0xFFFFFFFFu;
-            if (dz == 0) {
-                mbar_expect_tx(wbar, C::WB);
-                bulk_load(wsm, a.wimg, C::WB, wbar);
-            }
             uint32_t q = 0;
             bool ok = true;
             for (int it = blockIdx.x; ok && it < a.items; it += gridDim.x) {
@@ -643,6 +673,7 @@ __global__ void __launch_bounds__(256, 1) wgrad_kernel(const __grid_constant__ W
         mbar_init_fence();
     }
     if (warp == 1) tmem_alloc(smem_u32(tslot), C::TMEM_COLS);
+    grid_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -777,8 +808,8 @@ __global__ void __launch_bounds__(256, 1) wgrad_kernel(const __grid_constant__ W
 
 template <int CI, int CO, int EPI>
 cudaError_t conv_launch(const ConvArgs &a, int grid, cudaStream_t s) {
-    conv_kernel<CI, CO, EPI><<<grid, ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>::SMEM, s>>>(a);
-    return cudaGetLastError();
+    using C = ConvCfg<CI, CO>;
+    return launch_pdl(conv_kernel<CI, CO, EPI>, grid, C::threads(EPI), C::LAUNCH_SMEM, a, s);
 }
 
 template <int CI, int CO>
@@ -796,7 +827,7 @@ cudaError_t conv_launch_epi(int epi, const ConvArgs &a, int grid, cudaStream_t s
 template <int CI, int CO, int EPI>
 cudaError_t conv_attr() {
     return cudaFuncSetAttribute(conv_kernel<CI, CO, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                ConvCfg<CI, CO>::SMEM);
+                                ConvCfg<CI, CO>::LAUNCH_SMEM);
 }
 
 template <int CI, int CO>
@@ -855,12 +886,11 @@ cudaError_t launch_conv(int ci, int co, int epi, const ConvArgs &a, int grid, cu
 }
 
 cudaError_t launch_wgrad(int cx, int cz, const WgradArgs &a, int grid, cudaStream_t s) {
-    if (cx == 16 && cz == 16) wgrad_kernel<16, 16><<<grid, 256, WgCfg<16, 16>::SMEM, s>>>(a);
-    else if (cx == 16 && cz == 32) wgrad_kernel<16, 32><<<grid, 256, WgCfg<16, 32>::SMEM, s>>>(a);
-    else if (cx == 32 && cz == 16) wgrad_kernel<32, 16><<<grid, 256, WgCfg<32, 16>::SMEM, s>>>(a);
-    else if (cx == 32 && cz == 32) wgrad_kernel<32, 32><<<grid, 256, WgCfg<32, 32>::SMEM, s>>>(a);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (cx == 16 && cz == 16) return launch_pdl(wgrad_kernel<16, 16>, grid, 256, WgCfg<16, 16>::SMEM, a, s);
+    if (cx == 16 && cz == 32) return launch_pdl(wgrad_kernel<16, 32>, grid, 256, WgCfg<16, 32>::SMEM, a, s);
+    if (cx == 32 && cz == 16) return launch_pdl(wgrad_kernel<32, 16>, grid, 256, WgCfg<32, 16>::SMEM, a, s);
+    if (cx == 32 && cz == 32) return launch_pdl(wgrad_kernel<32, 32>, grid, 256, WgCfg<32, 32>::SMEM, a, s);
+    return cudaErrorInvalidValue;
 }
 
 }  // namespace nn
