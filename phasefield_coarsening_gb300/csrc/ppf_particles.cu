@@ -69,6 +69,16 @@ __device__ __forceinline__ int find_root(L lab, int i) {
     return -1;
 }
 
+// the root without halving, for labels that nobody changes any more
+__device__ __forceinline__ int climb(BrickLabels lab, int i) {
+    for (int it = 0; it < kMaxRetry; ++it) {
+        const int p = lab.get(i);
+        if (p == i) return i;
+        i = p;
+    }
+    return -1;
+}
+
 // Climbs from both nodes at once (two loads in flight), halving both paths.
 template <typename L>
 __device__ __forceinline__ bool unite(L lab, int a, int b) {
@@ -271,7 +281,9 @@ __global__ void __launch_bounds__(kBrickNT, 3) label_bricks(Geom g, Words q, con
         const bool face = lx == 0 || lx == bw - 1 || w == q.nw - 1 || ly == 0 || ly == kBrickY - 1 || y == q.ny - 1 ||
                           lz == 0 || lz == bz - 1 || z == q.nz - 1;
         for (int k = 0; k < nruns; ++k) {
-            const int i = k * kBrickNT + t, r = L.get(i), node = row * q.npr + 16 * w + k;
+            // (the label may be short of the root again: another thread's halving,
+            // begun before the root was set, can have put an ancestor there)
+            const int i = k * kBrickNT + t, r = climb(L, i), node = row * q.npr + 16 * w + k;
             if (r == i) {
                 lab[node] = node;
                 vol[node] = sm.vol[i];

@@ -162,3 +162,20 @@ def test_gpu_particles_over_bricks(shape, bc, fill):
     assert g["interface_area"] == o["interface_area"] and g["solid_volume"] == o["solid_volume"]
     assert n.value == o["count"] and some[few] == -1
     assert np.all(np.diff(some[:few]) >= 0) and np.all(np.isin(some[:few], o["volumes"]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fill", [0.3, 0.36])
+def test_gpu_particles_repeat(fill):
+    """Large branching components over many bricks, analysed again and again with
+    other contents of the scratch in between: the same components every time."""
+    shape = (64, 64, 256)
+    r = np.random.default_rng(int(100 * fill))
+    e = np.where(r.random(shape) < fill, 0.9, 0.1)
+    o = oracle.particles(e, bc=0)
+    with ppf.Simulation(shape, precision="f32") as s:
+        s.upload(e, 1.0 - e, np.full(shape, 0.7))
+        for k in range(40):
+            s.particles(0.05 if k % 2 else 0.95, volumes=True)
+            g = s.particles(volumes=True)
+            assert g["count"] == o["count"] and np.array_equal(g["volumes"], o["volumes"]), k
