@@ -112,6 +112,8 @@ static Coef<T> make_coef(const ppf_params &p, const ppf_derived &d) {
 
 int check_device_error(ppf_ctx *c);
 
+constexpr int kResults = 32, kWords = 16;   // dres: doubles, and the words behind them (derr)
+
 static Fields<float> ff(ppf_ctx *c, int be, int bc_) {
     return {(float *)c->fld[be][0], (float *)c->fld[be][1], (float *)c->fld[bc_][2]};
 }
@@ -178,14 +180,14 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
     cudaError_t e1 = cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking);
     cudaError_t e2 = e1 == cudaSuccess ? cudaMalloc(&c->state, 6 * fbytes) : e1;
     cudaError_t e3 = e2 == cudaSuccess ? cudaMalloc(&c->staging, 3 * (size_t)cells * sizeof(double)) : e2;
-    cudaError_t e4 = e3 == cudaSuccess ? cudaMalloc(&c->dres, 32 * sizeof(double) + 64) : e3;
+    cudaError_t e4 = e3 == cudaSuccess ? cudaMalloc(&c->dres, kResults * sizeof(double) + kWords * sizeof(int)) : e3;
     if (e4 != cudaSuccess) {
         ppf_destroy(c);
         return seterr(e4 == cudaErrorMemoryAllocation ? PPF_ENOMEM : PPF_ECUDA, "device setup failed: %s",
                       cudaGetErrorString(e4));
     }
     c->stream = c->own;
-    c->derr = (int *)(c->dres + 32);
+    c->derr = (int *)(c->dres + kResults);
     c->dsched = c->derr + 4;
     c->dbox = own_box(c);
     c->wait_limit_ns = 1000000000ULL;
@@ -211,7 +213,7 @@ extern "C" int ppf_create(int nz, int ny, int nx, const ppf_params *p, int bc, i
     }
     // zero the padding once so that unused ghost edges hold finite values
     e = cudaMemsetAsync(c->state, 0, 6 * fbytes, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->dres, 0, 32 * sizeof(double) + 64, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->dres, 0, kResults * sizeof(double) + kWords * sizeof(int), c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         ppf_destroy(c);
@@ -394,12 +396,10 @@ extern "C" int ppf_download_device(ppf_ctx *c, double *etaS, double *etaL, doubl
     return PPF_OK;
 }
 
-// Reads and clears the device error word; PPF_ETIMEOUT when a kernel's
-// bounded wait ran out since the last check.
-int check_device_error(ppf_ctx *c) {
-    int w[10] = {0};   // the error word, ..., the context's own box words
-    CU(cudaMemcpyAsync(w, c->derr, sizeof w, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
+// The context's words after a synchronisation: the error word, the scheduler
+// pairs, the context's own box words.  Clears a set error word; PPF_ETIMEOUT
+// when a kernel's bounded wait ran out since the last check.
+static int check_words(ppf_ctx *c, const int *w) {
     if (c->fx_ok && c->dbox == own_box(c) && w[8 + c->cur_c]) c->left_box = 1;
     if (w[0]) {
         // the error word, and the scheduler pairs that an abandoned step may leave set
@@ -408,6 +408,26 @@ int check_device_error(ppf_ctx *c) {
         return seterr(PPF_ETIMEOUT, "a device wait exceeded its limit; the state of that step is invalid");
     }
     return PPF_OK;
+}
+
+int check_device_error(ppf_ctx *c) {
+    int w[kWords];
+    CU(cudaMemcpyAsync(w, c->derr, sizeof w, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaStreamSynchronize(c->stream));
+    return check_words(c, w);
+}
+
+// The same with the results of reductions, which stand before the words: one
+// copy to the host instead of two (about 8 us each).
+static int fetch_results(ppf_ctx *c, double (&h)[kResults]) {
+    struct {
+        double d[kResults];
+        int w[kWords];
+    } r;
+    CU(cudaMemcpyAsync(&r, c->dres, sizeof r, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaStreamSynchronize(c->stream));
+    std::memcpy(h, r.d, sizeof h);
+    return check_words(c, r.w);
 }
 
 static int run_steps(ppf_ctx *c, int64_t nsteps, bool c_only) {
@@ -467,9 +487,8 @@ extern "C" int ppf_reduce(ppf_ctx *c, ppf_stats *out) {
         CU(launch_observe<double>(c->g, c->cd, c->fx_ok ? &c->kx : nullptr, cst(fd(c, c->cur_eta, c->cur_c)), c->partials,
                                   c->num_sms, c->stream));
     CU(launch_final_sum(c->partials, nb, 5, 5, c->dres + 3, c->stream));
-    double h[8];
-    CU(cudaMemcpyAsync(h, c->dres, 8 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    rc = check_device_error(c);
+    double h[kResults];
+    rc = fetch_results(c, h);
     if (rc) return rc;
     out->sum_dc2 = h[0];
     out->sum_detaS2 = h[1];
@@ -731,10 +750,10 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     else
         CU(launch_particles<double>(c->g, (const double *)c->fld[c->cur_eta][0], threshold, ps, c->partials, nb,
                                     c->num_sms, c->p.dx, dout, vols, cap, c->derr, c->stream));
-    double h[5];
-    CU(cudaMemcpyAsync(h, dout, 5 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    rc = check_device_error(c);
+    double res[kResults];
+    rc = fetch_results(c, res);
     if (rc) return rc;
+    const double *const h = res + 8;
     const double dx = c->p.dx;
     out->count = (int64_t)h[0];
     out->mean_radius = h[0] > 0 ? h[1] / h[0] / dx : 0.0;
