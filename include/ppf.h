@@ -365,8 +365,8 @@ int ppf_surrogate_advance(ppf_surrogate *s, ppf_ctx *ctx, int ncalls);
 int ppf_surrogate_debug_inject(ppf_surrogate *s, int fault);
 
 /* Measured FP64 FMA rate of the current device in TFLOP/s (2 FLOPs per
- * FMA): the denominator of the FP64 step's roofline, which the FP64 pipe
- * bounds on this GPU.  No counterpart in the reference.  Takes ~0.1 s. */
+ * FMA): what the FP64 step in fixed point is compared with.  No counterpart
+ * in the reference.  Takes ~0.1 s. */
 int ppf_measure_fp64_peak(double *tflops);
 
 /* Message for the calling thread's last failure ("" if none). */

@@ -36,7 +36,7 @@
 //   What bounds it: 24 MMAs a row, 56 cycles each (N = 96), 1344 cycles a row;
 //   loading nine X segments for every tile (40 copies) and 72 MMAs of N = 32
 //   (40 cycles each) it took about 5200 (146 us for 32 -> 32 channels on
-//   64 x 128 x 128).
+//   64 x 128 x 128; now 68 us, a third of it the ramp and the write-out).
 //
 // Every mbarrier wait is bounded by a time limit; on expiry the CTA sets
 // the error word, stops issuing work, drains its own copies and MMAs

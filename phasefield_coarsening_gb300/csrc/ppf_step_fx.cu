@@ -3,9 +3,9 @@
 //
 // What bounded the float64 step was the FP64 pipe: about 75 operations per
 // cell-step at 2 lanes per clock and SM, 2.2 ms at 256^3 against 0.12 ms for
-// its memory traffic.  Here a cell costs about 810 instructions, integer but
+// its memory traffic.  Here a cell costs about 820 instructions, integer but
 // for six FP64 operations (each field's increment converted and added by one
-// fused multiply-add): 0.67 ms at 256^3, 19 us at 64^3 (56 us).  What bounds
+// fused multiply-add): 0.64 ms at 256^3, 19 us at 64^3 (56 us).  What bounds
 // it now is instruction issue and the two integer pipes, each about half
 // busy (ncu: 53 % of issue slots; ALU 0.97, multiplier 0.91 instructions per
 // clock and SM of 2 each).
