@@ -363,7 +363,7 @@ struct FxSum {
 // Cells of an FP64 state in fixed-point arithmetic (ppf_fx.h), but for the
 // gradient's differences and squares: those twelve are what is left of about
 // 32 operations a cell for the FP64 pipe, which runs beside the integer
-// pipes.
+// pipes.  256^3: 0.49 ms; 1.12 ms with all of it in FP64.
 struct ObsFx {
     FxSum mass, h, w, f0;
     double gr = 0;

@@ -179,3 +179,21 @@ def test_gpu_particles_repeat(fill):
             s.particles(0.05 if k % 2 else 0.95, volumes=True)
             g = s.particles(volumes=True)
             assert g["count"] == o["count"] and np.array_equal(g["volumes"], o["volumes"]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(12, 16, 64), (33, 32, 64), (40, 48, 128), (80, 96, 128)])
+def test_gpu_particle_volumes_in_order(shape):
+    """Few, some and more volumes than one block sorts (single cells on a lattice,
+    one in five of them grown to a row of up to 19 cells in the gap planes)."""
+    r = np.random.default_rng(sum(shape))
+    e = np.zeros(shape)
+    e[::2, ::2, ::2] = 1.0
+    for z, y, x in np.argwhere(e > 0):
+        if r.random() < 0.2 and z + 1 < shape[0]:
+            e[z + 1, y, x:x + r.integers(1, 20)] = 1.0
+    o = oracle.particles(e, bc=1)
+    with ppf.Simulation(shape, bc=1) as s:
+        s.upload(e, 1.0 - e, np.full(shape, 0.7))
+        g = s.particles(volumes=True)
+    assert g["count"] == o["count"] and np.array_equal(g["volumes"], np.sort(o["volumes"]))
