@@ -312,9 +312,9 @@ struct ObsAcc {
     int n = 0, solid = 0, bad = 0;
 
     // a pair of finite cells (own values and the +x, +y, +z neighbours), of
-    // which only the first counts when `one` is set
+    // which the first nv count
     __device__ __forceinline__ void pair(const ObsCoef<T> &k, V2<T> eS, V2<T> eL, V2<T> c, V2<T> sx, V2<T> lx,
-                                         V2<T> sy, V2<T> ly, V2<T> sz, V2<T> lz, bool one = false) {
+                                         V2<T> sy, V2<T> ly, V2<T> sz, V2<T> lz, int nv = 2) {
         const V2<T> S2 = eS * eS, L2 = eL * eL, s2 = fma2(eL, eL, S2);
         const V2<T> hh = S2 * recip(s2);
         const V2<T> ww = fma2(hh, splat(k.dc0), c - splat(k.cL0));
@@ -339,7 +339,7 @@ struct ObsAcc {
         d = lz - eL;
         gr = fma2(d, d, gr);
         const V2<T> ff = fma2(splat(k.kg), gr, splat(k.m) * f0);
-        auto in = [&](V2<T> v) { return one ? V2<T>(v.x(), T(0)) : v; };
+        auto in = [&](V2<T> v) { return V2<T>(nv > 0 ? v.x() : T(0), nv > 1 ? v.y() : T(0)); };
         mass.add(in(c));
         h.add(in(hh));
         w.add(in(ch));
@@ -391,8 +391,12 @@ struct ObsFx {
 };
 
 // FX: an FP64 state whose parameters fit the fixed-point step; cells outside
-// its box take the FP64 path.
-template <typename T, bool FX>
+// its box take the FP64 path.  MASK: the rows' last groups hold fewer cells than
+// the others; a warp with such a group counts its cells by mask, all lanes alike
+// (250^3 FP32, whole reduction: 72 us, 115 us with those cells taken one by one;
+// 128 x 128 x 135 FP64: 118 and 152 us).  A kernel of its own, since the masks cost
+// the others 3 %.
+template <typename T, bool FX, bool MASK>
 __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoef<T> k, Fields<const T> fl, int nq, int zc,
                                                       double *partials, fx::FxCoef kx) {
     constexpr int Q = 16 / (int)sizeof(T), NP = Q / 2;   // cells and pairs per thread
@@ -401,9 +405,13 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
     const int cbias = FX ? fx::c_bias(kx.ec) : 0;
     const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int y = (int)(t / nq), x0 = (int)(t - (int64_t)y * nq) * Q;
+    // (a test at run time also where it always holds: without it the compiler
+    // orders the loads so that registers run out, 695 us at 512^3 instead of 520)
+    const bool whole = x0 + Q <= g.nx;
+    const int cells = MASK && y < g.ny ? min(Q, g.nx - x0) : Q;
+    const bool masked = MASK && __any_sync(0xffffffffu, cells < Q);
     if (y < g.ny) {
         const int z0 = blockIdx.y * zc, z1 = min(g.nz, z0 + zc);
-        const bool whole = x0 + Q <= g.nx;
         int64_t j = g.at(x0, y, z0);        // rows start on a sector: 16-byte aligned
         T s[Q], l[Q];
         auto load = [](const T *p, T (&v)[Q]) {
@@ -425,34 +433,41 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
             load(fl.eL + j + g.PS, lz);
             // the cell after the last one (a ghost at the domain's end)
             const T sx = whole ? fl.eS[j + Q] : T(0), lx = whole ? fl.eL[j + Q] : T(0);
-            bool fine = whole;
+            bool fine = MASK || whole;
 #pragma unroll
-            for (int i = 0; i < Q; ++i) fine = fine && finite_(s[i]) && finite_(l[i]) && finite_(c[i]);
+            for (int i = 0; i < Q; ++i) fine = fine && (i >= cells || (finite_(s[i]) && finite_(l[i]) && finite_(c[i])));
             if constexpr (FX) {
 #pragma unroll
-                for (int i = 0; i < Q; ++i) fine = fine && !out_of_box(s[i], l[i], c[i], kx.cmax);
+                for (int i = 0; i < Q; ++i) fine = fine && (i >= cells || !out_of_box(s[i], l[i], c[i], kx.cmax));
             }
             if (fine) {
-                acc.n += Q;
+                acc.n += cells;
 #pragma unroll
-                for (int i = 0; i < Q; ++i) acc.solid += above_half(s[i]) ? 1 : 0;
+                for (int i = 0; i < Q; ++i) acc.solid += i < cells && above_half(s[i]) ? 1 : 0;
                 if constexpr (FX) {
 #pragma unroll
                     for (int i = 0; i < Q; ++i)
-                        ax.cell(kx, cbias, s[i], l[i], c[i], i == Q - 1 ? sx : s[(i + 1) % Q],
-                                i == Q - 1 ? lx : l[(i + 1) % Q], sy[i], ly[i], sz[i], lz[i]);
-                } else
+                        if (i < cells)
+                            ax.cell(kx, cbias, s[i], l[i], c[i], i == Q - 1 ? sx : s[(i + 1) % Q],
+                                    i == Q - 1 ? lx : l[(i + 1) % Q], sy[i], ly[i], sz[i], lz[i]);
+                } else {
+                    auto pairs = [&](int n) {
 #pragma unroll
-                for (int i = 0; i < NP; ++i) {
-                    const int a = 2 * i, b = a + 1;
-                    const bool e = b == Q - 1;
-                    acc.pair(k, V2<T>(s[a], s[b]), V2<T>(l[a], l[b]), V2<T>(c[a], c[b]),
-                             V2<T>(s[b], e ? sx : s[(b + 1) % Q]), V2<T>(l[b], e ? lx : l[(b + 1) % Q]),
-                             V2<T>(sy[a], sy[b]), V2<T>(ly[a], ly[b]), V2<T>(sz[a], sz[b]), V2<T>(lz[a], lz[b]));
+                        for (int i = 0; i < NP; ++i) {
+                            const int a = 2 * i, b = a + 1;
+                            const bool e = b == Q - 1;
+                            acc.pair(k, V2<T>(s[a], s[b]), V2<T>(l[a], l[b]), V2<T>(c[a], c[b]),
+                                     V2<T>(s[b], e ? sx : s[(b + 1) % Q]), V2<T>(l[b], e ? lx : l[(b + 1) % Q]),
+                                     V2<T>(sy[a], sy[b]), V2<T>(ly[a], ly[b]), V2<T>(sz[a], sz[b]),
+                                     V2<T>(lz[a], lz[b]), n - a);
+                        }
+                    };
+                    if (masked) pairs(cells);
+                    else pairs(Q);
                 }
             } else {
-                // a partial group at the row's end, or non-finite cells (counted
-                // and left out): cell by cell, twice the same cell in a pair
+                // non-finite cells (counted and left out), or cells outside the box:
+                // cell by cell, twice the same cell in a pair
                 for (int i = 0; i < Q && x0 + i < g.nx; ++i) {
                     const int64_t a = j + i;
                     const T S = fl.eS[a], L = fl.eL[a], C = fl.c[a];
@@ -464,7 +479,7 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
                     acc.solid += above_half(S) ? 1 : 0;
                     acc.pair(k, splat(S), splat(L), splat(C), splat(fl.eS[a + 1]), splat(fl.eL[a + 1]),
                              splat(fl.eS[a + g.P]), splat(fl.eL[a + g.P]), splat(fl.eS[a + g.PS]),
-                             splat(fl.eL[a + g.PS]), true);
+                             splat(fl.eL[a + g.PS]), 1);
                 }
             }
 #pragma unroll
@@ -557,13 +572,16 @@ cudaError_t launch_observe(const Geom &g, const CoefD &k, const fx::FxCoef *kx, 
     o.dC = k.CS - k.CL;
     o.vol = k.vol;
     const dim3 grid((unsigned)bx, (unsigned)bz);
+    const bool ragged = g.nx % (16 / (int)sizeof(T)) != 0;
     if constexpr (std::is_same<T, double>::value) {
         if (kx) {
-            observe_kernel<T, true><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, *kx);
+            if (ragged) observe_kernel<T, true, true><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, *kx);
+            else observe_kernel<T, true, false><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, *kx);
             return cudaGetLastError();
         }
     }
-    observe_kernel<T, false><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, fx::FxCoef());
+    if (ragged) observe_kernel<T, false, true><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, fx::FxCoef());
+    else observe_kernel<T, false, false><<<grid, 256, 0, s>>>(g, o, f, nq, zc, partials, fx::FxCoef());
     return cudaGetLastError();
 }
 
