@@ -85,8 +85,12 @@ __device__ __forceinline__ void block_sum_store(double (&v)[NV], double *partial
 // are worked out once and a lane only adds x (no 64-bit divisions per cell).
 // The caller's three arrays are read and written in place when they are
 // device memory of this device; host arrays pass through the staging array.
-// 256^3 FP32, state to device arrays: 101 us, 6.0 TB/s; through the staging
-// array with one thread per cell it was 106 us and 126 us of copies.
+// A lane loads four of its accesses before it stores one, by predicate, so that
+// rows that end inside them wait for memory as often as whole ones do.
+// Whole download, FP32: 256^3 109 us (117 with a loop the compiler unrolled by
+// four, whose remainder went one access at a time), 250^3 107 (152), 251^3 106
+// (224), 512^3 798 (938); through the staging array with one thread per cell
+// 256^3 took 106 us and 126 us of copies.
 
 constexpr int kRowWarps = 8;   // rows per block and pass
 
@@ -106,17 +110,30 @@ __device__ __forceinline__ void pack_rows(const Geom &g, const double *__restric
         const int64_t i0 = (int64_t)r * g.nx;
         const bool inner = y > 0 && y < g.ny - 1 && z > 0 && z < g.nz - 1;   // feeds x ghosts only
         const int64_t a0 = g.at(0, y, z);
-#pragma unroll 4
-        for (int x = lane; x < g.nx; x += 32) {
-            const T s = (T)s0[i0 + x], l = (T)s1[i0 + x], c = (T)s2[i0 + x];
-            if (std::is_same<T, double>::value && box.word)
-                bad = bad || out_of_box(s, l, c, box.cmax);
-            if (inner && x > 0 && x < g.nx - 1) {
-                dst.eS[a0 + x] = s;
-                dst.eL[a0 + x] = l;
-                dst.c[a0 + x] = c;
-            } else {
-                store_with_ghosts(g, dst, x, y, z, s, l, c, false);
+        for (int x0 = lane; x0 < g.nx; x0 += 128) {
+            double v[4][3];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (x0 + 32 * k < g.nx) {
+                    const int64_t i = i0 + x0 + 32 * k;
+                    v[k][0] = s0[i];
+                    v[k][1] = s1[i];
+                    v[k][2] = s2[i];
+                }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int x = x0 + 32 * k;
+                if (x >= g.nx) continue;
+                const T s = (T)v[k][0], l = (T)v[k][1], c = (T)v[k][2];
+                if (std::is_same<T, double>::value && box.word)
+                    bad = bad || out_of_box(s, l, c, box.cmax);
+                if (inner && x > 0 && x < g.nx - 1) {
+                    dst.eS[a0 + x] = s;
+                    dst.eL[a0 + x] = l;
+                    dst.c[a0 + x] = c;
+                } else {
+                    store_with_ghosts(g, dst, x, y, z, s, l, c, false);
+                }
             }
         }
     }
@@ -152,19 +169,44 @@ __device__ __forceinline__ void unpack_rows(const Geom &g, const T *__restrict__
         const int z = r / g.ny, y = r - z * g.ny;
         const int64_t i0 = (int64_t)r * g.nx, a0 = g.at(0, y, z);
         if (two) {
-#pragma unroll 4
-            for (int x = 2 * lane; x < g.nx; x += 64) {
-                const V2<T> s = ld2(eS + a0 + x), l = ld2(eL + a0 + x), q = ld2(c + a0 + x);
-                st2(d0 + i0 + x, V2<double>(widen(s.x()), widen(s.y())));
-                st2(d1 + i0 + x, V2<double>(widen(l.x()), widen(l.y())));
-                st2(d2 + i0 + x, V2<double>(widen(q.x()), widen(q.y())));
+            for (int x0 = 2 * lane; x0 < g.nx; x0 += 256) {
+                V2<T> s[4], l[4], q[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x0 + 64 * k < g.nx) {
+                        const int64_t a = a0 + x0 + 64 * k;
+                        s[k] = ld2(eS + a);
+                        l[k] = ld2(eL + a);
+                        q[k] = ld2(c + a);
+                    }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x0 + 64 * k < g.nx) {
+                        const int64_t i = i0 + x0 + 64 * k;
+                        st2(d0 + i, V2<double>(widen(s[k].x()), widen(s[k].y())));
+                        st2(d1 + i, V2<double>(widen(l[k].x()), widen(l[k].y())));
+                        st2(d2 + i, V2<double>(widen(q[k].x()), widen(q[k].y())));
+                    }
             }
         } else {
-#pragma unroll 4
-            for (int x = lane; x < g.nx; x += 32) {
-                d0[i0 + x] = widen(eS[a0 + x]);
-                d1[i0 + x] = widen(eL[a0 + x]);
-                d2[i0 + x] = widen(c[a0 + x]);
+            for (int x0 = lane; x0 < g.nx; x0 += 128) {
+                T s[4], l[4], q[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x0 + 32 * k < g.nx) {
+                        const int64_t a = a0 + x0 + 32 * k;
+                        s[k] = eS[a];
+                        l[k] = eL[a];
+                        q[k] = c[a];
+                    }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (x0 + 32 * k < g.nx) {
+                        const int64_t i = i0 + x0 + 32 * k;
+                        d0[i] = widen(s[k]);
+                        d1[i] = widen(l[k]);
+                        d2[i] = widen(q[k]);
+                    }
             }
         }
     }
@@ -183,7 +225,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) unpack_kernel(Geom g, Fields<c
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32 * kRowWarps) pack_multi_kernel(const IoDesc *__restrict__ table) {
+__global__ void __launch_bounds__(32 * kRowWarps, 3) pack_multi_kernel(const IoDesc *__restrict__ table) {
     const IoDesc &d = table[blockIdx.y];
     const Geom g = d.g;
     const Fields<T> dst = {(T *)d.fld[0][0], (T *)d.fld[0][1], (T *)d.fld[0][2]};
@@ -193,7 +235,7 @@ __global__ void __launch_bounds__(32 * kRowWarps) pack_multi_kernel(const IoDesc
 }
 
 template <typename T>
-__global__ void __launch_bounds__(32 * kRowWarps) unpack_multi_kernel(const IoDesc *__restrict__ table, int buf) {
+__global__ void __launch_bounds__(32 * kRowWarps, 3) unpack_multi_kernel(const IoDesc *__restrict__ table, int buf) {
     const IoDesc &d = table[blockIdx.y];
     const Geom g = d.g;
     const int64_t n = (int64_t)g.nx * g.ny * g.nz;
