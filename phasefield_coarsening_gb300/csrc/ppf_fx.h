@@ -5,12 +5,24 @@
 // busy).  Every quantity of the step but the state itself is bounded once
 // the state lies in a box (|eta| < 1.75, eta_S^2 + eta_L^2 >= 1/4, |c| below
 // twice a power of two above the parabola minima), so it is held here as a
-// 64-bit integer with a fixed binary scale ("x@s" is x 2^s).  The absolute
-// resolution of the products, 2^-56 to 2^-59, is finer than the rounding of
-// the same values in float64 (2^-53 to 2^-54 near 1), and the increments are
-// added to the float64 state with one rounding (a fused multiply-add), so
-// the result is no less accurate than float64 arithmetic throughout;
-// integer sums are exact, and a face's flux is the same number with the
+// 64-bit integer with a fixed binary scale ("x@s" is x 2^s).
+//
+// A fixed scale bounds errors absolutely, so it serves the quantities whose
+// float64 arithmetic has an absolute error too: the interpolation h, w and M',
+// the fluxes (differences of numbers of the size of the parabola minima), and
+// the rates of the phase fields, in which terms of the size of the model's
+// constants cancel.  The products' resolution, 2^-56 to 2^-62, is finer than
+// float64's rounding of the same values.  A phase field itself falls off by
+// orders of magnitude behind an interface, where float64 keeps 53 bits of
+// whatever is left, and a fixed scale would lose them.  So a cell's larger
+// field, at least 0.35 in the box, takes its increment in fixed point, and the
+// smaller one's, rate x eta - kt x Laplacian, is formed in float64, as exact
+// relative to a value of 1e-300 as to one of 1.  The new values are as close to
+// the exact ones as float64 arithmetic's (root mean square within 0.01 %, each
+// relative to its own size); an increment of a larger field is resolved to
+// 2^(eu-62), 1e-19 with the reference's constants, where float64's own error in
+// an interface is 3e-19.
+// Integer sums are exact, and a face's flux is the same number with the
 // opposite sign seen from its other side.  A product is three 32 x 32 ->
 // 64-bit multiply-adds.
 //
@@ -43,11 +55,13 @@ struct FxCoef {
     i64 cL0;       // @59, in units of 2^ec
     i64 dc0;       // @62
     i64 m0, m1;    // A M' = m0 + m1 h: m0@64, m1@65
-    i64 k0, k1;    // drive k = k0 + k1 w, in units of 2^eu: k0@60, k1@65
+    i64 k0, k1;    // drive k = k0 + k1 w, in units of 2^eu: k0@62, k1@65
     i64 mt, mtg;   // mt and mt (2 gamma - 1) @68, units of 2^eu
-    i64 nkt;       // @66, units of 2^eu
+    i64 nkt, nk6;  // -kt @67 and -6 kt @61, units of 2^eu
     i64 g;         // gamma @61
-    double su, sc; // 2^(eu-59), 2^(ec-59): increments of eta and c
+    double su, sc; // 2^(eu-61), 2^(ec-59): increments of eta and c
+    double kb;     // -kt in units of su
+    int se;        // -eu (0 to 40)
     int ec, eu;
     unsigned cmax; // high word of the box bound of |c|, 2^(ec+1)
 };
@@ -124,17 +138,18 @@ PPF_FX i64 recip(i64 s2) {
 
 // what a cell's neighbours need
 struct Nb {
-    i64 S, L;      // eta @57
+    i64 S, L;      // eta @58
     i64 W, M;      // w @59 in units of 2^ec, A M' @64
 };
-// what the cell itself needs besides
+// the cell's rates @61 (units of 2^eu, below 2.1 of them): the increment of
+// eta is rate x eta - kt x its Laplacian
 struct Own {
-    i64 h;         // @61
-    i64 G;         // drive k / (etaS^2 + etaL^2) @59, units of 2^eu
+    i64 bS, bL;
 };
 
+// `rates`: whether the cell's own rates are wanted too
 template <bool C_ONLY>
-PPF_FX void pass_a(const FxCoef &k, double eS, double eL, double c, int cbias, Nb &n, Own &o) {
+PPF_FX void pass_a(const FxCoef &k, double eS, double eL, double c, int cbias, Nb &n, Own &o, bool rates = true) {
     const i64 S = to_fx(eS, kEtaBias), L = to_fx(eL, kEtaBias);
     const i64 S2 = mulx<2>(S, S), L2 = mulx<2>(L, L);        // @60
     const i64 R = recip(S2 + L2);                            // @60
@@ -143,30 +158,49 @@ PPF_FX void pass_a(const FxCoef &k, double eS, double eL, double c, int cbias, N
     n.W = C - k.cL0 + mulq(k.dc0, h);
     n.M = k.m0 + (mulq(k.m1, h) << 2);
     if (!C_ONLY) {
-        n.S = S >> 4;
-        n.L = L >> 4;
-        o.h = h;
-        o.G = mulx<3>(k.k0 + mulq(k.k1, n.W), R);            // @59
+        n.S = S >> 3;
+        n.L = L >> 3;
+        if (!rates) return;
+        // phasefield.c:360-373 divided by eta:
+        //   mt (eta^2 - 1 + 2 gamma other^2) + drive k other^2 / (etaS^2 + etaL^2)^2,
+        // the first as mt (etaS^2 + etaL^2 - 1) + mt (2 gamma - 1) other^2, @64;
+        // the second with G = k / (etaS^2 + etaL^2) as G (1 - h), -G h, all @61
+        const i64 u = mulq(k.mt, S2 + L2 - (1ll << 60)) + 4;
+        const i64 G = mulx<3>(k.k0 + mulx<2>(k.k1, n.W), R);
+        o.bS = ((u + mulq(k.mtg, L2)) >> 3) + mulx<3>(G, (1ll << 61) - h);
+        o.bL = ((u + mulq(k.mtg, S2)) >> 3) - mulx<3>(G, h);
     }
 }
 
 // (M' + M)(mu' - mu) of one face, @59
 PPF_FX i64 face(i64 Mn, i64 M, i64 Wn, i64 W) { return mulq(Mn + M, Wn - W); }
 
-// the increments of etaS and etaL @59 (units of 2^eu): phasefield.c:360-373,
-// from the cell's own values S, L @57 and the sums S6, L6 of its six
-// neighbours' @57
+// The increment of a phase field in units of su, @61 in fixed point (below
+// 1.1 of 2^eu: eta other^2 / (etaS^2 + etaL^2)^2 is at most 0.77): from its
+// rate, its own value and the sum of its six neighbours', all @58.
+PPF_FX i64 eta_inc(const FxCoef &k, i64 rate, i64 v, i64 six) {
+    return mulx<3>(v << 3, rate) + mulq(k.nkt, six - 6 * v);
+}
 PPF_FX void eta_inc(const FxCoef &k, const Own &o, i64 S, i64 L, i64 S6, i64 L6, i64 &dS, i64 &dL) {
-    const i64 lS = S6 - 6 * S, lL = L6 - 6 * L;
-    S <<= 4;                                                                                         // @61
-    L <<= 4;
-    // mt eta (eta^2 - 1 + 2 gamma other^2), as eta (mt (etaS^2 + etaL^2 - 1) + mt (2 gamma - 1) other^2)
-    const i64 S2 = mulq(S, S), L2 = mulq(L, L);                                                      // @58
-    const i64 u = mulq(k.mt, S2 + L2 - (1ll << 58));                                                 // @62
-    const i64 wS = mulq(S, u + mulq(k.mtg, L2)), wL = mulq(L, u + mulq(k.mtg, S2));                  // @59
-    const i64 aS = mulq(S, (1ll << 61) - o.h), aL = mulq(L, o.h);                                    // @58
-    dS = wS + mulq(k.nkt, lS) + mulx<6>(aS, o.G);
-    dL = wL + mulq(k.nkt, lL) - mulx<6>(aL, o.G);
+    dS = eta_inc(k, o.bS, S, S6);
+    dL = eta_inc(k, o.bL, L, L6);
+}
+// The new value of a cell's larger field, from the value @58 (exact: at least
+// 0.35) and its increment: added as integers @60, then rounded once.
+PPF_FX double eta_large(const FxCoef &k, i64 v, i64 inc) {
+    const i64 n = (v << 2) + ((inc + (1ll << k.se)) >> (k.se + 1));
+#ifdef __CUDA_ARCH__
+    const double d = (double)n;
+    return __hiloint2double(n ? __double2hiint(d) - (60 << 20) : 0, __double2loint(d));
+#else
+    return std::ldexp((double)n, -60);
+#endif
+}
+// The increment of the smaller one, in the same units, in float64.  Its six
+// neighbours' weight is not in the rate; add it with one rounding,
+// fma(increment, su, v).
+PPF_FX double eta_inc(const FxCoef &k, i64 rate, double v, double six) {
+    return fma(k.kb, six, (double)(rate - k.nk6) * v);
 }
 
 // A cell's terms of the observables: c @59 and w^2 @59 (in units of 2^ec and
@@ -232,20 +266,23 @@ inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0
         std::frexp(need, &e);                  // need < 2^e
         if (e > eu) eu = e;
     }
-    if (eu > 0) return false;                  // increments coarser than 2^-59
+    if (eu > 0) return false;                  // rates coarser than 2^-61
     auto q = [](ld v, int s) { return (i64)std::llrint(std::ldexp(v, s)); };
     f.cL0 = q(cL0, 59 - ec);
     f.dc0 = q(dc0, 62 - ec);
     f.m0 = q(m0, 64);
     f.m1 = q(m1, 65);
-    f.k0 = q(k0, 60 - eu);
+    f.k0 = q(k0, 62 - eu);
     f.k1 = q(k1, 65 - eu);
     f.mt = q(mt, 68 - eu);
     f.mtg = q((ld)mt * ((ld)tg - 1), 68 - eu);
-    f.nkt = q(-kt, 66 - eu);
+    f.nkt = q(-kt, 67 - eu);
+    f.nk6 = q(-6 * (ld)kt, 61 - eu);
+    f.se = -eu;
     f.g = q(0.5 * tg, 61);
-    f.su = std::ldexp(1.0, eu - 59);
+    f.su = std::ldexp(1.0, eu - 61);
     f.sc = std::ldexp(1.0, ec - 59);
+    f.kb = std::ldexp(-kt, 61 - eu);
     f.ec = ec;
     f.eu = eu;
     f.cmax = (unsigned)(1023 + ec + 1) << 20;

@@ -3,12 +3,14 @@
 //
 // What bounded the float64 step was the FP64 pipe: about 75 operations per
 // cell-step at 2 lanes per clock and SM, 2.2 ms at 256^3 against 0.12 ms for
-// its memory traffic.  Here a cell costs about 820 instructions, integer but
-// for six FP64 operations (each field's increment converted and added by one
-// fused multiply-add): 0.64 ms at 256^3, 19 us at 64^3 (56 us).  What bounds
-// it now is instruction issue and the two integer pipes, each about half
-// busy (ncu: 53 % of issue slots; ALU 0.97, multiplier 0.91 instructions per
-// clock and SM of 2 each).
+// its memory traffic.  Here a cell has twelve: nine for the increment of its
+// smaller phase field, which keeps float64's relative precision however small
+// the value is (ppf_fx.h), one conversion of the larger one, two for c.
+// 0.64 ms at 256^3, 19 us at 64^3 (56 us).  The FP64 pipe and instruction
+// issue bound it together.  With both fields' increments in fixed point (six
+// operations, small values lost) it took as long, with both in float64 0.90 ms;
+// two additions in place of each conversion instruction, 0.78 against 0.70;
+// rates in the halo planes too, 0.64 ms and 20.6 us.
 //
 // The data flow is that of ppf_step_tma.cuh: work items (z chunk, 32 x 16
 // tile) marched up z, etaS/etaL/c boxes streamed by TMA, pass A once per
@@ -30,9 +32,9 @@ namespace {
 
 using G = TmaGeo<double, 0>;
 constexpr int kStages = 3;
-// Two cells per thread (0.67 ms at 256^3) interleave two chains of
-// arithmetic; one cell and twice the warps needs more than its 64 registers
-// (0.78 ms), and an unrolled plane loop more than 128 (0.76 ms).
+// Two cells per thread interleave two chains of arithmetic; one cell and twice
+// the warps needs more than its 64 registers, and an unrolled plane loop more
+// than 128 (0.78 and 0.76 ms at 256^3 where this form took 0.67).
 constexpr int kCells = 2;                      // cells per thread, stacked in y
 constexpr int kThreads = G::TX * G::TY / kCells;
 
@@ -131,6 +133,11 @@ __device__ __noinline__ void slow_cell(const Coef<double> &k, const Geom &g, con
     if (y == g.ny - 1) put(per ? j - g.ny * g.P : j + g.P);
     if (z == 0) put(per ? j + g.nz * g.PS : j - g.PS);
     if (z == g.nz - 1) put(per ? j - g.nz * g.PS : j + g.PS);
+}
+
+// which of a cell's fields is the smaller one: 0 etaS, 1 etaL
+__device__ __forceinline__ int smaller(double eS, double eL) {
+    return ((unsigned)__double2hiint(eL) & 0x7fffffffu) < ((unsigned)__double2hiint(eS) & 0x7fffffffu) ? 1 : 0;
 }
 
 // sum of three doubles over the CTA, in a fixed order, to partials[3 item ..]
@@ -295,16 +302,19 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         const int cbias = fx::c_bias(kx.ec);
 
-        // Registers between planes: h and the drive of the plane below (its other
-        // values are in the shared ring), the flux through its lower face and
-        // the etas of the plane below that.
-        fx::Own Q[kCells], X[kCells];
+        // Registers between planes: of the plane below, which field is the smaller
+        // one, the two rates (its other values are in the shared planes) and the
+        // flux through the lower face; of the plane below that, the larger field's
+        // value in fixed point and the smaller one's.
+        int small[kCells];
+        i64 rb[kCells], rs[kCells], Fz[kCells], zb[kCells];
+        double zs[kCells];
         fx::Nb Xn[kCells];
-        i64 Fz[kCells], Sm[kCells], Lm[kCells];
 #pragma unroll
         for (int j = 0; j < kCells; ++j) {
-            Q[j].h = Q[j].G = 0;
-            Fz[j] = Sm[j] = Lm[j] = 0;
+            small[j] = 0;
+            rb[j] = rs[j] = Fz[j] = zb[j] = 0;
+            zs[j] = 0;
         }
         double acc[3] = {0, 0, 0};
         int st = 0, mb = 0, st_prev = 0, mb_prev = 0, consumed = 0;
@@ -332,6 +342,8 @@ __global__ void __launch_bounds__(kThreads, 2)
                 const bool late = !mbar_wait(smem_u32(&sm.bar[st]), par, a.limit_ns);
                 if (late) atomicOr(a.err, 1);
                 const double *rS = sm.raw[st][0], *rL = sm.raw[st][1], *rC = sm.raw[st][2];
+                fx::Own X[kCells] = {};
+                int sm_new[kCells];
                 i64(*nb)[G::BOX] = sm.nb[mb];
                 auto put_nb = [&](int o, const fx::Nb &n) {
                     if (!C_ONLY) {
@@ -344,13 +356,14 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
                 for (int j = 0; j < kCells; ++j) {
                     const int o = ob + j * BX;
-                    fx::pass_a<C_ONLY>(kx, rS[o], rL[o], rC[o], cbias, Xn[j], X[j]);
+                    fx::pass_a<C_ONLY>(kx, rS[o], rL[o], rC[o], cbias, Xn[j], X[j], pz >= z0 && pz < z1);
                     put_nb(o, Xn[j]);
+                    if (!C_ONLY) sm_new[j] = smaller(rS[o], rL[o]);
                 }
                 if (rt >= 0) {
                     fx::Nb n;
                     fx::Own unused;
-                    fx::pass_a<C_ONLY>(kx, rS[ro], rL[ro], rC[ro], cbias, n, unused);
+                    fx::pass_a<C_ONLY>(kx, rS[ro], rL[ro], rC[ro], cbias, n, unused, false);
                     put_nb(ro, n);
                 }
                 // the plane barrier also tells every thread whether any wait ran out
@@ -361,8 +374,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 if (tid == 0 && p_item < nitems) issue();   // refill the stage freed two planes ago
 
                 const int q = pz - 1;
-                const i64 *nS = sm.nb[mb_prev][0], *nL = sm.nb[mb_prev][1], *nW = sm.nb[mb_prev][2],
-                          *nM = sm.nb[mb_prev][3];
+                const i64 *nW = sm.nb[mb_prev][2], *nM = sm.nb[mb_prev][3];
                 i64 W[kCells], M[kCells], Fu[kCells];
 #pragma unroll
                 for (int j = 0; j < kCells; ++j) {
@@ -387,25 +399,27 @@ __global__ void __launch_bounds__(kThreads, 2)
                         const double df = (double)fl;
                         gC[j] = fma(df, kx.sc, c);
                         if (!C_ONLY) {
-                            const i64 S6 = (nS[o + 1] + nS[o - 1]) + (nS[o + BX] + nS[o - BX]) + (Xn[j].S + Sm[j]);
-                            const i64 L6 = (nL[o + 1] + nL[o - 1]) + (nL[o + BX] + nL[o - BX]) + (Xn[j].L + Lm[j]);
-                            const i64 So = nS[o], Lo = nL[o];
-                            i64 dS, dL;
-                            fx::eta_inc(kx, Q[j], So, Lo, S6, L6, dS, dL);
-                            Sm[j] = So;
-                            Lm[j] = Lo;
-                            const double ds = (double)dS, dl = (double)dL;
-                            gS[j] = fma(ds, kx.su, sm.raw[st_prev][0][o]);
-                            gL[j] = fma(dl, kx.su, sm.raw[st_prev][1][o]);
+                            const int f = small[j];
+                            const i64 *nB = sm.nb[mb_prev][1 - f];
+                            const i64 b6 = (nB[o + 1] + nB[o - 1]) + (nB[o + BX] + nB[o - BX]) + (sm.nb[mb][1 - f][o] + zb[j]);
+                            const i64 ib = fx::eta_inc(kx, rb[j], nB[o], b6);
+                            const double gb = fx::eta_large(kx, nB[o], ib);
+                            const double *ps = sm.raw[st_prev][f];
+                            const double s6 = (ps[o + 1] + ps[o - 1]) + (ps[o + BX] + ps[o - BX]) + (sm.raw[st][f][o] + zs[j]);
+                            const double ds = fx::eta_inc(kx, rs[j], ps[o], s6);
+                            const double gs = fma(ds, kx.su, ps[o]);
+                            gS[j] = f ? gb : gs;
+                            gL[j] = f ? gs : gb;
                             if (a.partials && vj[j]) {
-                                acc[1] = fma(ds * kx.su, ds * kx.su, acc[1]);
-                                acc[2] = fma(dl * kx.su, dl * kx.su, acc[2]);
+                                const double db = (double)ib, iS = f ? db : ds, iL = f ? ds : db;
+                                acc[1] = fma(iS, iS, acc[1]);
+                                acc[2] = fma(iL, iL, acc[2]);
                             }
                             bad = bad || (vj[j] && !fx::in_box_eta((unsigned)__double2hiint(gS[j]) & 0x7fffffffu,
                                                                    (unsigned)__double2hiint(gL[j]) & 0x7fffffffu));
                         }
                         bad = bad || (vj[j] && !fx::in_box_c((unsigned)__double2hiint(gC[j]), kx.cmax));
-                        if (a.partials && vj[j]) acc[0] = fma(df * kx.sc, df * kx.sc, acc[0]);
+                        if (a.partials && vj[j]) acc[0] = fma(df, df, acc[0]);
                         // a cell outside the domain stores to padding that nothing reads
                         const uint32_t at = vj[j] ? base + (uint32_t)j * (uint32_t)g.P : sink;
                         put_ghost<double, C_ONLY, uint32_t>(out, at, gS[j], gL[j], gC[j]);
@@ -427,17 +441,18 @@ __global__ void __launch_bounds__(kThreads, 2)
                         if (q == 0) put_row(j, per ? (uint32_t)g.nz * (uint32_t)g.PS : (uint32_t)-g.PS);
                         if (q == g.nz - 1) put_row(j, per ? (uint32_t)(-g.nz) * (uint32_t)g.PS : (uint32_t)g.PS);
                     }
-                } else if (!C_ONLY && q == z0 - 1) {
-#pragma unroll
-                    for (int j = 0; j < kCells; ++j) {
-                        Sm[j] = nS[ob + j * BX];
-                        Lm[j] = nL[ob + j * BX];
-                    }
                 }
 #pragma unroll
                 for (int j = 0; j < kCells; ++j) {
                     Fz[j] = Fu[j];
-                    Q[j] = X[j];
+                    if (!C_ONLY) {
+                        const int f = sm_new[j], o = ob + j * BX;
+                        small[j] = f;
+                        rb[j] = f ? X[j].bS : X[j].bL;
+                        rs[j] = f ? X[j].bL : X[j].bS;
+                        zb[j] = sm.nb[mb_prev][1 - f][o];
+                        zs[j] = sm.raw[st_prev][f][o];
+                    }
                 }
                 st_prev = st;
                 mb_prev = mb;
@@ -449,6 +464,10 @@ __global__ void __launch_bounds__(kThreads, 2)
                 ++consumed;
             }
             if (a.partials && !dead) {
+                // (sums of squares in the increments' units until here)
+                acc[0] = acc[0] * kx.sc * kx.sc;
+                acc[1] = acc[1] * kx.su * kx.su;
+                acc[2] = acc[2] * kx.su * kx.su;
                 put_sums(acc, a.partials, item);
                 acc[0] = acc[1] = acc[2] = 0;
             }
