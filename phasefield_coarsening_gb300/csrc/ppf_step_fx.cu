@@ -79,60 +79,105 @@ __device__ __forceinline__ void mu_m(const Coef<double> &k, double eS, double eL
     M = fma(h, k.Mt1, k.Mt0);
 }
 
-// One cell of a step whose input has left the box, in float64 and straight
-// from global memory, with the general kernel's operations in its order.
-// Rare (a state leaves the box between two host calls at most once), so
-// neither tiled nor inlined.
+// One item of a step whose input has left the box, in float64 with the
+// general kernel's operations in its order: mu and M' once per cell, in the
+// ring of three shared planes (`mm`, next slot `mb`), everything else straight
+// from global memory.  A domain that leaves the box stays on this path until
+// its next upload, so it has to keep the general kernel's rate; FP64 operations
+// bound both: 2.66 ms at 256^3, 0.28 ms at 96 x 128 x 128 (general 2.22 and 0.24;
+// cell by cell, with mu and M' of all seven cells, 4.37 and 0.44).
 template <bool C_ONLY>
-__device__ __noinline__ void slow_cell(const Coef<double> &k, const Geom &g, const Fields<const double> &in,
-                                       const Fields<double> &out, int x, int y, int z, double *inc) {
-    const int64_t j = g.at(x, y, z);
-    const int64_t nb[6] = {j + g.PS, j - g.PS, j + g.P, j - g.P, j + 1, j - 1};
-    const double eS = in.eS[j], eL = in.eL[j], c = in.c[j];
-    double mu, M, rs;
-    mu_m(k, eS, eL, c, mu, M, rs);
-    double fl = 0, S6 = 0, L6 = 0;
-    for (int q = 0; q < 6; ++q) {
-        double mn, Mn, r;
-        const double sn = in.eS[nb[q]], ln = in.eL[nb[q]];
-        mu_m(k, sn, ln, in.c[nb[q]], mn, Mn, r);
-        fl = q ? fma(Mn + M, mn - mu, fl) : __dmul_rn(Mn + M, mn - mu);
-        // z+, z-, then y+, y-, x+, x-, each added in turn
-        S6 = q ? __dadd_rn(S6, sn) : sn;
-        L6 = q ? __dadd_rn(L6, ln) : ln;
-    }
-    const double cn = __dadd_rn(c, fl);
-    double Sn = eS, Ln = eL;
-    inc[0] += fl * fl;
-    if (!C_ONLY) {
-        const double D = fma(mu, -k.q1, k.dC);
-        const double dmu = __dmul_rn(__dmul_rn(__dmul_rn(k.dm2, __dmul_rn(eS, eL)), __dmul_rn(rs, rs)), D);
-        const double S2 = __dmul_rn(eS, eS), L2 = __dmul_rn(eL, eL);
-        const double lapS = fma(-6.0, eS, S6), lapL = fma(-6.0, eL, L6);
-        const double dS = fma(__dmul_rn(k.mt, eS), fma(k.tg, L2, __dadd_rn(S2, -1.0)),
-                              fma(-k.kt, lapS, __dmul_rn(eL, dmu)));
-        const double dL = fma(__dmul_rn(k.mt, eL), fma(k.tg, S2, __dadd_rn(L2, -1.0)),
-                              fma(-k.kt, lapL, __dadd_rn(0.0, -__dmul_rn(eS, dmu))));
-        Sn = __dadd_rn(eS, dS);
-        Ln = __dadd_rn(eL, dL);
-        inc[1] += dS * dS;
-        inc[2] += dL * dL;
-    }
-    auto put = [&](int64_t a) {
-        if (!C_ONLY) {
-            out.eS[a] = Sn;
-            out.eL[a] = Ln;
+__device__ __noinline__ void slow_item(const Coef<double> &k, const Geom &g, const Fields<const double> &in,
+                                       const Fields<double> &out, const Item &it, double (*mm)[2][G::BOX], int &mb,
+                                       double *inc) {
+    constexpr int TX = G::TX, TY = G::TY, XH = G::XH, BX = G::BX;
+    const int tid = threadIdx.x, tx = tid & 31, ty0 = (tid >> 5) * kCells;
+    const int x = it.bx * TX + tx, y = it.by * TY + ty0, ob = (ty0 + 1) * BX + tx + XH;
+    // this thread's ring cell, tile coordinates (the last threads: the rows -1
+    // and TY, then the columns -1 and TX)
+    const int rt = tid - (kThreads - G::RING);
+    const int rx = rt < 2 * TX ? rt % TX : rt < 2 * TX + TY ? -1 : TX;
+    const int ry = rt < TX ? -1 : rt < 2 * TX ? TY : (rt - 2 * TX) % TY;
+    const bool ring = rt >= 0 && it.bx * TX + rx <= g.nx && it.by * TY + ry <= g.ny;
+    double mu[kCells], M[kCells], rs[kCells], mq[kCells], Mq[kCells], rq[kCells], mz[kCells], Mz[kCells];
+#pragma unroll
+    for (int j = 0; j < kCells; ++j) mu[j] = M[j] = rs[j] = mq[j] = Mq[j] = rq[j] = mz[j] = Mz[j] = 0;
+    int prev = mb;
+    for (int pz = it.z0 - 1; pz <= it.z1; ++pz) {
+#pragma unroll
+        for (int j = 0; j < kCells; ++j)
+            if (x <= g.nx && y + j <= g.ny) {      // (with the ghosts that cells of this tile see)
+                const int64_t i = g.at(x, y + j, pz);
+                mu_m(k, in.eS[i], in.eL[i], in.c[i], mu[j], M[j], rs[j]);
+                mm[mb][0][ob + j * BX] = mu[j];
+                mm[mb][1][ob + j * BX] = M[j];
+            }
+        if (ring) {
+            const int64_t i = g.at(it.bx * TX + rx, it.by * TY + ry, pz);
+            const int o = (ry + 1) * BX + rx + XH;
+            double r;
+            mu_m(k, in.eS[i], in.eL[i], in.c[i], mm[mb][0][o], mm[mb][1][o], r);
         }
-        out.c[a] = cn;
-    };
-    put(j);
-    const bool per = g.bc == 0;
-    if (x == 0) put(per ? j + g.nx : j - 1);
-    if (x == g.nx - 1) put(per ? j - g.nx : j + 1);
-    if (y == 0) put(per ? j + g.ny * g.P : j - g.P);
-    if (y == g.ny - 1) put(per ? j - g.ny * g.P : j + g.P);
-    if (z == 0) put(per ? j + g.nz * g.PS : j - g.PS);
-    if (z == g.nz - 1) put(per ? j - g.nz * g.PS : j + g.PS);
+        __syncthreads();
+        const int q = pz - 1;
+#pragma unroll
+        for (int j = 0; j < kCells; ++j) {
+            if (q < it.z0 || x >= g.nx || y + j >= g.ny) continue;
+            const int64_t i = g.at(x, y + j, q);
+            const int o = ob + j * BX;
+            const double *pm = mm[prev][0], *pM = mm[prev][1];
+            double fl = __dmul_rn(M[j] + Mq[j], mu[j] - mq[j]);
+            fl = fma(Mz[j] + Mq[j], mz[j] - mq[j], fl);
+            fl = fma(pM[o + BX] + Mq[j], pm[o + BX] - mq[j], fl);
+            fl = fma(pM[o - BX] + Mq[j], pm[o - BX] - mq[j], fl);
+            fl = fma(pM[o + 1] + Mq[j], pm[o + 1] - mq[j], fl);
+            fl = fma(pM[o - 1] + Mq[j], pm[o - 1] - mq[j], fl);
+            const double eS = in.eS[i], eL = in.eL[i], cn = __dadd_rn(in.c[i], fl);
+            double Sn = eS, Ln = eL;
+            inc[0] += fl * fl;
+            if (!C_ONLY) {
+                // z+, z-, then y+, y-, x+, x-, each added in turn
+                auto six = [&](const double *f) {
+                    double s = __dadd_rn(f[i + g.PS], f[i - g.PS]);
+                    s = __dadd_rn(s, f[i + g.P]);
+                    s = __dadd_rn(s, f[i - g.P]);
+                    s = __dadd_rn(s, f[i + 1]);
+                    return __dadd_rn(s, f[i - 1]);
+                };
+                const double D = fma(mq[j], -k.q1, k.dC);
+                const double dmu = __dmul_rn(__dmul_rn(__dmul_rn(k.dm2, __dmul_rn(eS, eL)), __dmul_rn(rq[j], rq[j])), D);
+                const double S2 = __dmul_rn(eS, eS), L2 = __dmul_rn(eL, eL);
+                const double lapS = fma(-6.0, eS, six(in.eS)), lapL = fma(-6.0, eL, six(in.eL));
+                const double dS = fma(__dmul_rn(k.mt, eS), fma(k.tg, L2, __dadd_rn(S2, -1.0)),
+                                      fma(-k.kt, lapS, __dmul_rn(eL, dmu)));
+                const double dL = fma(__dmul_rn(k.mt, eL), fma(k.tg, S2, __dadd_rn(L2, -1.0)),
+                                      fma(-k.kt, lapL, __dadd_rn(0.0, -__dmul_rn(eS, dmu))));
+                Sn = __dadd_rn(eS, dS);
+                Ln = __dadd_rn(eL, dL);
+                inc[1] += dS * dS;
+                inc[2] += dL * dL;
+            }
+            auto put = [&](int64_t a) { put_ghost<double, C_ONLY>(out, a, Sn, Ln, cn); };
+            put(i);
+            const bool per = g.bc == 0;
+            if (x == 0) put(per ? i + g.nx : i - 1);
+            if (x == g.nx - 1) put(per ? i - g.nx : i + 1);
+            if (y + j == 0) put(per ? i + g.ny * g.P : i - g.P);
+            if (y + j == g.ny - 1) put(per ? i - g.ny * g.P : i + g.P);
+            if (q == 0) put(per ? i + g.nz * g.PS : i - g.PS);
+            if (q == g.nz - 1) put(per ? i - g.nz * g.PS : i + g.PS);
+        }
+#pragma unroll
+        for (int j = 0; j < kCells; ++j) {
+            mz[j] = mq[j];
+            Mz[j] = Mq[j];
+            mq[j] = mu[j];
+            Mq[j] = M[j];
+            rq[j] = rs[j];
+        }
+        prev = mb;
+        mb = mb + 1 == 3 ? 0 : mb + 1;
+    }
 }
 
 // which of a cell's fields is the smaller one: 0 etaS, 1 etaL
@@ -196,6 +241,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
     if (any) {
         // their items in float64, and their outputs stay marked
+        int mb = 0;
         for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
             const Item it = fx_item<MULTI>(a, item);
             if (MULTI && !left_box(it.dom)) continue;
@@ -210,11 +256,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                        (double *)d.fld[1 - a.parity][2]};
             }
             double inc[3] = {0, 0, 0};
-            for (int z = it.z0; z < it.z1; ++z)
-                for (int j = 0; j < kCells; ++j) {
-                    const int x = it.bx * TX + tx, y = it.by * TY + ty0 + j;
-                    if (x < g.nx && y < g.ny) slow_cell<C_ONLY>(a.k, g, in, out, x, y, z, inc);
-                }
+            slow_item<C_ONLY>(a.k, g, in, out, it, reinterpret_cast<double(*)[2][G::BOX]>(sm.nb), mb, inc);
             if (tid == 0) (MULTI ? a.table[it.dom].box : a.box)[1 - a.parity] = 1;
             if (a.partials) put_sums(inc, a.partials, item);
         }

@@ -1,0 +1,58 @@
+"""FP64 states outside the fixed-point step's box: they step in float64 inside
+the same kernel, at the general kernel's rate, and nothing that shares a
+launch, a stream or an autotuner with them changes another domain's bits."""
+import time
+
+import numpy as np
+import pytest
+
+import phasefield_coarsening_gb300 as ppf
+from helpers import smooth_state
+from test_gpu_fx import GROW, growing, params
+
+pytestmark = pytest.mark.gpu
+
+
+def ms_per_step(obj, n=20):
+    best = 1e9
+    for _ in range(4):
+        obj.sync()
+        t = time.perf_counter()
+        obj.step(n)
+        obj.sync()
+        best = min(best, (time.perf_counter() - t) * 1e3 / n)
+    return best
+
+
+def test_states_that_left_the_box_step_at_the_general_rate():
+    """A domain that leaves the box during a run, in an ensemble, as slabs and
+    alone in one long call, against a state known to be outside from its upload
+    on: the same arithmetic, so a step may not take half as long again."""
+    shape = (96, 128, 128)
+    st = growing(shape)
+    with ppf.Simulation(shape, params(GROW)) as a, ppf.Ensemble([shape], params(GROW), precision="f64") as e, \
+            ppf.Slabs(shape, 2, params(GROW)) as t, ppf.Simulation(shape, params(GROW)) as b:
+        for s in (a, t):
+            s.upload(*st)
+        e.upload_all([st])
+        n = 8
+        while True:
+            a.step(n)
+            out = a.download()
+            if out[0].max() > 1.9:
+                break
+            t.step(n)
+            e.step(n)
+        t.step(n)
+        e.step(n)
+        b.upload(*out)                   # outside from the start
+        general = ms_per_step(b)
+        assert ms_per_step(e) <= 1.5 * general
+        assert ms_per_step(t) <= 1.5 * general
+        a.upload(*st)
+        a.step(1)
+        a.sync()
+        t0 = time.perf_counter()
+        a.step(2000)                     # one call, outside for most of it
+        a.sync()
+        assert (time.perf_counter() - t0) * 1e3 / 2000 <= 1.5 * general
