@@ -256,6 +256,7 @@ extern "C" int ppf_set_stream(ppf_ctx *c, void *stream) {
 static int pack_from(ppf_ctx *c, const double *const src[3]) {
     c->cur_eta = 0;
     c->cur_c = 0;
+    c->left_box = 0;
     // (slabs of one domain share the first one's words, cleared with its upload)
     if (c->fx_ok && !c->shared_box) CU(cudaMemsetAsync(c->dbox, 0, 2 * sizeof(int), c->stream));
     const BoxCheck box = {c->fx_ok ? c->dbox : nullptr, c->kx.cmax};
@@ -647,7 +648,7 @@ extern "C" int ppf_autotune(ppf_ctx *c, int trial_steps, ppf_tune *best) {
         for (int sp = 0; sp < nsplit && rc == PPF_OK; ++sp)
         for (int sd = 1; sd >= (tl == 0 ? 0 : 1) && rc == PPF_OK; --sd)
         for (int pdl = 1; pdl >= (tl == 0 ? 0 : 1) && rc == PPF_OK; --pdl)
-        for (int r = 0; r < 2 && rc == PPF_OK; ++r)
+        for (int r = 0; r < (c->fx_ok ? 1 : 2) && rc == PPF_OK; ++r)    // (the fixed-point kernel has one form)
             for (int i = 0; i < nzc && rc == PPF_OK; ++i) {
                 StepTune t = keep;
                 t.tile = tl;
@@ -695,10 +696,7 @@ extern "C" int ppf_autotune(ppf_ctx *c, int trial_steps, ppf_tune *best) {
     c->tune = rc == PPF_OK ? win : keep;
     int rc2 = do_pack(c);           // restore the state saved above
     c->steps = steps0;
-    if (rc2 == PPF_OK) {
-        cudaError_t e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) rc2 = seterr(PPF_ECUDA, "restore failed: %s", cudaGetErrorString(e));
-    }
+    if (rc2 == PPF_OK) rc2 = read_box(c);
     if (rc) return rc;
     if (rc2) return rc2;
     if (best) {

@@ -56,3 +56,23 @@ def test_states_that_left_the_box_step_at_the_general_rate():
         a.step(2000)                     # one call, outside for most of it
         a.sync()
         assert (time.perf_counter() - t0) * 1e3 / 2000 <= 1.5 * general
+
+
+def test_autotuning_leaves_the_state_and_its_arithmetic_alone():
+    """Trials that leave the box do not count for the restored state, which is in
+    it: bit for bit the steps of a context that was never tuned."""
+    shape = (6, 20, 40)
+    st = growing(shape)
+    with ppf.Simulation(shape, params(GROW)) as a, ppf.Simulation(shape, params(GROW)) as b, \
+            ppf.Simulation(shape, params(GROW)) as c:
+        for s in (a, b, c):
+            s.upload(*st)
+        c.step(400)
+        assert not c.download()[0].max() < 1.9       # a trial of so many steps leaves the box
+        a.autotune(400)
+        for n in (1, 2, 5):
+            a.step(n)
+            b.step(n)
+            assert a.reduce()["steps"] == b.reduce()["steps"]
+            for x, y in zip(a.download(), b.download()):
+                assert np.array_equal(x, y)
