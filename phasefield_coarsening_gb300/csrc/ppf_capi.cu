@@ -323,17 +323,26 @@ static bool direct_io(ppf_ctx *c, const double *const p[3]) {
     return true;
 }
 
+// From now on the context's steps are launched in float64, until its next
+// upload.  Those steps do not keep the box words, so both are set: a
+// fixed-point launch on this state computes it in float64 too.
+static int set_left_box(ppf_ctx *c) {
+    c->left_box = 1;
+    CU(cudaMemsetAsync(c->dbox, 1, 2 * sizeof(int), c->stream));
+    return PPF_OK;
+}
+
 // Waits for the stream, and learns whether the uploaded state lies outside
-// the fixed-point step's box (its steps are then launched in float64).
+// the fixed-point step's box.
 static int read_box(ppf_ctx *c) {
     int h = 0;
     if (c->fx_ok) CU(cudaMemcpyAsync(&h, c->dbox, sizeof h, cudaMemcpyDeviceToHost, c->stream));
     CU(cudaStreamSynchronize(c->stream));
-    c->left_box = h != 0;
-    return PPF_OK;
+    return h ? set_left_box(c) : PPF_OK;
 }
 
 int recheck_box(ppf_ctx *c) {
+    c->left_box = 0;
     if (c->fx_ok) {
         CU(cudaMemsetAsync(c->dbox, 0, 2 * sizeof(int), c->stream));
         CU(launch_box_check(c->g, cst(fd(c, 0, 0)), BoxCheck{c->dbox, c->kx.cmax}, c->stream));
@@ -401,7 +410,10 @@ extern "C" int ppf_download_device(ppf_ctx *c, double *etaS, double *etaL, doubl
 // pairs, the context's own box words.  Clears a set error word; PPF_ETIMEOUT
 // when a kernel's bounded wait ran out since the last check.
 static int check_words(ppf_ctx *c, const int *w) {
-    if (c->fx_ok && c->dbox == own_box(c) && w[8 + c->cur_c]) c->left_box = 1;
+    if (c->fx_ok && c->dbox == own_box(c) && w[8 + c->cur_c] && !c->left_box) {
+        const int rc = set_left_box(c);
+        if (rc) return rc;
+    }
     if (w[0]) {
         // the error word, and the scheduler pairs that an abandoned step may leave set
         CU(cudaMemsetAsync(c->derr, 0, 8 * sizeof(int), c->stream));

@@ -46,7 +46,8 @@ struct ppf_ctx {
     int eqA;              // AS == AL: the mu reciprocal is a constant
     ppf::fx::FxCoef kx;   // FP64: coefficients of the fixed-point step
     int fx_ok;            // FP64: the parameters and the grid fit the fixed-point step
-    int left_box;         // the host knows that the state has left the fixed-point step's box
+    int left_box;         // the host knows that the state has left the fixed-point step's box, and
+                          // has set both box words
     int shared_box;       // dbox belongs to another slab of the same domain
     int *dbox;            // box words of the two buffers (launch_step_fx): the context's own, behind the
                           // scheduler words, or shared with the slabs of one domain / in the ensemble's array

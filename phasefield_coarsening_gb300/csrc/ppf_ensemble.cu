@@ -89,7 +89,7 @@ struct ppf_ensemble {
     int64_t steps;
     cudaStream_t stream;
     cudaGraphExec_t graph;       // kGraphSteps plain steps, starting and ending at parity 0
-    int graph_ok, graph_fx;      // graph_fx: of fixed-point steps
+    int graph_ok;
     int num_sms;
 };
 
@@ -172,13 +172,10 @@ static int build_table(ppf_ensemble *e) {
     return PPF_OK;
 }
 
-// whether the next step runs in fixed-point arithmetic (the kernel computes
-// domains that leave the box later in float64)
-static bool fx_ensemble(const ppf_ensemble *e) {
-    for (const ppf_ctx *c : e->dom)
-        if (!fx_step(c)) return false;
-    return true;
-}
+// Whether the ensemble steps with the fixed-point kernel: by its parameters
+// alone.  That kernel keeps every domain's box words and computes the marked
+// ones in float64, so a domain's bits do not depend on the others.
+static bool fx_ensemble(const ppf_ensemble *e) { return e->dom[0]->fx_ok != 0; }
 
 static int launch_one(ppf_ensemble *e, bool stats) {
     const int inj = 0;
@@ -203,10 +200,7 @@ static int launch_one(ppf_ensemble *e, bool stats) {
 }
 
 static int ensure_graph(ppf_ensemble *e) {
-    if (e->graph_ok && e->graph_fx == (int)fx_ensemble(e)) return PPF_OK;
-    if (e->graph_ok) cudaGraphExecDestroy(e->graph);
-    e->graph_ok = 0;
-    e->graph_fx = fx_ensemble(e);
+    if (e->graph_ok) return PPF_OK;
     cudaGraph_t g;
     const int p0 = e->parity;
     e->parity = 0;
@@ -383,12 +377,10 @@ extern "C" int ppf_ensemble_upload_all(ppf_ensemble *e, const double *const *eta
         x->cur_eta = x->cur_c = 0;
         x->uploaded = 1;
         x->steps = 0;
+        x->left_box = 0;
     }
     e->parity = 0;
-    std::vector<int> box((size_t)e->n * 2);
-    ECU(cudaMemcpyAsync(box.data(), e->boxes, box.size() * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
     ECU(cudaStreamSynchronize(e->stream));
-    for (int d = 0; d < e->n; ++d) e->dom[(size_t)d]->left_box = box[2 * (size_t)d] != 0;
     return PPF_OK;
 }
 

@@ -166,6 +166,7 @@ extern "C" int ppf_slabs_upload(ppf_slabs *s, const double *etaS, const double *
     SCU(cudaMemcpyAsync(&h, s->ctx[0]->dbox, sizeof h, cudaMemcpyDeviceToHost, s->stream));
     SCU(cudaStreamSynchronize(s->stream));
     for (ppf_ctx *c : s->ctx) c->left_box = h != 0;
+    if (h) SCU(cudaMemsetAsync(s->ctx[0]->dbox, 1, 2 * sizeof(int), s->stream));
     return PPF_OK;
 }
 
@@ -183,6 +184,8 @@ extern "C" int ppf_slabs_download(ppf_slabs *s, double *etaS, double *etaL, doub
 extern "C" int ppf_slabs_step(ppf_slabs *s, int64_t nsteps) {
     if (!s) return err_(PPF_EINVAL, "null slabs");
     if (nsteps < 0) return err_(PPF_EINVAL, "negative step count");
+    // (the first slab, whose words they are, learns that the state left the box)
+    for (ppf_ctx *c : s->ctx) c->left_box = s->ctx[0]->left_box;
     for (int64_t t = 0; t < nsteps; ++t) {
         for (ppf_ctx *c : s->ctx) {
             int rc = ppf_step(c, 1);

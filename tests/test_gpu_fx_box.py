@@ -76,3 +76,60 @@ def test_autotuning_leaves_the_state_and_its_arithmetic_alone():
             assert a.reduce()["steps"] == b.reduce()["steps"]
             for x, y in zip(a.download(), b.download()):
                 assert np.array_equal(x, y)
+
+
+def test_ensemble_domains_do_not_depend_on_one_another():
+    """A domain that leaves the box while another one is outside from its upload
+    on, over an even number of steps; then that one is replaced by a state
+    inside.  Every domain has the bits of a context of its own throughout."""
+    shape = (6, 20, 40)
+    st = growing(shape)
+    out = [x.copy() for x in growing(shape, seed=1)]
+    out[0][2, 3, 4] = 1.8
+    inside = smooth_state(shape, seed=2)
+    with ppf.Ensemble([shape, shape], params(GROW), precision="f64") as e, ppf.Simulation(shape, params(GROW)) as a, \
+            ppf.Simulation(shape, params(GROW)) as b:
+        e.upload_all([out, st])
+        a.upload(*out)
+        b.upload(*st)
+
+        def same(s, d):
+            return all(np.array_equal(x, y) for x, y in zip(s.download(), e.download(d)))
+
+        n = 0
+        while n < 100 or not b.download()[0].max() > 1.9:
+            for s in (e, a, b):
+                s.step(20)
+            n += 20
+            assert n <= 400
+        assert same(a, 0) and same(b, 1)
+        e.upload(0, *inside)
+        a.upload(*inside)
+        for n in (2, 5, 18):
+            for s in (e, a, b):
+                s.step(n)
+            assert same(a, 0) and same(b, 1)
+        ra, rb = e.reduce(0), e.reduce(1)
+        for r, s in ((ra, a), (rb, b)):
+            q = s.reduce()
+            for k in ("sum_dc2", "sum_detaS2", "sum_detaL2"):
+                assert abs(r[k] - q[k]) <= 1e-12 * abs(q[k])
+
+
+def test_slabs_that_left_the_box_and_an_upload_back():
+    """Slabs learn together that the state has left the box, and that an upload
+    brought it back."""
+    shape = (9, 20, 40)
+    st = growing(shape, seed=4)
+    with ppf.Slabs(shape, 3, params(GROW)) as t, ppf.Simulation(shape, params(GROW)) as s:
+        for back in (0, 1):
+            t.upload(*st)
+            s.upload(*st)
+            for n in (100, 90, 1, 2):
+                t.step(n)
+                s.step(n)
+                t.sync()
+                s.sync()
+                for x, y in zip(s.download(), t.download()):
+                    assert np.array_equal(x, y)
+                assert t.reduce()["steps"] == s.reduce()["steps"]
