@@ -234,7 +234,7 @@ PPF_FX bool in_box_eta(unsigned hS, unsigned hL) {
 PPF_FX bool in_box_c(unsigned hC, unsigned cmax) { return (hC & 0x7fffffffu) < cmax; }
 
 // The coefficients for a parameter set; false when they do not fit (AS !=
-// AL, a time step above the solute equation's explicit limit, phase-field
+// AL, a liquid minimum below 1/16 of the scale of c, a time step above the solute equation's explicit limit, phase-field
 // rates so large that their increments would lose resolution): then the
 // step stays in float64 arithmetic.  `A` .. `kt` as in Coef<double>.
 inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0, double Mt1, double dC, double q1,
@@ -250,6 +250,10 @@ inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0
         std::frexp(cmag, &ec);                 // cmag < 2^ec
     }
     if (ec < -500 || ec > 500) return false;
+    // c - cL0 has an absolute error of 2^-54 |cL0| in float64 for any |c| below
+    // cL0; with a liquid minimum near zero it has none, and small values of c would
+    // lose bits on the fixed scale
+    if (std::fabs(cL0) < std::ldexp(1.0, ec - 4)) return false;
     // (products of coefficients in extended precision: rounded once, here)
     typedef long double ld;
     const ld m0 = (ld)AS * Mt0, m1 = (ld)AS * Mt1;

@@ -90,3 +90,35 @@ def test_small_values_step_as_in_float64(floor, bc):
             size = np.maximum.reduce([size, np.roll(size, 1, ax), np.roll(size, -1, ax)])
         assert (np.abs(a - b) <= 100 * 2.0 ** -53 * size).all(), (np.abs(a - b) / size).max()
     np.testing.assert_allclose([g["sum_dc2"], g["sum_detaS2"], g["sum_detaL2"]], ref[3], rtol=1e-10)
+
+
+# a liquid minimum at or near zero: float64 keeps the relative precision of a
+# dilute composition
+DILUTE = dict(cS0=0.5, cSeq=0.02, cLeq=0.5)
+
+
+@pytest.mark.parametrize("cL0", [0.0, 1e-12, 1e-3, -0.02])
+def test_dilute_liquids_are_left_to_float64(host, cL0):
+    shape = (2, 2, 2)
+    i = np.arange(8).reshape(shape)
+    nb = np.stack([np.roll(i, -s, a).ravel() for a in (0, 1, 2) for s in (1, -1)], 1).astype(np.int32).copy()
+    a, err = np.ones(24) * 0.5, np.zeros(32)
+    for c, fits in ((cL0, 0), (0.3 + cL0, 1)):
+        k = coef(ppf.params_default(dt=DT08, cL0=c, **DILUTE))
+        assert host.fx_tail_errors(8, *[v.ctypes.data_as(ctypes.c_void_p) for v in (nb, k, a, err)]) == fits
+
+
+@pytest.mark.gpu
+def test_dilute_compositions_step_as_in_float64():
+    """Compositions of 1e-9 beside a liquid minimum of 0: sums of six products of
+    relative error 2^-53 and their neighbours' over five steps, 1e-13 of the value."""
+    shape = (6, 18, 40)
+    r = np.random.default_rng(5)
+    p = dict(dt=DT08, cL0=0.0, **DILUTE)
+    st = np.zeros(shape), np.ones(shape), 1e-9 * (1 + 0.3 * r.random(shape))
+    with ppf.Simulation(shape, ppf.params_default(**p)) as s:
+        s.upload(*st)
+        s.step(5)
+        got = s.download()
+    ref = oracle.run(*st, 5, bc=0, params=oracle.reference_params(**p))
+    assert np.abs(got[2] / ref[2] - 1).max() <= 1e-13
