@@ -203,18 +203,30 @@ PPF_FX double eta_inc(const FxCoef &k, i64 rate, double v, double six) {
     return fma(k.kb, six, (double)(rate - k.nk6) * v);
 }
 
-// A cell's terms of the observables: c @59 and w^2 @59 (in units of 2^ec and
-// 2^(2 ec)), hS @61 and the well energy f0 @53 (its constant 1/4 included).
-PPF_FX void observe(const FxCoef &k, double eS, double eL, double c, int cbias, i64 &C, i64 &h, i64 &w2, i64 &f0) {
+// v 2^-60 as a double, for 2^52 <= v < 2^63, without FP64 operations
+PPF_FX double unit60(i64 v) {
+#ifdef __CUDA_ARCH__
+    const int z = __clzll(v);
+    const unsigned long long m = (unsigned long long)v << z;
+    // (a carry out of the mantissa goes on into the exponent)
+    return __longlong_as_double((i64)(((unsigned long long)(1025 - z) << 52) + (m >> 11) + ((m >> 10) & 1)));
+#else
+    return std::ldexp((double)v, -60);
+#endif
+}
+
+// A cell's terms of the observables: c @59 and w @59 (in units of 2^ec), the
+// reciprocal of etaS^2 + etaL^2 @60 and the well energy f0 @57 (its constant 1/4
+// included).
+PPF_FX void observe(const FxCoef &k, double eS, double eL, double c, int cbias, i64 &C, i64 &W, i64 &R, i64 &f0) {
     const i64 S = to_fx(eS, kEtaBias), L = to_fx(eL, kEtaBias);
     const i64 S2 = mulx<2>(S, S), L2 = mulx<2>(L, L);                                                // @60
+    R = recip(S2 + L2);
     C = to_fx(c, cbias);
-    h = mulx<5>(S2, recip(S2 + L2));
-    const i64 W = C - k.cL0 + mulq(k.dc0, h);
-    w2 = mulx<5>(W, W);
+    W = C - k.cL0 + mulq(k.dc0, mulx<5>(S2, R));
     // S2 (S2/4 - 1/2 + gamma L2) + L2 (L2/4 - 1/2) + 1/4, the factors @57
     const i64 xS = (S2 >> 5) - (1ll << 56) + mulq(k.g, L2), xL = (L2 >> 5) - (1ll << 56);
-    f0 = mulq(S2, xS) + mulq(L2, xL) + (1ll << 51);
+    f0 = mulx<4>(S2, xS) + mulx<4>(L2, xL) + (1ll << 55);
 }
 
 // Whether a state cell lies in the box, from the high words alone (a margin

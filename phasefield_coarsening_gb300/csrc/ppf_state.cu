@@ -402,20 +402,43 @@ struct FxSum {
     }
 };
 
-// Cells of an FP64 state in fixed-point arithmetic (ppf_fx.h), but for the
-// gradient's differences and squares: those twelve are what is left of about
-// 32 operations a cell for the FP64 pipe, which runs beside the integer
-// pipes.  256^3: 0.49 ms; 1.12 ms with all of it in FP64.
+// Squares of fixed-point numbers below 3.5 2^59, taken to 2^4 units: exact for
+// 2^14 of them (128 bits).
+struct FxSquares {
+    unsigned long long lo = 0, hi = 0;
+    __device__ __forceinline__ void add(fx::i64 v) {
+        const fx::i64 a = (v + 8) >> 4;
+        const unsigned long long p = (unsigned long long)a * (unsigned long long)a;
+        lo += p;
+        hi += (unsigned long long)__mul64hi(a, a) + (lo < p);
+    }
+    __device__ __forceinline__ double get(double scale) const {
+        return scale * ((double)hi * 18446744073709551616.0 + (double)lo) * scale;
+    }
+};
+
+// Cells of an FP64 state in fixed-point arithmetic (ppf_fx.h) as far as its
+// absolute errors are below those of float64: w and the sum of its squares
+// (exact, w to 2^-56), the reciprocal, the well energy, and the solute mass where c
+// has no bits below 2^-59.  What float64 holds relative to its own size stays
+// float64: smaller values of c, the solid fraction of states that have little
+// of it, the gradient's differences and squares.  Fourteen of about 32
+// operations a cell are left for the FP64 pipe, which runs beside the integer
+// pipes.  256^3: 0.58 ms; 1.12 ms with all of it in FP64, 0.49 with all but the
+// gradient in fixed point.
 struct ObsFx {
-    FxSum mass, h, w, f0;
-    double gr = 0;
+    FxSum f0, c;
+    FxSquares w;
+    double mass = 0, h = 0, gr = 0;
     __device__ __forceinline__ void cell(const fx::FxCoef &k, int cbias, double eS, double eL, double c, double sx,
                                          double lx, double sy, double ly, double sz, double lz) {
-        fx::i64 C, hh, w2, f;
-        fx::observe(k, eS, eL, c, cbias, C, hh, w2, f);
-        mass.add(C);
-        h.add(hh);
-        w.add(w2);
+        fx::i64 C, W, R, f;
+        fx::observe(k, eS, eL, c, cbias, C, W, R, f);
+        // cmax is the high word of 2^(ec + 1)
+        if (((unsigned)__double2hiint(c) & 0x7fffffffu) >= k.cmax - (7u << 20)) this->c.add(C);
+        else mass += c;
+        h = fma(eS * eS, fx::unit60(R), h);
+        w.add(W);
         f0.add(f);
         double d = sx - eS;
         gr = fma(d, d, gr);
@@ -538,10 +561,10 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double v[4] = {acc.mass.get(), acc.h.get(), acc.w.get(), acc.f.get()};
     if constexpr (FX) {
-        v[0] += ax.mass.get(kx.sc);
-        v[1] += ax.h.get(4.3368086899420177e-19);                                  // 2^-61
-        v[2] += ax.w.get(kx.sc) * (kx.sc * 5.7646075230342349e+17);                // 2^(2 ec - 59)
-        v[3] += fma(k.kg, ax.gr, k.m * ax.f0.get(1.1102230246251565e-16));         // 2^-53
+        v[0] += ax.c.get(kx.sc) + ax.mass;
+        v[1] += ax.h;
+        v[2] += ax.w.get(16.0 * kx.sc);
+        v[3] += fma(k.kg, ax.gr, k.m * ax.f0.get(6.9388939039072284e-18));         // 2^-57
     }
     const bool up = lane & 16, up2 = lane & 8;
     double a0 = (up ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, up ? v[0] : v[2], 16);

@@ -1,0 +1,31 @@
+"""Observables of states whose terms are small, huge or differ by orders of
+magnitude: every sum keeps the precision of its own terms."""
+import numpy as np
+import pytest
+
+import phasefield_coarsening_gb300 as ppf
+
+pytestmark = pytest.mark.gpu
+
+DT08 = 0.8 / (6.0 * 1e-14)
+SHAPES = [(6, 18, 40), (5, 7, 33)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_fp64_sums_of_small_terms(shape):
+    """A dilute liquid with next to no solid: mass and solid relative to
+    themselves (a few roundings of 2^-53 a term and a sum of about 5000), and the
+    chemical energy of compositions 1e-6 from the minimum (w to 2^-54 of c)."""
+    r = np.random.default_rng(1)
+    S, L = 1e-9 * (1 + r.random(shape)), np.ones(shape)
+    c = 1e-10 * (1 + r.random(shape))
+    p = ppf.params_default(dt=DT08, AS=300.0, AL=300.0, CS=0.0, CL=0.0)
+    with ppf.Simulation(shape, p) as s:
+        s.upload(S, L, c)
+        g = s.reduce()
+        assert abs(g["mass"] / c.sum() - 1) <= 1e-13
+        assert abs(g["solid"] / (S * S / (S * S + L * L)).sum() - 1) <= 1e-13
+        c = 0.978 + 1e-6 * (1 + r.random(shape))
+        s.upload(np.zeros(shape), L, c)
+        w = c.astype(np.longdouble) - np.longdouble(0.978)
+        assert abs(s.reduce()["free_energy"] / float((150 * w * w).sum()) - 1) <= 1e-10
