@@ -307,7 +307,7 @@ cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[
 // accumulation per cell is what bounded the FP32 form (one conversion and
 // one addition per cell, each 1/64 of the FP32 rate); the FP64 state's form
 // in FP64 arithmetic is bound by the FP64 pipe, so it has few operations
-// (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 54 us (186 us with
+// (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 56 us (186 us with
 // one cell per thread and FP64 sums of the solute mass); 64^3: 7 us (33 us).
 
 // 1/x of a pair: the hardware's estimate (about 1 ulp) and a Newton step
@@ -380,12 +380,13 @@ struct ObsAcc {
         gr = fma2(d, d, gr);
         d = lz - eL;
         gr = fma2(d, d, gr);
-        const V2<T> ff = fma2(splat(k.kg), gr, splat(k.m) * f0);
         auto in = [&](V2<T> v) { return V2<T>(nv > 0 ? v.x() : T(0), nv > 1 ? v.y() : T(0)); };
         mass.add(in(c));
         h.add(in(hh));
         w.add(in(ch));
-        f.add(in(ff));
+        // (each on its own: they can differ by orders of magnitude)
+        f.add(in(splat(k.m) * f0));
+        f.add(in(splat(k.kg) * gr));
     }
 };
 

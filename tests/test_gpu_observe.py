@@ -29,3 +29,24 @@ def test_fp64_sums_of_small_terms(shape):
         s.upload(np.zeros(shape), L, c)
         w = c.astype(np.longdouble) - np.longdouble(0.978)
         assert abs(s.reduce()["free_energy"] / float((150 * w * w).sum()) - 1) <= 1e-10
+
+
+def test_fp32_gradient_energy_beside_a_larger_well_energy():
+    """Two arrangements of the same values differ by their gradients alone, a third
+    of an FP32 ulp of a cell's well energy: the sum has 48 bits of them (a hundredth
+    of the difference allowed)."""
+    shape = (8, 16, 32)
+    d = 8.4e-6
+    z, y, x = np.meshgrid(*[np.arange(n) for n in shape], indexing="ij")
+    L = np.full(shape, 0.5)
+    c = np.full(shape, 0.7)
+    p = ppf.params_default(dt=DT08, AS=1e-9, AL=1e-9, CS=0.0, CL=0.0)
+    m = ppf.derive(p)
+    got, want = [], []
+    with ppf.Simulation(shape, p, precision="f32") as s:
+        for sign in (np.where((x + y + z) % 2, 1, -1), np.where(x < 16, 1, -1)):
+            S = (0.5 + d * sign).astype(np.float32).astype(np.float64)
+            s.upload(S, L, c)
+            got.append(s.reduce()["free_energy"])
+            want.append(0.5 * m.kappa * m.h2 * sum(((np.roll(S, -1, a) - S) ** 2).sum() for a in range(3)))
+    assert abs((got[0] - got[1]) / (want[0] - want[1]) - 1) <= 1e-2
