@@ -320,17 +320,33 @@ __device__ __forceinline__ V2<float> recip(V2<float> x) {
 }
 // 1/x by one third-order Newton step y (1 + e + e^2), e = 1 - x y, on the
 // hardware's estimate (e below 2^-20, so the remainder e^3 is far below an
-// ulp): three FP64 operations.  Operands near the ends of the range take
-// the exact division.
+// ulp): three FP64 operations.
 __device__ __forceinline__ double recip(double x) {
-    const unsigned ex = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-    if (ex - 64u > 1920u) return 1.0 / x;
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double e = fma(-x, y, 1.0);
     return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ V2<double> recip(V2<double> x) { return V2<double>(recip(x.x()), recip(x.y())); }
+
+// whether a^2 + b^2 and its reciprocal lie inside the normal range, as these
+// estimates need them: the larger one in [2^-63, 2^62), [2^-480, 2^480) (NaN and
+// infinities are not)
+__device__ __forceinline__ bool invertible(float a, float b) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(fabsf(a)), "f"(fabsf(b)));
+    return __float_as_uint(m) - 0x20000000u < 0x3e800000u;
+}
+__device__ __forceinline__ bool invertible(double a, double b) {
+    const unsigned m = max((unsigned)__double2hiint(a) & 0x7fffffffu, (unsigned)__double2hiint(b) & 0x7fffffffu);
+    return m - 0x21f00000u < 0x3c000000u;
+}
+
+// a / b of a pair whose values are alike, for anything
+template <typename T>
+__device__ __noinline__ T divide1(T a, T b) { return a / b; }
+template <typename T>
+__device__ __forceinline__ V2<T> divide(V2<T> a, V2<T> b) { return splat(divide1<T>(a.x(), b.x())); }
 
 // finite, and above one half, without FP64 instructions
 __device__ __forceinline__ bool finite_(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
@@ -353,17 +369,19 @@ struct ObsAcc {
     Sum<T> h, w, f;      // solid fraction, chemical energy, m f0 + gradient energy
     int n = 0, solid = 0, bad = 0;
 
-    // a pair of finite cells (own values and the +x, +y, +z neighbours), of
-    // which the first nv count
+    // A pair of finite cells (own values and the +x, +y, +z neighbours), of
+    // which the first nv count.  DIV: etaS^2 + etaL^2 and AS + (AL - AS) h may be
+    // anything; else both are invertible.
+    template <bool DIV = false>
     __device__ __forceinline__ void pair(const ObsCoef<T> &k, V2<T> eS, V2<T> eL, V2<T> c, V2<T> sx, V2<T> lx,
                                          V2<T> sy, V2<T> ly, V2<T> sz, V2<T> lz, int nv = 2) {
         const V2<T> S2 = eS * eS, L2 = eL * eL, s2 = fma2(eL, eL, S2);
-        const V2<T> hh = S2 * recip(s2);
+        const V2<T> hh = DIV ? divide(S2, s2) : S2 * recip(s2);
         const V2<T> ww = fma2(hh, splat(k.dc0), c - splat(k.cL0));
         V2<T> ch = ww * ww;
         if (!k.eq) {
             const V2<T> den = fma2(hh, splat(k.dA), splat(k.AS));
-            ch = ch * recip(den);
+            ch = DIV ? divide(ch, den) : ch * recip(den);
         }
         // f0 = S2 (S2/4 - 1/2 + gamma L2) + L2 (L2/4 - 1/2) + 1/4
         const V2<T> q = splat(T(0.25)), hf = splat(T(-0.5));
@@ -500,11 +518,11 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
             // the cell after the last one (a ghost at the domain's end)
             const T sx = whole ? fl.eS[j + Q] : T(0), lx = whole ? fl.eL[j + Q] : T(0);
             bool fine = MASK || whole;
+            // (bitwise: a chain of branches made the loop a third slower)
 #pragma unroll
-            for (int i = 0; i < Q; ++i) fine = fine && (i >= cells || (finite_(s[i]) && finite_(l[i]) && finite_(c[i])));
-            if constexpr (FX) {
-#pragma unroll
-                for (int i = 0; i < Q; ++i) fine = fine && (i >= cells || !out_of_box(s[i], l[i], c[i], kx.cmax));
+            for (int i = 0; i < Q; ++i) {
+                if constexpr (FX) fine = fine && (i >= cells || !out_of_box(s[i], l[i], c[i], kx.cmax));
+                else fine = fine & ((i >= cells) | (invertible(s[i], l[i]) & finite_(c[i])));
             }
             if (fine) {
                 acc.n += cells;
@@ -532,8 +550,8 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
                     else pairs(Q);
                 }
             } else {
-                // non-finite cells (counted and left out), or cells outside the box:
-                // cell by cell, twice the same cell in a pair
+                // non-finite cells (counted and left out), or cells outside the box or
+                // the reciprocal's range: cell by cell, twice the same cell in a pair
                 for (int i = 0; i < Q && x0 + i < g.nx; ++i) {
                     const int64_t a = j + i;
                     const T S = fl.eS[a], L = fl.eL[a], C = fl.c[a];
@@ -543,7 +561,7 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
                     }
                     ++acc.n;
                     acc.solid += above_half(S) ? 1 : 0;
-                    acc.pair(k, splat(S), splat(L), splat(C), splat(fl.eS[a + 1]), splat(fl.eL[a + 1]),
+                    acc.template pair<true>(k, splat(S), splat(L), splat(C), splat(fl.eS[a + 1]), splat(fl.eL[a + 1]),
                              splat(fl.eS[a + g.P]), splat(fl.eL[a + g.P]), splat(fl.eS[a + g.PS]),
                              splat(fl.eL[a + g.PS]), 1);
                 }

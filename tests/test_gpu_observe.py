@@ -50,3 +50,21 @@ def test_fp32_gradient_energy_beside_a_larger_well_energy():
             got.append(s.reduce()["free_energy"])
             want.append(0.5 * m.kappa * m.h2 * sum(((np.roll(S, -1, a) - S) ** 2).sum() for a in range(3)))
     assert abs((got[0] - got[1]) / (want[0] - want[1]) - 1) <= 1e-2
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("precision,size,tol", [("f32", 6e-20, 3e-6), ("f32", 1e19, 1e-6), ("f64", 1e-157, 1e-8), ("f64", 1e153, 1e-13)])
+def test_solid_fraction_at_the_ends_of_the_range(shape, precision, size, tol):
+    """Phase fields whose squares are denormal or near the largest number: the
+    ratio etaS^2 / (etaS^2 + etaL^2) is what the type's division gives (a denormal
+    square is exact to a unit, 1.4e-45 or 5e-324)."""
+    r = np.random.default_rng(3)
+    t = np.float32 if precision == "f32" else np.float64
+    S, L = ((size * r.uniform(0.7, 1.3, shape)).astype(t) for _ in range(2))
+    c = r.uniform(0.4, 1.0, shape)
+    with ppf.Simulation(shape, precision=precision) as s:
+        s.upload(S.astype(np.float64), L.astype(np.float64), c)
+        g = s.reduce()
+    S2, s2 = S * S, S * S + L * L
+    assert s2.max() < np.finfo(t).max and g["nonfinite"] == 0
+    assert abs(g["solid"] / (S2 / s2).astype(np.float64).sum() - 1) <= tol
