@@ -474,6 +474,17 @@ struct ObsFx {
     }
 };
 
+// The solute mass of a thread's finite cells in FP64, for FP32 compositions so
+// large that their sum in floats is none (FP64 holds any such sum).
+template <typename T>
+__device__ __noinline__ double column_mass(const Geom &g, const Fields<const T> &f, int64_t j, int nz, int cells) {
+    double m = 0;
+    for (int z = 0; z < nz; ++z, j += g.PS)
+        for (int i = 0; i < cells; ++i)
+            if (finite_(f.eS[j + i]) && finite_(f.eL[j + i]) && finite_(f.c[j + i])) m += (double)f.c[j + i];
+    return m;
+}
+
 // FX: an FP64 state whose parameters fit the fixed-point step; cells outside
 // its box take the FP64 path.  MASK: the rows' last groups hold fewer cells than
 // the others; a warp with such a group counts its cells by mask, all lanes alike
@@ -579,6 +590,12 @@ __global__ void __launch_bounds__(256, FX ? 2 : 3) observe_kernel(Geom g, ObsCoe
     // lanes 0, 8, 16, 24 end with mass, h, w and f.
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double v[4] = {acc.mass.get(), acc.h.get(), acc.w.get(), acc.f.get()};
+    if constexpr (!std::is_same<T, double>::value) {
+        if (!finite_(v[0])) {
+            const int z0 = blockIdx.y * zc;
+            v[0] = column_mass<T>(g, fl, g.at(x0, y, z0), min(g.nz - z0, zc), min(Q, g.nx - x0));
+        }
+    }
     if constexpr (FX) {
         v[0] += ax.c.get(kx.sc) + ax.mass;
         v[1] += ax.h;

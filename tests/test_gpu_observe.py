@@ -68,3 +68,22 @@ def test_solid_fraction_at_the_ends_of_the_range(shape, precision, size, tol):
     S2, s2 = S * S, S * S + L * L
     assert s2.max() < np.finfo(t).max and g["nonfinite"] == 0
     assert abs(g["solid"] / (S2 / s2).astype(np.float64).sum() - 1) <= tol
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("bad", [False, True])
+def test_fp32_mass_of_huge_compositions(shape, bad):
+    """Finite compositions whose sum no float holds: an FP64 sum of the stored
+    values, non-finite cells left out."""
+    r = np.random.default_rng(4)
+    S, L = r.uniform(0.2, 1.0, shape), r.uniform(0.2, 1.0, shape)
+    c = (3e38 * r.uniform(0.5, 1.0, shape)).astype(np.float32).astype(np.float64)
+    if bad:
+        c[1, 2, 3] = np.inf
+        S[2, 3, 5] = np.nan
+    with ppf.Simulation(shape, precision="f32") as s:
+        s.upload(S, L, c)
+        g = s.reduce()
+    ok = np.isfinite(S) & np.isfinite(c)
+    assert g["nonfinite"] == (~ok).sum()
+    assert abs(g["mass"] / c[ok].sum() - 1) <= 1e-12
