@@ -750,23 +750,23 @@ extern "C" int ppf_particles(ppf_ctx *c, double threshold, ppf_particle_stats *o
     }
     int nb = (int)((cells + 255) / 256);
     if (nb > 8 * c->num_sms) nb = 8 * c->num_sms;
-    int rc = ensure_partials(c, 5 * nb + 3 * c->num_sms);
+    int rc = ensure_partials(c, 6 * nb + 3 * c->num_sms);
     if (rc) return rc;
     double *dout = c->dres + 8;
     int *const vols = cap > 0 ? c->plist : nullptr;
     if (c->prec == PPF_F32)
         CU(launch_particles<float>(c->g, (const float *)c->fld[c->cur_eta][0], threshold, ps, c->partials, nb, c->num_sms,
-                                   c->p.dx, dout, vols, cap, c->derr, c->stream));
+                                   dout, vols, cap, c->derr, c->stream));
     else
         CU(launch_particles<double>(c->g, (const double *)c->fld[c->cur_eta][0], threshold, ps, c->partials, nb,
-                                    c->num_sms, c->p.dx, dout, vols, cap, c->derr, c->stream));
+                                    c->num_sms, dout, vols, cap, c->derr, c->stream));
     double res[kResults];
     rc = fetch_results(c, res);
     if (rc) return rc;
     const double *const h = res + 8;
     const double dx = c->p.dx;
     out->count = (int64_t)h[0];
-    out->mean_radius = h[0] > 0 ? h[1] / h[0] / dx : 0.0;
+    out->mean_radius = h[0] > 0 ? h[1] / h[0] : 0.0;
     out->solid_volume = h[2] * dx * dx * dx;
     out->largest_volume = h[3] * dx * dx * dx;
     out->interface_area = h[4] * dx * dx;

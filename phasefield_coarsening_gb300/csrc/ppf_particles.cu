@@ -364,13 +364,38 @@ __global__ void __launch_bounds__(kNT) add_volumes(const int *__restrict__ list,
     }
 }
 
+// Radii are summed exactly, in units of 2^-53 cells (any two words of a sum apart,
+// the low one's carries left in it): the list is in no order, and a rounded
+// sum's last bits would depend on it.
+struct RadiusSum {
+    unsigned long long lo = 0, hi = 0;
+    __device__ __forceinline__ void add(double r) {               // 0.6 <= r < 801: volumes below 2^31
+        const unsigned long long v = (unsigned long long)__double2ll_rn(r * 9007199254740992.0);
+        lo += (unsigned)v;
+        hi += v >> 32;
+    }
+    __device__ __forceinline__ void add(const RadiusSum &o) {
+        lo += o.lo;
+        hi += o.hi;
+    }
+    __device__ __forceinline__ void add_lane(int d) {             // that of the lane at distance d (xor)
+        lo += __shfl_xor_sync(0xffffffffu, lo, d);
+        hi += __shfl_xor_sync(0xffffffffu, hi, d);
+    }
+    __device__ __forceinline__ double get() const {
+        return ((double)(hi + (lo >> 32)) * 4294967296.0 + (double)(unsigned)lo) * 1.1102230246251565e-16;
+    }
+};
+
 // per root: count, sum of equivalent radii, sum of volumes, largest volume;
-// optionally the volumes themselves, in no order
+// optionally the volumes themselves, in no order.  partials: count, volumes,
+// largest volume, then the radius sum's two words.
 __global__ void __launch_bounds__(kNT) root_stats(const int *__restrict__ list, const int *__restrict__ nlist,
-                                                  const int *__restrict__ lab, const int *__restrict__ vol, double dx3,
+                                                  const int *__restrict__ lab, const int *__restrict__ vol,
                                                   double *__restrict__ partials, int *__restrict__ volumes, int64_t cap,
                                                   int *__restrict__ nvolumes) {
-    double cnt = 0, rsum = 0, vsum = 0, vmax = 0;
+    double cnt = 0, vsum = 0, vmax = 0;
+    RadiusSum rsum;
     const double k = 3.0 / (4.0 * 3.14159265358979323846);
     const int n = *nlist, step = gridDim.x * kNT, lane = threadIdx.x & 31;
     for (int i0 = blockIdx.x * kNT; i0 < n; i0 += step) {
@@ -381,7 +406,7 @@ __global__ void __launch_bounds__(kNT) root_stats(const int *__restrict__ list, 
         if (root) {
             const double v = (double)iv;
             cnt += 1.0;
-            rsum += cbrt(k * v * dx3);
+            rsum.add(cbrt(k * v));
             vsum += v;
             vmax = v > vmax ? v : vmax;
         }
@@ -394,26 +419,36 @@ __global__ void __launch_bounds__(kNT) root_stats(const int *__restrict__ list, 
         }
         if (n - i0 <= step) break;
     }
-    __shared__ double red[kNT / 32][4];
-    double v4[4] = {cnt, rsum, vsum, vmax};
-    for (int q = 0; q < 4; ++q) {
-        double a = v4[q];
+    __shared__ double red[kNT / 32][3];
+    __shared__ unsigned long long rred[kNT / 32][2];
+    double v3[3] = {cnt, vsum, vmax};
+    for (int q = 0; q < 3; ++q) {
+        double a = v3[q];
         for (int o = 16; o > 0; o >>= 1) {
             const double b = __shfl_xor_sync(0xffffffffu, a, o);
-            a = q == 3 ? (b > a ? b : a) : a + b;
+            a = q == 2 ? (b > a ? b : a) : a + b;
         }
         if (lane == 0) red[threadIdx.x >> 5][q] = a;
     }
+    for (int o = 16; o > 0; o >>= 1) rsum.add_lane(o);
+    if (lane == 0) {
+        rred[threadIdx.x >> 5][0] = rsum.lo;
+        rred[threadIdx.x >> 5][1] = rsum.hi;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double s[4] = {0, 0, 0, 0};
+        double s[3] = {0, 0, 0};
+        unsigned long long u[2] = {0, 0};
         for (int w = 0; w < kNT / 32; ++w) {
             s[0] += red[w][0];
             s[1] += red[w][1];
-            s[2] += red[w][2];
-            s[3] = red[w][3] > s[3] ? red[w][3] : s[3];
+            s[2] = red[w][2] > s[2] ? red[w][2] : s[2];
+            u[0] += rred[w][0];
+            u[1] += rred[w][1];
         }
-        for (int q = 0; q < 4; ++q) partials[(int64_t)blockIdx.x * 4 + q] = s[q];
+        double *p = partials + (int64_t)blockIdx.x * 5;
+        for (int q = 0; q < 3; ++q) p[q] = s[q];
+        for (int q = 0; q < 2; ++q) p[3 + q] = __longlong_as_double((long long)u[q]);
     }
 }
 
@@ -552,9 +587,25 @@ __global__ void __launch_bounds__(kNT) finish_stats(const double *__restrict__ f
                                                     const double *__restrict__ rs, int nb, double *__restrict__ out) {
     __shared__ double red[kNT];
     const int q = blockIdx.x;
+    if (q == 1) {
+        __shared__ RadiusSum rred[kNT];
+        RadiusSum s;
+        for (int b = threadIdx.x; b < nb; b += kNT) {
+            s.lo += (unsigned long long)__double_as_longlong(rs[(int64_t)b * 5 + 3]);
+            s.hi += (unsigned long long)__double_as_longlong(rs[(int64_t)b * 5 + 4]);
+        }
+        rred[threadIdx.x] = s;
+        __syncthreads();
+        for (int h = kNT / 2; h > 0; h >>= 1) {
+            if ((int)threadIdx.x < h) rred[threadIdx.x].add(rred[threadIdx.x + h]);
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) out[q] = rred[0].get();
+        return;
+    }
     double a = 0.0;
     for (int b = threadIdx.x; b < (q < 4 ? nb : nf); b += kNT) {
-        const double v = q < 4 ? rs[(int64_t)b * 4 + q] : faces[b];
+        const double v = q < 4 ? rs[(int64_t)b * 5 + (q == 0 ? 0 : q - 1)] : faces[b];
         a = q == 3 ? (v > a ? v : a) : a + v;
     }
     red[threadIdx.x] = a;
@@ -605,7 +656,7 @@ ParticleScratch particle_scratch(const Geom &g, int *mem) {
 
 template <typename T>
 cudaError_t launch_particles(const Geom &g, const T *etaS, double threshold, const ParticleScratch &p, double *partials,
-                             int nblocks, int num_sms, double dx, double *out, int *volumes, int64_t cap, int *err,
+                             int nblocks, int num_sms, double *out, int *volumes, int64_t cap, int *err,
                              cudaStream_t s) {
     const Words q = words_of(g);
     cudaError_t e =
@@ -621,7 +672,7 @@ cudaError_t launch_particles(const Geom &g, const T *etaS, double threshold, con
                                                               p.counts, partials, err);
     merge_bricks<<<nblocks, kNT, 0, s>>>(q, p.bits, p.lab, partials + nb1, err);
     add_volumes<<<nblocks, kNT, 0, s>>>(p.list, p.counts, p.lab, p.vol, err);
-    root_stats<<<nb4, kNT, 0, s>>>(p.list, p.counts, p.lab, p.vol, dx * dx * dx, stats, volumes, cap, p.counts + 1);
+    root_stats<<<nb4, kNT, 0, s>>>(p.list, p.counts, p.lab, p.vol, stats, volumes, cap, p.counts + 1);
     finish_stats<<<5, kNT, 0, s>>>(partials, nb1 + nblocks, stats, nb4, out);
     return cudaGetLastError();
 }
@@ -657,8 +708,8 @@ cudaError_t launch_sort_volumes(int *keys, int *spare, int64_t n, int64_t larges
 }
 
 template cudaError_t launch_particles<float>(const Geom &, const float *, double, const ParticleScratch &, double *, int,
-                                             int, double, double *, int *, int64_t, int *, cudaStream_t);
+                                             int, double *, int *, int64_t, int *, cudaStream_t);
 template cudaError_t launch_particles<double>(const Geom &, const double *, double, const ParticleScratch &, double *,
-                                              int, int, double, double *, int *, int64_t, int *, cudaStream_t);
+                                              int, int, double *, int *, int64_t, int *, cudaStream_t);
 
 }  // namespace ppf

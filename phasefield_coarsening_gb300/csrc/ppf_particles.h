@@ -19,13 +19,13 @@ ParticleScratch particle_scratch(const Geom &g, int *mem);
 
 // Labels the solid (etaS > threshold) of the state whose etaS is `etaS`
 // (padded layout), then writes out[0..4] = {particles, sum of equivalent
-// radii, solid cells, largest particle (cells), solid/liquid faces}.
-// partials: 5 nblocks + 3 num_sms doubles; volumes (nullable): up to `cap`
+// radii (cells), solid cells, largest particle (cells), solid/liquid faces}.
+// partials: 6 nblocks + 3 num_sms doubles; volumes (nullable): up to `cap`
 // particle volumes, in no order; err: a device word, bit 1 set if a retry cap
 // was reached.
 template <typename T>
 cudaError_t launch_particles(const Geom &g, const T *etaS, double threshold, const ParticleScratch &p, double *partials,
-                             int nblocks, int num_sms, double dx, double *out, int *volumes, int64_t cap, int *err,
+                             int nblocks, int num_sms, double *out, int *volumes, int64_t cap, int *err,
                              cudaStream_t s);
 
 // Sorts n >= 1 volumes, none above `largest`, into *sorted (in the scratch of a

@@ -197,3 +197,22 @@ def test_gpu_particle_volumes_in_order(shape):
         s.upload(e, 1.0 - e, np.full(shape, 0.7))
         g = s.particles(volumes=True)
     assert g["count"] == o["count"] and np.array_equal(g["volumes"], np.sort(o["volumes"]))
+
+
+@pytest.mark.gpu
+def test_gpu_mean_radius_repeats_and_is_exact():
+    """Thousands of particles in an order that differs from call to call: the mean
+    radius is the same number every time, the exact sum of the (correctly rounded to
+    an ulp) radii to a few ulps."""
+    import math
+    rng = np.random.default_rng(11)
+    shape = (40, 70, 130)
+    etaS = np.where(rng.random(shape) < 0.24, 0.9, 0.1)
+    with ppf.Simulation(shape, ppf.params_default(dx=0.7), bc="noflux") as s:
+        s.upload(etaS, 1 - etaS, np.full(shape, 0.7))
+        first = s.particles(volumes=True)
+        assert first["count"] > 10000
+        for _ in range(60):
+            assert s.particles()["mean_radius"] == first["mean_radius"]
+    exact = math.fsum(np.cbrt(3 / (4 * math.pi) * first["volumes"])) / first["count"]
+    assert abs(first["mean_radius"] / exact - 1) <= 1e-15
