@@ -284,14 +284,23 @@ struct ReduceJobs {
     double *loss;
 };
 
+// the plain FP64 sum, for sums that floats do not hold
+__device__ __noinline__ double wide_sum(const float *part, int nb, int stride) {
+    double s = 0;
+    for (int b = 0; b < nb; ++b) s += (double)part[(int64_t)b * stride];
+    return s;
+}
+
 // A block takes 32 values, its eight warps an eighth of the partial sums each:
 // independent loads in flight instead of one thread's chain (21 us for 152
-// partials of 27 x 32 x 32 weights), and sums carried with their rounding
-// errors in float (Knuth's TwoSum, about 48 bits) instead of FP64, whose
-// conversions and additions alone would take 14 us.  All jobs of a step in one
-// launch: 24 us for the 84 MB of a width-32 network (62 us in twelve launches).
+// partials of 27 x 32 x 32 weights), and sums in three floats (about 72 bits,
+// more than an FP64 sum keeps) instead of FP64, whose conversions and additions
+// alone would take 14 us; one that overflows or holds no number is summed in
+// FP64 after all.  All jobs of a step in one launch: 33 us for the 84 MB of a
+// width-32 network (62 us in twelve launches; 42 us with the eight parts of a
+// value put together by one lane; 24 us in two floats, 48 bits).
 __global__ void __launch_bounds__(kNT) reduce_kernel(const __grid_constant__ ReduceJobs q) {
-    __shared__ float2 red[kNT / 32][32];
+    __shared__ Mass1 red[kNT / 32][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int j = 0;
     while ((int)blockIdx.x >= q.first[j + 1]) ++j;
@@ -300,26 +309,30 @@ __global__ void __launch_bounds__(kNT) reduce_kernel(const __grid_constant__ Red
     const int b0 = nb * warp / (kNT / 32), b1 = nb * (warp + 1) / (kNT / 32);
     const int i = ((int)blockIdx.x - q.first[j]) * 32 + lane;
     const float *part = q.part[j] + i;
-    float2 s = make_float2(0.f, 0.f);
-    auto add = [](float2 &a, float x) {
-        float e;
-        a.x = two_sum1(a.x, x, e);
-        a.y += e;
-    };
+    Mass1 s;
     if (i < nv) {
 #pragma unroll 8
-        for (int b = b0; b < b1; ++b) add(s, part[(int64_t)b * q.stride[j]]);
+        for (int b = b0; b < b1; ++b) s.add(part[(int64_t)b * q.stride[j]]);
     }
     red[warp][lane] = s;
     __syncthreads();
-    if (warp == 0 && i < nv) {
-        for (int w = 1; w < kNT / 32; ++w) {
-            const float2 o = red[w][lane];
-            add(s, o.x);
-            s.y += o.y;
-        }
-        if (i < n) q.out[j][i] = s.x + s.y;
-        else *q.loss = (double)s.x + (double)s.y;
+    // eight lanes per value now
+    static_assert(kNT == 256, "32 values of eight parts");
+    const int v = i - lane + ((int)threadIdx.x >> 3);
+    s = red[threadIdx.x & 7][threadIdx.x >> 3];
+#pragma unroll
+    for (int d = 1; d < 8; d *= 2) {
+        const float hi = __shfl_xor_sync(0xffffffffu, s.hi, d), mid = __shfl_xor_sync(0xffffffffu, s.mid, d);
+        const float lo = __shfl_xor_sync(0xffffffffu, s.lo, d);
+        s.add(hi);
+        s.add(mid);
+        s.lo += lo;
+    }
+    if ((threadIdx.x & 7) == 0 && v < nv) {
+        double t = s.get();
+        if (!isfinite(t)) t = wide_sum(q.part[j] + v, nb, q.stride[j]);
+        if (v < n) q.out[j][v] = (float)t;
+        else *q.loss = t;
     }
 }
 
