@@ -90,12 +90,13 @@ __device__ __forceinline__ bool wait_backoff(uint32_t bar, uint32_t parity, unsi
 // Programmatic dependent launch: a convolution or weight-gradient kernel starts
 // while the CTAs of the one before finish, sets itself up, and waits here until
 // that one is complete and its results are visible.  The next kernel may start
-// only after this point, so at most two are in flight.  (64 x 128 x 128, width
-// 32: @T1@ us a training step, 1223 us without.)
-__device__ __forceinline__ void grid_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// only after grid_release, so at most two are in flight.  A CTA calls that behind
+// the barrier that follows its TMEM allocation: earlier, a CTA of the next kernel
+// could take the columns first and wait for this grid, which waits for the
+// columns.  (64 x 128 x 128, width 32: 1186 us a training step, 1232 us without
+// the overlap on the same machine.)
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // launch with that attribute
 template <typename Args>
@@ -278,6 +279,7 @@ __global__ void __launch_bounds__(ConvCfg<CI, CO>::threads(EPI), ConvCfg<CI, CO>
     grid_wait();
     tc_fence_before();
     __syncthreads();
+    grid_release();
     tc_fence_after();
     const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(tslot);
 
@@ -676,6 +678,7 @@ __global__ void __launch_bounds__(256, 1) wgrad_kernel(const __grid_constant__ W
     grid_wait();
     tc_fence_before();
     __syncthreads();
+    grid_release();
     tc_fence_after();
     const uint32_t tbase = *reinterpret_cast<volatile uint32_t *>(tslot);
 
