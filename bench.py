@@ -615,15 +615,15 @@ def run_ensemble(args):
 # Arithmetic of one cell-step in FP64 with AS == AL (the reference's
 # constants): pass A 18 (incl. one reciprocal), pass B 61; an FMA counts 2.
 # Algorithmic: the ring and halo-plane recomputation are not counted.  The
-# kernel does all but six of these operations in 64-bit fixed point.
+# kernel does all but twelve of its operations in 64-bit fixed point.
 FP64_FLOP_PER_CELL = 79
 
 
 def fp64_section(state, shape, steps=30):
     """The reference's precision on the GPU: the FP64 fused step on the same
     256^3 state, device-timed (CUDA events on its stream), against the
-    measured HBM peak (48 B per cell-step; issue and the integer pipes bound
-    the fixed-point arithmetic before that) and, for comparison, as FP64 FLOPs
+    measured HBM peak (48 B per cell-step; issue and the FP64 pipe bound the
+    kernel before that) and, for comparison, as FP64 FLOPs
     against this GPU's measured FP64 FMA rate."""
     import torch
 

@@ -176,7 +176,8 @@ typedef struct ppf_particle_stats {
 
 /* `volumes` (may be NULL) receives up to `capacity` particle volumes in
  * cells, in ascending order; *nvolumes (may be NULL) the particle count.
- * Device scratch of about 6 bytes per cell is allocated on the first call. */
+ * Device scratch of about 6 bytes per cell (8 to 16 where the x edge has 1 to 3
+ * cells) is allocated on the first call. */
 int ppf_particles(ppf_ctx *ctx, double threshold, ppf_particle_stats *out, int64_t *volumes, int64_t capacity,
                   int64_t *nvolumes);
 /* The first n volumes of the last ppf_particles call on this context, which
