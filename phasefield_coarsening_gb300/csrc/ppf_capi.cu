@@ -626,6 +626,7 @@ extern "C" int ppf_autotune(ppf_ctx *c, int trial_steps, ppf_tune *best) {
     int rc = do_unpack(c);
     if (rc) return rc;
     const StepTune keep = c->tune;
+    const bool fixed = c->prec == PPF_F64 && fx_step(c);
     cudaEvent_t e0, e1;
     CU(cudaEventCreate(&e0));
     CU(cudaEventCreate(&e1));
@@ -646,6 +647,8 @@ extern "C" int ppf_autotune(ppf_ctx *c, int trial_steps, ppf_tune *best) {
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
         if (best_ms < 0 || ms < best_ms) { best_ms = ms; win = t; }
+        // (a trial that left the box: the next one times the fixed-point kernel again)
+        if (fixed && c->left_box) rc = do_pack(c);
     };
     // uniform chunks; with edge tiles, as one launch or two; the first tile
     // shape with every deal and overlap, the others with the counter's deal
@@ -660,7 +663,7 @@ extern "C" int ppf_autotune(ppf_ctx *c, int trial_steps, ppf_tune *best) {
         for (int sp = 0; sp < nsplit && rc == PPF_OK; ++sp)
         for (int sd = 1; sd >= (tl == 0 ? 0 : 1) && rc == PPF_OK; --sd)
         for (int pdl = 1; pdl >= (tl == 0 ? 0 : 1) && rc == PPF_OK; --pdl)
-        for (int r = 0; r < (c->fx_ok ? 1 : 2) && rc == PPF_OK; ++r)    // (the fixed-point kernel has one form)
+        for (int r = 0; r < (fixed ? 1 : 2) && rc == PPF_OK; ++r)    // (the fixed-point kernel has one form)
             for (int i = 0; i < nzc && rc == PPF_OK; ++i) {
                 StepTune t = keep;
                 t.tile = tl;
