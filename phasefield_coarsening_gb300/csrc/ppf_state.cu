@@ -310,24 +310,28 @@ cudaError_t launch_unpack(const Geom &g, Fields<const T> src, double *const dst[
 // (about 32 per cell; ObsFx below has fewer).  256^3 FP32: 56 us (186 us with
 // one cell per thread and FP64 sums of the solute mass); 64^3: 7 us (33 us).
 
-// 1/x of a pair: the hardware's estimate (about 1 ulp) and a Newton step
-__device__ __forceinline__ V2<float> recip(V2<float> x) {
-    float a, b;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(a) : "f"(x.x()));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(x.y()));
-    const V2<float> y(a, b), e = fma2(splat(0.f) - x, y, splat(1.f));
-    return fma2(y, e, y);
+// a / b of a pair, as accurate as a division: the quotient by the hardware's
+// reciprocal estimate (about 1 ulp), and its residual times the estimate
+__device__ __forceinline__ V2<float> ratio(V2<float> a, V2<float> b) {
+    float y0, y1;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(b.x()));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(b.y()));
+    const V2<float> y(y0, y1), q = a * y;
+    return fma2(fma2(splat(0.f) - b, q, a), y, q);
 }
-// 1/x by one third-order Newton step y (1 + e + e^2), e = 1 - x y, on the
-// hardware's estimate (e below 2^-20, so the remainder e^3 is far below an
-// ulp): three FP64 operations.
-__device__ __forceinline__ double recip(double x) {
+// The FP64 estimate has 20 bits: one third-order Newton step y (1 + e + e^2),
+// e = 1 - b y, first.
+__device__ __forceinline__ double ratio(double a, double b) {
     double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
 }
-__device__ __forceinline__ V2<double> recip(V2<double> x) { return V2<double>(recip(x.x()), recip(x.y())); }
+__device__ __forceinline__ V2<double> ratio(V2<double> a, V2<double> b) {
+    return V2<double>(ratio(a.x(), b.x()), ratio(a.y(), b.y()));
+}
 
 // whether a^2 + b^2 and its reciprocal lie inside the normal range, as these
 // estimates need them: the larger one in [2^-63, 2^62), [2^-480, 2^480) (NaN and
@@ -376,12 +380,12 @@ struct ObsAcc {
     __device__ __forceinline__ void pair(const ObsCoef<T> &k, V2<T> eS, V2<T> eL, V2<T> c, V2<T> sx, V2<T> lx,
                                          V2<T> sy, V2<T> ly, V2<T> sz, V2<T> lz, int nv = 2) {
         const V2<T> S2 = eS * eS, L2 = eL * eL, s2 = fma2(eL, eL, S2);
-        const V2<T> hh = DIV ? divide(S2, s2) : S2 * recip(s2);
+        const V2<T> hh = DIV ? divide(S2, s2) : ratio(S2, s2);
         const V2<T> ww = fma2(hh, splat(k.dc0), c - splat(k.cL0));
         V2<T> ch = ww * ww;
         if (!k.eq) {
             const V2<T> den = fma2(hh, splat(k.dA), splat(k.AS));
-            ch = DIV ? divide(ch, den) : ch * recip(den);
+            ch = DIV ? divide(ch, den) : ratio(ch, den);
         }
         // f0 = S2 (S2/4 - 1/2 + gamma L2) + L2 (L2/4 - 1/2) + 1/4
         const V2<T> q = splat(T(0.25)), hf = splat(T(-0.5));
@@ -443,7 +447,7 @@ struct FxSquares {
 // float64: smaller values of c, the solid fraction of states that have little
 // of it, the gradient's differences and squares.  Fourteen of about 32
 // operations a cell are left for the FP64 pipe, which runs beside the integer
-// pipes.  256^3: 0.58 ms; 1.12 ms with all of it in FP64, 0.49 with all but the
+// pipes.  256^3: 0.58 ms; 1.24 ms with all of it in FP64, 0.49 with all but the
 // gradient in fixed point.
 struct ObsFx {
     FxSum f0, c;

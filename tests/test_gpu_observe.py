@@ -87,3 +87,23 @@ def test_fp32_mass_of_huge_compositions(shape, bad):
     ok = np.isfinite(S) & np.isfinite(c)
     assert g["nonfinite"] == (~ok).sum()
     assert abs(g["mass"] / c[ok].sum() - 1) <= 1e-12
+
+
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_solid_fraction_of_a_cell_is_its_quotient(precision):
+    """One cell's h = etaS^2 / (etaS^2 + etaL^2): the quotient of the rounded squares
+    to 0.51 ulp (a correctly rounded division's 0.5), by the one sum of one term.
+    (FP64 states in the box have no rounded squares: parameters outside it.)"""
+    from fractions import Fraction
+    r = np.random.default_rng(6)
+    t = np.float32 if precision == "f32" else np.float64
+    with ppf.Simulation((1, 1, 1), ppf.params_default(dt=DT08, AL=2e9), precision=precision) as s:
+        for _ in range(300):
+            S, L = r.uniform(0.05, 1.2, 2).astype(t)
+            s.upload(*[np.full((1, 1, 1), float(v)) for v in (S, L, t(0.7))])
+            got = s.reduce()["solid"]
+            S2 = S * S
+            exact = Fraction(float(L)) ** 2 + Fraction(float(S2))
+            s2 = float(exact) if precision == "f64" else float(np.float32(float(exact)))
+            q = Fraction(float(S2)) / Fraction(s2)
+            assert abs(Fraction(got) - q) <= Fraction(51, 100) * Fraction(float(np.spacing(t(float(q)))))
