@@ -19,9 +19,9 @@
 // smaller one's, rate x eta - kt x Laplacian, is formed in float64, as exact
 // relative to a value of 1e-300 as to one of 1.  The new values are as close to
 // the exact ones as float64 arithmetic's (root mean square within 0.01 %, each
-// relative to its own size); an increment of a larger field is resolved to
-// 2^(eu-62), 1e-19 with the reference's constants, where float64's own error in
-// an interface is 3e-19.
+// relative to its own size).  An increment of a larger field is resolved to
+// 2^(eu-62), 1e-19 with the reference's constants, where a bulk phase may change by
+// less: sums of squares take it from a formula of its own.
 // Integer sums are exact, and a face's flux is the same number with the
 // opposite sign seen from its other side.  A product is three 32 x 32 ->
 // 64-bit multiply-adds.
@@ -61,6 +61,9 @@ struct FxCoef {
     i64 g;         // gamma @61
     double su, sc; // 2^(eu-61), 2^(ec-59): increments of eta and c
     double kb;     // -kt in units of su
+    i64 mtm, mtgm; // mt and mt (2 gamma - 1) @68 in units of 2^em (finer than 2^eu)
+    i64 nktm;      // -kt @67 in units of 2^em
+    int um;        // em - eu
     int se;        // -eu (0 to 40)
     int ec, eu;
     unsigned cmax; // high word of the box bound of |c|, 2^(ec+1)
@@ -136,6 +139,39 @@ PPF_FX i64 recip(i64 s2) {
     return ((i64)r0 << 38) + ((v + (1ll << 11)) >> 12);
 }
 
+// v 2^e of a normal number whose product is normal, without FP64 operations
+PPF_FX double times_2(double v, int e) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(__double2hiint(v) + (e << 20), __double2loint(v));
+#else
+    return std::ldexp(v, e);
+#endif
+}
+
+// v 2^e as a double (|v| < 2^63, the result normal or 0), without FP64 operations:
+// a conversion instruction takes the FP64 pipe as long as two or three additions.
+// unit60 is the same for 2^52 <= v < 2^63 and e = -60.
+PPF_FX double unit60(i64 v) {
+#ifdef __CUDA_ARCH__
+    const int z = __clzll(v);
+    const unsigned long long m = (unsigned long long)v << z;
+    // (a carry out of the mantissa goes on into the exponent)
+    return __longlong_as_double((i64)(((unsigned long long)(1025 - z) << 52) + (m >> 11) + ((m >> 10) & 1)));
+#else
+    return std::ldexp((double)v, -60);
+#endif
+}
+PPF_FX double to_double(i64 v, int e) {
+#ifdef __CUDA_ARCH__
+    const i64 neg = v >> 63;
+    const i64 a = (v ^ neg) - neg;
+    const double d = times_2(unit60(a), e + 60);
+    return a ? __hiloint2double(__double2hiint(d) | (hi32(neg) & (int)0x80000000), __double2loint(d)) : 0.0;
+#else
+    return std::ldexp((double)v, e);
+#endif
+}
+
 // what a cell's neighbours need
 struct Nb {
     i64 S, L;      // eta @58
@@ -191,28 +227,31 @@ PPF_FX double eta_large(const FxCoef &k, i64 v, i64 inc) {
     const i64 n = (v << 2) + ((inc + (1ll << k.se)) >> (k.se + 1));
 #ifdef __CUDA_ARCH__
     const double d = (double)n;
-    return __hiloint2double(n ? __double2hiint(d) - (60 << 20) : 0, __double2loint(d));
+    return n ? times_2(d, -60) : 0.0;
 #else
     return std::ldexp((double)n, -60);
 #endif
+}
+// The same increment, in units of su, with a relative precision of its own, for
+// the sums of squares: the well and Laplacian terms @61 on their own scale, the
+// drive with the smaller field's square in float64 (against extended precision at
+// least as close as float64 arithmetic, in interfaces ten times).  (Below 2^-62 of the units
+// the integer holds nothing, and a bulk phase may change by less.)  v and s are
+// the larger and the smaller field, iv and is the same @58, W the cell's w, lap the
+// larger field's six neighbours less six times itself @58; `solid`: v is etaS.
+PPF_FX double eta_inc_large(const FxCoef &k, double v, double s, i64 iv, i64 is, i64 W, i64 lap, bool solid) {
+    const i64 V = iv << 3, V2 = mulx<2>(V, V), s2 = mulx<2>(is << 3, is << 3);                       // @61, @60
+    const i64 R = recip(V2 + s2);
+    const i64 u = mulq(k.mtm, V2 + s2 - (1ll << 60)) + mulq(k.mtgm, s2);                             // @64
+    const i64 e = mulq(V, u) + mulq(k.nktm, lap);                                                    // @61
+    const i64 d = mulx<2>(mulx<3>(k.k0 + mulx<2>(k.k1, W), R), R);                                   // @59
+    return fma(to_double(solid ? d : -d, 2), s * s * v, to_double(e, k.um));
 }
 // The increment of the smaller one, in the same units, in float64.  Its six
 // neighbours' weight is not in the rate; add it with one rounding,
 // fma(increment, su, v).
 PPF_FX double eta_inc(const FxCoef &k, i64 rate, double v, double six) {
     return fma(k.kb, six, (double)(rate - k.nk6) * v);
-}
-
-// v 2^-60 as a double, for 2^52 <= v < 2^63, without FP64 operations
-PPF_FX double unit60(i64 v) {
-#ifdef __CUDA_ARCH__
-    const int z = __clzll(v);
-    const unsigned long long m = (unsigned long long)v << z;
-    // (a carry out of the mantissa goes on into the exponent)
-    return __longlong_as_double((i64)(((unsigned long long)(1025 - z) << 52) + (m >> 11) + ((m >> 10) & 1)));
-#else
-    return std::ldexp((double)v, -60);
-#endif
 }
 
 // A cell's terms of the observables: c @59 and w @59 (in units of 2^ec), the
@@ -276,6 +315,11 @@ inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0
     const double a0 = std::fabs((double)k0), a1 = std::fabs((double)k1);
     const double need = std::fmax(std::fmax(8.0 * a1, 2.0 * (a0 + 3.5 * a1)),
                                   std::fmax(1024.0 * std::fabs(mt), 32.0 * std::fabs(kt)));
+    // the same for the well and the Laplacian alone
+    const double need_m = std::fmax(1024.0 * std::fabs(mt), 32.0 * std::fabs(kt));
+    int em = 0;
+    if (need_m > 0) std::frexp(need_m, &em);
+    if (need_m > 0 && em < -500) em = -500;
     int eu = -40;
     if (need > 0) {
         int e;
@@ -295,6 +339,10 @@ inline bool make_fxcoef(double AS, double AL, double cL0, double dc0, double Mt0
     f.nkt = q(-kt, 67 - eu);
     f.nk6 = q(-6 * (ld)kt, 61 - eu);
     f.se = -eu;
+    f.mtm = q(mt, 68 - em);
+    f.mtgm = q((ld)mt * ((ld)tg - 1), 68 - em);
+    f.nktm = q(-kt, 67 - em);
+    f.um = em - eu;
     f.g = q(0.5 * tg, 61);
     f.su = std::ldexp(1.0, eu - 61);
     f.sc = std::ldexp(1.0, ec - 59);

@@ -6,12 +6,12 @@
 // its memory traffic.  Here a cell has twelve: nine for the increment of its
 // smaller phase field, which keeps float64's relative precision however small
 // the value is (ppf_fx.h), one conversion of the larger one, two for c.
-// 0.64 ms at 256^3, 19 us at 64^3 (56 us).  What bounds it are dependency waits
-// at sixteen warps an SM: the FP64 pipe is busy 56 % of the time, 55 % of the
-// issue slots are taken (813 instructions a cell), the ALU 46 %.  With both fields' increments in fixed point (six
-// operations, small values lost) it took as long, with both in float64 0.90 ms;
-// two additions in place of each conversion instruction, 0.78 against 0.70;
-// rates in the halo planes too, 0.64 ms and 20.6 us.
+// 0.61 ms at 256^3, 18 us at 64^3 (56 us).  What bounds it are dependency waits
+// at sixteen warps an SM: the FP64 pipe is busy 53 % of the time, 54 % of the
+// issue slots are taken (780 instructions a cell), the ALU 46 %.  With both
+// fields' increments in fixed point (six operations, small values lost) it took
+// 0.64 ms, with both in float64 0.90; two additions in place of each conversion
+// instruction, 0.78 against 0.70; rates in the halo planes too, 20.6 us at 64^3.
 //
 // The data flow is that of ppf_step_tma.cuh: work items (z chunk, 32 x 16
 // tile) marched up z, etaS/etaL/c boxes streamed by TMA, pass A once per
@@ -207,8 +207,12 @@ __device__ __forceinline__ void put_sums(const double (&acc)[3], double *partial
         }
 }
 
-// FULL: every tile of the launch lies inside its domain.
-template <bool C_ONLY, bool FULL, bool MULTI>
+// FULL: every tile of the launch lies inside its domain.  STATS: the increments'
+// sums of squares go to a.partials, the larger field's increments computed once
+// more for them with a precision of their own (a kernel of its own: their code
+// costs the others 4 % in registers; 256^3 0.61 and 0.89 ms, 0.70 with the
+// increments that are added).
+template <bool C_ONLY, bool FULL, bool MULTI, bool STATS>
 __global__ void __launch_bounds__(kThreads, 2)
     step_fx_kernel(const __grid_constant__ CUtensorMap mapS, const __grid_constant__ CUtensorMap mapL,
                    const __grid_constant__ CUtensorMap mapC, const __grid_constant__ FxArgs a) {
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             double inc[3] = {0, 0, 0};
             slow_item<C_ONLY>(a.k, g, in, out, it, reinterpret_cast<double(*)[2][G::BOX]>(sm.nb), mb, inc);
             if (tid == 0) (MULTI ? a.table[it.dom].box : a.box)[1 - a.parity] = 1;
-            if (a.partials) put_sums(inc, a.partials, item);
+            if (STATS) put_sums(inc, a.partials, item);
         }
     }
     if ((MULTI || !any) && (a.sched || (int)blockIdx.x < nitems)) {
@@ -398,13 +402,17 @@ __global__ void __launch_bounds__(kThreads, 2)
                     nb[2][o] = n.W;
                     nb[3][o] = n.M;
                 };
+                auto own_cells = [&](bool rates) {
 #pragma unroll
-                for (int j = 0; j < kCells; ++j) {
-                    const int o = ob + j * BX;
-                    fx::pass_a<C_ONLY>(kx, rS[o], rL[o], rC[o], cbias, Xn[j], X[j], pz >= z0 && pz < z1);
-                    put_nb(o, Xn[j]);
-                    if (!C_ONLY) sm_new[j] = smaller(rS[o], rL[o]);
-                }
+                    for (int j = 0; j < kCells; ++j) {
+                        const int o = ob + j * BX;
+                        fx::pass_a<C_ONLY>(kx, rS[o], rL[o], rC[o], cbias, Xn[j], X[j], rates);
+                        put_nb(o, Xn[j]);
+                        if (!C_ONLY) sm_new[j] = smaller(rS[o], rL[o]);
+                    }
+                };
+                if (C_ONLY || (pz >= z0 && pz < z1)) own_cells(true);
+                else own_cells(false);             // a halo plane
                 if (rt >= 0) {
                     fx::Nb n;
                     fx::Own unused;
@@ -455,8 +463,10 @@ __global__ void __launch_bounds__(kThreads, 2)
                             const double gs = fma(ds, kx.su, ps[o]);
                             gS[j] = f ? gb : gs;
                             gL[j] = f ? gs : gb;
-                            if (a.partials && vj[j]) {
-                                const double db = (double)ib, iS = f ? db : ds, iL = f ? ds : db;
+                            if (STATS && vj[j]) {
+                                const double db = fx::eta_inc_large(kx, sm.raw[st_prev][1 - f][o], ps[o], nB[o], sm.nb[mb_prev][f][o], W[j],
+                                                                    b6 - 6 * nB[o], f);
+                                const double iS = f ? db : ds, iL = f ? ds : db;
                                 acc[1] = fma(iS, iS, acc[1]);
                                 acc[2] = fma(iL, iL, acc[2]);
                             }
@@ -464,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                                                                    (unsigned)__double2hiint(gL[j]) & 0x7fffffffu));
                         }
                         bad = bad || (vj[j] && !fx::in_box_c((unsigned)__double2hiint(gC[j]), kx.cmax));
-                        if (a.partials && vj[j]) acc[0] = fma(df, df, acc[0]);
+                        if (STATS && vj[j]) acc[0] = fma(df, df, acc[0]);
                         // a cell outside the domain stores to padding that nothing reads
                         const uint32_t at = vj[j] ? base + (uint32_t)j * (uint32_t)g.P : sink;
                         put_ghost<double, C_ONLY, uint32_t>(out, at, gS[j], gL[j], gC[j]);
@@ -508,7 +518,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 mb = mb + 1 == 3 ? 0 : mb + 1;
                 ++consumed;
             }
-            if (a.partials && !dead) {
+            if (STATS && !dead) {
                 // (sums of squares in the increments' units until here)
                 acc[0] = acc[0] * kx.sc * kx.sc;
                 acc[1] = acc[1] * kx.su * kx.su;
@@ -532,18 +542,27 @@ __global__ void __launch_bounds__(kThreads, 2)
 
 template <bool C_ONLY, bool FULL, bool MULTI>
 cudaError_t attr() {
-    return cudaFuncSetAttribute(step_fx_kernel<C_ONLY, FULL, MULTI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kSmemBytes);
+    const cudaError_t e = cudaFuncSetAttribute(step_fx_kernel<C_ONLY, FULL, MULTI, false>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(step_fx_kernel<C_ONLY, FULL, MULTI, true>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
 }
 
 void launch(const CUtensorMap *maps, const FxArgs &a, bool c_only, bool multi, int grid, bool pdl, cudaStream_t s) {
     if (a.nitems < grid) grid = a.nitems;
     const bool full = a.set == SET_WHOLE;
-#define PPF_FX_LAUNCH(CO, FU, MU) \
-    launch_step_ex(pdl, step_fx_kernel<CO, FU, MU>, grid, kThreads, kSmemBytes, s, maps[0], maps[1], maps[2], a)
-    if (multi) { if (full) PPF_FX_LAUNCH(false, true, true); else PPF_FX_LAUNCH(false, false, true); }
-    else if (c_only) { if (full) PPF_FX_LAUNCH(true, true, false); else PPF_FX_LAUNCH(true, false, false); }
-    else { if (full) PPF_FX_LAUNCH(false, true, false); else PPF_FX_LAUNCH(false, false, false); }
+#define PPF_FX_LAUNCH(CO, FU, MU)                                                                                      \
+    {                                                                                                                  \
+        if (a.partials)                                                                                                \
+            launch_step_ex(pdl, step_fx_kernel<CO, FU, MU, true>, grid, kThreads, kSmemBytes, s, maps[0], maps[1],     \
+                           maps[2], a);                                                                                \
+        else                                                                                                           \
+            launch_step_ex(pdl, step_fx_kernel<CO, FU, MU, false>, grid, kThreads, kSmemBytes, s, maps[0], maps[1],    \
+                           maps[2], a);                                                                                \
+    }
+    if (multi) { if (full) PPF_FX_LAUNCH(false, true, true) else PPF_FX_LAUNCH(false, false, true) }
+    else if (c_only) { if (full) PPF_FX_LAUNCH(true, true, false) else PPF_FX_LAUNCH(true, false, false) }
+    else { if (full) PPF_FX_LAUNCH(false, true, false) else PPF_FX_LAUNCH(false, false, false) }
 #undef PPF_FX_LAUNCH
 }
 
@@ -584,8 +603,8 @@ int fx_occupancy(bool multi) {
         if (!multi && e == cudaSuccess) e = attr<true, false, false>();
         int o = 0;
         if (e == cudaSuccess)
-            e = multi ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, step_fx_kernel<false, true, true>, kThreads, kSmemBytes)
-                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, step_fx_kernel<false, true, false>, kThreads, kSmemBytes);
+            e = multi ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, step_fx_kernel<false, true, true, true>, kThreads, kSmemBytes)
+                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, step_fx_kernel<false, true, false, true>, kThreads, kSmemBytes);
         if (e != cudaSuccess || o < 1) return 0;
         occ = o;
     }

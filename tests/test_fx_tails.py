@@ -122,3 +122,19 @@ def test_dilute_compositions_step_as_in_float64():
         got = s.download()
     ref = oracle.run(*st, 5, bc=0, params=oracle.reference_params(**p))
     assert np.abs(got[2] / ref[2] - 1).max() <= 1e-13
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,L", [(1 - 1e-6, 1e-7), (1e-7, 1 - 1e-6), (0.999, 1e-9), (1e-4, 1.01)])
+def test_sums_of_the_increments_of_a_bulk_phase(S, L):
+    """Uniform phases near their equilibrium, whose increments lie far below an ulp
+    of the value: the sums of squares against the oracle's, 1e-9 (float64's own
+    error of etaS^2 - 1 is 1e-10 of it at 1e-6 from 1)."""
+    shape = (3, 17, 40)
+    st = np.full(shape, S), np.full(shape, L), np.full(shape, 0.7)
+    with ppf.Simulation(shape, ppf.params_default(dt=DT08)) as s:
+        s.upload(*st)
+        s.step(1)
+        g = s.reduce()
+    ref = oracle.run(*st, 1, bc=0, params=oracle.reference_params(dt=DT08))
+    np.testing.assert_allclose([g["sum_detaS2"], g["sum_detaL2"]], ref[3][1:], rtol=1e-9)
