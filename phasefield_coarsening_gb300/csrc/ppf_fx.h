@@ -150,7 +150,7 @@ PPF_FX double times_2(double v, int e) {
 
 // v 2^e as a double (|v| < 2^63, the result normal or 0), without FP64 operations:
 // a conversion instruction takes the FP64 pipe as long as two or three additions.
-// unit60 is the same for 2^52 <= v < 2^63 and e = -60.
+// unit60 is the same for v > 0 and e = -60.
 PPF_FX double unit60(i64 v) {
 #ifdef __CUDA_ARCH__
     const int z = __clzll(v);
